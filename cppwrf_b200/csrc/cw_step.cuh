@@ -290,6 +290,29 @@ struct Launcher {
       check();
     }
   }
+  // a level-thread column kernel: shared level arrays of doubles (`arrays`) and of the fields' type (`fields`), and
+  // `scalars` per-column doubles; the shape is the columns per block (lc_cols), narrower where they would be too many
+  // threads
+  template <class R, int NM, class K, class... Args>
+  void run_lc(const char* name, int arrays, int fields, int scalars, const std::array<K, kNumShapes>& kerns,
+              const Packs<R, NM>& ps, Args... args) {
+    flush();
+    if (plan) return;
+    int sh = shape_for(name);
+    if (lc_threads(sh, h->nzmax) > kLcMaxThreads) sh = 0;
+    if (lc_threads(sh, h->nzmax) > kLcMaxThreads) sh = 2;
+    const int cb = lc_cols(sh);
+    const dim3 bs(unsigned(cb), unsigned(lc_threads(sh, h->nzmax) / cb));
+    const size_t smem = (size_t(h->nzmax + 1) * (arrays * sizeof(double) + fields * sizeof(R)) + scalars * sizeof(double)) * cb;
+    CW_CUDA(cudaFuncSetAttribute(kerns[size_t(sh)], cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    for (size_t c = 0; c < ps.p.size(); ++c) {
+      const int nb = ps.blocks[c][size_t(RG_LCOLS_STAG)][size_t(sh)];
+      if (nb == 0) continue;
+      begin(name);
+      kerns[size_t(sh)]<<<nb, bs, smem, h->stream>>>(ps.p[c], args...);
+      check();
+    }
+  }
   // one block per member
   template <class R, int NM, class K>
   void run_members(const char* name, int threads, K kern, const Packs<R, NM>& ps) {
@@ -379,7 +402,7 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
     for (int it = 1; it <= ns; ++it) {
       L.run_t("k_uv", RG_STAG, 1, KV(k_uv), d, rk);
       if (!spec_all) L.halo(cw_handle::H_UV);
-      L.run_cbt("k_ac", RG_COLS_STAG, kCbArrays, KC(k_ac), d, rk, it, ns);
+      L.run_lc("k_ac", kAcArrays, kAcFields, kAcScalars, KV(k_ac), d, rk, it, ns);
       if (lbc && (!spec_all || it == ns)) L.run("k_ring", RG_RING, k_ring<R, NM>, d, int(RO_ZERO_GRAD_W), rk);
       if (!spec_all) L.halo(cw_handle::H_AC);
     }

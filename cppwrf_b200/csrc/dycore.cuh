@@ -115,7 +115,7 @@ struct Dom {
 // arithmetic) and no store of a kernel can alias them. A batch (NM = 0, any number of members): the members'
 // descriptors and block prefix sums in device memory, so one launch of each kernel covers the whole batch.
 // start(kind, shape, m) is member m's first block of a launch over the index range `kind` in block shape `shape`.
-constexpr int kNumKinds = 8;
+constexpr int kNumKinds = 9;
 constexpr int kNumShapes = 3;  // point-kernel block shapes (autotuned per kernel): 128 x 1, 64 x 2, 32 x 4
 template <class R, int NM>
 struct Pack {
@@ -168,6 +168,13 @@ constexpr int CX = 32, CNW = 8;
 // their launch bound asks for keeps 3 x 256, 2 x 512 and 6 x 128 threads resident)
 __host__ __device__ constexpr int cb_warps(int s) { return s == 0 ? CNW : (s == 1 ? 2 * CNW : CNW / 2); }
 __host__ __device__ constexpr int cb_minblocks(int nw) { return nw == CNW ? 3 : (nw > CNW ? 2 : 6); }
+// the level-thread column kernels: lc_cols(s) columns per block in shape s; a thread per column and w level (whole warps)
+// and one warp for the columns' recurrences, kLcMaxThreads in all (a narrower shape where nz does not fit)
+__host__ __device__ constexpr int lc_cols(int s) { return s == 0 ? 8 : (s == 1 ? 16 : 4); }
+__host__ __device__ constexpr int lc_threads(int s, int nz) { return (lc_cols(s) * (nz + 1) + 31) / 32 * 32 + 32; }
+constexpr int kLcMaxThreads = 1024;
+// k_ac's shared memory: level arrays of doubles and of the fields' type, per-column scalars
+constexpr int kAcArrays = 5, kAcFields = 13, kAcScalars = 8;
 constexpr int kCbArrays = 6;  // shared-memory level arrays of the acoustic column block: kCbArrays x (nz + 2) x CX doubles
 __host__ __device__ __forceinline__ int cdiv(int a, int b) { return (a + b - 1) / b; }
 

@@ -25,6 +25,7 @@ enum RangeKind {
   RG_MASS_W,      // [0, nx) x [0, ny) x [0, nz+1)
   RG_FACES,       // as RG_STAG; in a patch, the faces of its cells up to the face after its last cell
   RG_TILES,       // as RG_MASS, in blocks of kQTx x kQTy columns and q_chunk(shape) levels (the TMA-staged scalars)
+  RG_LCOLS_STAG,  // as RG_COLS_STAG, in blocks of lc_cols(shape) columns (the level-thread column kernels)
 };
 // The TMA-staged scalar update's block: a tile of kQTx x kQTy columns and a chunk of levels, one thread per point
 constexpr int kQTx = 32, kQTy = 4;
@@ -44,7 +45,7 @@ __host__ __device__ __forceinline__ Range range_of(int kind, int nx, int ny, int
   switch (kind) {
     case RG_STAG: return {pi0, iu, pj0, jv, 0, nz + 1};
     case RG_MASS: return {pi0, pi1, pj0, pj1, 0, nz};
-    case RG_COLS_STAG: return {pi0, iu, pj0, jv, 0, 1};
+    case RG_COLS_STAG: case RG_LCOLS_STAG: return {pi0, iu, pj0, jv, 0, 1};
     case RG_COLS_MASS: return {pi0, pi1, pj0, pj1, 0, 1};
     case RG_RING: return {0, (nx > ny ? nx : ny) + 1, 0, nz + 1, 0, 4};
     case RG_FACES: return {pi0, pi1 + 1, pj0, jf, 0, nz + 1};
@@ -59,6 +60,7 @@ __host__ __device__ __forceinline__ Range range_of(int kind, const Dom<R>& D) {
 __host__ __device__ __forceinline__ bool is_column(int kind) { return kind == RG_COLS_STAG || kind == RG_COLS_MASS; }
 __host__ __device__ __forceinline__ int blocks_of(const Range& r, int kind, int shape = 0) {
   if (is_column(kind)) return cdiv(r.i1 - r.i0, CX) * (r.j1 - r.j0) * (r.k1 - r.k0);
+  if (kind == RG_LCOLS_STAG) return cdiv(r.i1 - r.i0, lc_cols(shape)) * (r.j1 - r.j0);
   if (kind == RG_TILES) return cdiv(r.i1 - r.i0, kQTx) * cdiv(r.j1 - r.j0, kQTy) * cdiv(r.k1 - r.k0, q_chunk(shape));
   return cdiv(r.i1 - r.i0, shape_x(shape)) * cdiv(r.j1 - r.j0, shape_y(shape)) * (r.k1 - r.k0);
 }

@@ -45,6 +45,70 @@ __device__ __forceinline__ double* cb_array(int a, int nz) {
   return cb_smem + size_t(a) * (nz + 2) * CX;
 }
 
+// ---- level-thread column kernels: a block holds lc_cols(SH) neighbouring columns along i and one thread per column and
+// w level (threadIdx.x the column, threadIdx.y the level), so that a column's levels are all in flight at once
+template <int SH, class R, int NM>
+__device__ __forceinline__ const Dom<R>& lc_member(const Pack<R, NM>& P, int& i, int& j, int& ilim) {
+  constexpr int CB = lc_cols(SH);
+  const int b = blockIdx.x;
+  const int m = member_of(P, RG_LCOLS_STAG, SH, b);
+  const Dom<R>& D = P.d[m];
+  const Range r = range_of(RG_LCOLS_STAG, D);
+  const int bx = cdiv(r.i1 - r.i0, CB);
+  const int local = b - P.start(RG_LCOLS_STAG, SH, m);
+  i = r.i0 + (local % bx) * CB + int(threadIdx.x);
+  j = r.j0 + local / bx;
+  ilim = r.i1;
+  return D;
+}
+// A column's recurrence over n levels on one thread: step(e, v) in order, e = 0, S, 2 S, ... the element's offset from the
+// arrays' first one and v[a] the element of array a (S = CB upwards, -CB downwards). The values of the next kLcAhead levels
+// are read while the present ones are stepped through, ahead of the stores that the steps make (the compiler may not move
+// a load across those): the chain is then its arithmetic, and not a shared-memory load a level as well. The last
+// read-ahead runs up to 2 kLcAhead - 1 levels past the arrays' last element: the callers' arrays have others of the
+// block's shared memory there.
+constexpr int kLcAhead = 4;
+template <int S, class F, class... T>
+__device__ __forceinline__ void lc_serial(int n, F step, const T*... a) {
+  constexpr int NA = sizeof...(T);
+  double nxt[kLcAhead][NA];
+  auto read = [&](int e) {
+#pragma unroll
+    for (int u = 0; u < kLcAhead; ++u) {
+      int m = 0;
+      ((nxt[u][m++] = double(a[e + u * S])), ...);
+    }
+  };
+  read(0);
+  int e = 0, left = n;
+  for (; left >= kLcAhead; left -= kLcAhead) {
+    double v[kLcAhead][NA];
+#pragma unroll
+    for (int u = 0; u < kLcAhead; ++u)
+#pragma unroll
+      for (int m = 0; m < NA; ++m) v[u][m] = nxt[u][m];
+    read(e + kLcAhead * S);
+#pragma unroll
+    for (int u = 0; u < kLcAhead; ++u) step(e + u * S, v[u]);
+    e += kLcAhead * S;
+  }
+#pragma unroll
+  for (int u = 0; u < kLcAhead - 1; ++u)
+    if (u < left) step(e + u * S, nxt[u]);
+}
+// one element from global to shared memory without a register in between (lc_wait: this thread's copies are done)
+template <class T>
+__device__ __forceinline__ void lc_copy(T* dst, const T* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(sizeof(T)) : "memory");
+}
+__device__ __forceinline__ void lc_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// the block's barrier, reached by its point warps and its column warp at different places of the code
+__device__ __forceinline__ void lc_bar() { asm volatile("bar.sync 0;" ::: "memory"); }
+__device__ __forceinline__ double* lc_smem() {
+  extern __shared__ double cb_smem[];
+  return cb_smem;
+}
+
 // rk_step_prep: KMu (large_step.cpp:49-66), KPrep3 (:68-81), KWW (:83-108), KCq (:127-148)
 template <class R, int NM, int NW = CNW>
 __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_ls_prep(const __grid_constant__ Pack<R, NM> P) {
@@ -273,377 +337,353 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_ss_prep(const __g
   }
 }
 
-// One acoustic substep of a column block: advance_mu_t + sumflux (KMuTCol :208-249, KMuTPoint :251-277,
-// KSumEdge :281-290) (phase 1), advance_w (KWRhs / KWExpl / KWSolve :295-408) (phase 2), calc_p_rho with
-// divergence damping (KWPRho :411-416) (phase 3). The column mass sum, the running
-// omega integral and the tridiagonal sweeps are evaluated in double in both forms, on terms staged in
-// shared memory. With lateral boundaries the spec zone's columns take LateralBC::update_mu_t (phase 1) and
-// the phi'' part of update_ph_w (phase 2); the zero-gradient w of that zone needs the neighbours' new w and
-// follows in its own launch.
-template <class R, int NM, int NW = CNW>
-__global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_ac(const __grid_constant__ Pack<R, NM> P, int rk, int it,
-                                                    int nsteps) {
-  int i, j, ilim;
-  const Dom<R>& D = cb_member(P, RG_COLS_STAG, i, j, ilim);
+// One acoustic substep of a block of columns: advance_mu_t + sumflux (KMuTCol :208-249, KMuTPoint :251-277,
+// KSumEdge :281-290), advance_w (KWRhs / KWExpl / KWSolve :295-408) and calc_p_rho with divergence damping
+// (KWPRho :411-416). One thread per column and w level (lc_cols(SH) columns, nz + 1 levels): every field is loaded once,
+// all loads of a point in flight together -- the mass divergence's into registers, advance_w's as asynchronous copies into
+// the point's own shared-memory slots -- and what a level needs from its neighbours goes through shared memory. The
+// block's last warp runs the column sum, the running omega integral and the tridiagonal sweeps, one lane per column, in
+// the reference's order and in double in both forms. With lateral boundaries the spec zone's columns take
+// LateralBC::update_mu_t and update_ph_w; the zero-gradient w of that zone needs the neighbours' new w and follows in its
+// own launch.
+// What bounds it: a block's latency (the loads, ten barriers, the column warp's chains of about 60 cycles a level), so
+// what counts is how many points an SM holds: 48 registers keep two blocks of 8 columns resident up to nz = 79 (64
+// registers: one block from nz = 60 on, 414 us instead of 268 at 200 x 200 x 60). 8 columns are the narrowest segment
+// that serves double precision (4: 76 against 59 us at 119 x 89 x 44). One warp per level row of 32 columns and 8 or 16
+// levels in turn, the form this replaced, took (us per launch, now in parentheses): 64 x 32 30 (12.8), 200 x 100 83 (19),
+// 119 x 89 x 44 90 (59), mixed 67 (46), 200 x 200 x 60 308 (268), mixed 300 x 300 x 60 737 (516).
+template <class R, int NM, int SH>
+__global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int rk, int it, int nsteps) {
   using A = double;
+  constexpr int CB = lc_cols(SH);
+  int i, j, ilim;
+  const Dom<R>& D = lc_member<SH>(P, i, j, ilim);
+  const int c = threadIdx.x, k = threadIdx.y;
   const int nx = D.nx, ny = D.ny, nz = D.nz;
-  const int lane = threadIdx.x;
-  const bool w0 = threadIdx.y == 0;
-  const bool col = i < ilim;  // a column of the member (its faces' range)
-  const R dts = R(rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound);
-  const R epssm = R(D.epssm);
+  const A dtsA = rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound;
+  const R dts = R(dtsA);
+  const bool pcol = i < nx && i < ilim && j < ny;  // a column of mass points
+  const bool espec = pcol && edge_mass(D, i, j);
+  const int ns = (nz + 1) * CB, x = k * CB + c;  // a level array's elements; this thread's element
+  double* const s0 = lc_smem();    // wdwn, then the pressure term, then the new phi''
+  double* const s1 = s0 + ns;      // the column sums' terms, then the buoyancy term
+  double* const s2 = s1 + ns;      // ww'', then w''
+  double* const s3 = s2 + ns;      // R (explicit phi'')
+  double* const s_phb = s3 + ns;
+  double* const sc = s_phb + ns + c;  // per-column scalars: sc[n * CB]
+  R* const s_ph = reinterpret_cast<R*>(s_phb + ns + kAcScalars * CB);
+  R* const s_pht = s_ph + ns;
+  R* const s_phs = s_pht + ns;
+  R* const s_w = s_phs + ns;
+  R* const s_rwt = s_w + ns;
+  R* const s_c2a = s_rwt + ns;
+  R* const s_alt = s_c2a + ns;
+  R* const s_pm1 = s_alt + ns;
+  R* const s_cqw = s_pm1 + ns;
+  R* const s_ts = s_cqw + ns;
+  R* const s_a = s_ts + ns;
+  R* const s_al = s_a + ns;
+  R* const s_ga = s_al + ns;
+  const int o2 = i + j * D.mu2.sj;
+
+  if (k >= int(blockDim.y) - 32 / CB) {  // the column warp: its first CB lanes, one per column
+    const bool on = x - (int(blockDim.y) - 32 / CB) * CB < CB && pcol, dyn = on && !espec;
+    R mu_old = 0, mut = 0, mt = 0, muts_old = 0;
+    if (on) {
+      mu_old = D.mu2.p[o2];
+      mt = __ldg(D.mu_tend.p + o2);
+      if (dyn) mut = __ldg(D.mut.p + o2);
+      else muts_old = D.muts.p[o2];
+    }
+    if (dyn) {  // w'' of the ground (KWExpl at k = 0), while the points load
+      A ws = 0;
+      if (!D.flat) {
+        const A cf1 = D.cf1, cf2 = D.cf2, cf3 = D.cf3;
+        auto U = [&](int ii, int kk) { return A(D.u2.ld(ii, j, kk)); };
+        auto V = [&](int jj, int kk) { return A(D.v2.ld(i, jj, kk)); };
+        auto H = [&](int ii, int jj) { return A(D.ht(ii, jj)); };
+        ws = A(D.msftx(i, j)) * 0.5 * D.rdx *
+             ((H(i + 1, j) - H(i, j)) * (cf1 * U(i + 1, 0) + cf2 * U(i + 1, 1) + cf3 * U(i + 1, 2)) +
+              (H(i, j) - H(i - 1, j)) * (cf1 * U(i, 0) + cf2 * U(i, 1) + cf3 * U(i, 2)));
+        if (D.do_y)
+          ws = A(D.msfty(i, j)) * 0.5 * D.rdy *
+                   ((H(i, j + 1) - H(i, j)) * (cf1 * V(j + 1, 0) + cf2 * V(j + 1, 1) + cf3 * V(j + 1, 2)) +
+                    (H(i, j) - H(i, j - 1)) * (cf1 * V(j, 0) + cf2 * V(j, 1) + cf3 * V(j, 2))) +
+               ws;
+      }
+      sc[7 * CB] = ws;
+    }
+    lc_bar();
+    if (dyn) {  // the column mass tendency: sum over k in order
+      A dmdt = 0;
+      lc_serial<CB>(nz, [&](int, const double* v) { dmdt += v[0]; }, s1 + c);
+      const A mtend = A(mt);
+      const A mu_new = A(mu_old) + A(dts) * (dmdt + mtend);
+      const R muts = mut + R(mu_new);
+      const R mav = R(0.5) * ((R(1) + R(D.epssm)) * R(mu_new) + (R(1) - R(D.epssm)) * R(A(mu_old)));
+      D.mu2.p[o2] = R(mu_new);
+      D.mudf.p[o2] = R(dmdt + mtend);
+      D.muts.p[o2] = muts;
+      D.muave.p[o2] = mav;
+      sc[0] = dmdt;
+      sc[CB] = mtend;
+      sc[2 * CB] = A(R(mu_new));
+      sc[3 * CB] = A(muts);
+      sc[4 * CB] = A(mav);
+      sc[5 * CB] = A(mut);
+    } else if (on) {  // the spec zone: mu and mu_ts take dts mu_tend (LateralBC::update_mu_t :363-372)
+      const R mu = mu_old + dts * mt, muts = muts_old + dts * mt;
+      D.mu2.p[o2] = mu;
+      D.muts.p[o2] = muts;
+      sc[CB] = A(mt);
+      sc[2 * CB] = A(mu);
+      sc[3 * CB] = A(muts);
+    }
+    lc_bar();
+    lc_bar();
+    if (dyn) {  // ww'' by the running integral (ww1 of level k + 1 staged in s2[k + 1])
+      A ww_full = 0;
+      double* const w = s2 + CB + c;
+      lc_serial<CB>(nz - 1, [&](int e, const double* v) {
+        ww_full = ww_full - v[0];
+        w[e] = A(R(ww_full - v[1]));
+      }, s1 + c, w);
+    }
+    lc_bar();
+    lc_bar();
+    lc_bar();
+    lc_bar();
+    lc_bar();
+    if (dyn) {  // KWSolve: forward and backward sweeps
+      A wprev = s2[c];
+      double* const wu = s2 + CB + c;
+      lc_serial<CB>(nz, [&](int e, const double* v) {
+        wprev = (v[0] - v[1] * wprev) * v[2];
+        wu[e] = wprev;
+      }, wu, s_a + CB + c, s_al + CB + c);
+      A wnext = wprev;
+      double* const wd = s2 + (nz - 1) * CB + c;
+      lc_serial<-CB>(nz - 1, [&](int e, const double* v) {
+        wnext = v[0] - v[1] * wnext;
+        wd[e] = wnext;
+      }, wd, s_ga + (nz - 1) * CB + c);
+    }
+    lc_bar();
+    lc_bar();
+    return;
+  }
+
+  const A eps = D.epssm, ope = 1.0 + eps, ome = 1.0 - eps;
   const bool first = it == 1, last = it == nsteps;
   const R rn = R(nsteps);
-  const bool mass = col && i < nx && j < ny;
-  const bool spec = mass && edge_mass(D, i, j);
-  const bool dyn = mass && !spec;
-  double* s0 = cb_array(0, nz);
-  double* s1 = cb_array(1, nz);
-  double* s2 = cb_array(2, nz);
-  double* sc = cb_array(3, nz);  // per-column scalars: sc[n * CX + lane]
-  double* s_t2s = cb_array(4, nz);  // theta'' before the substep's update (t_2save), phase 1 to phase 2
+  const bool lm = k < nz, mass = pcol && k <= nz, spec = espec && k <= nz, dyn = mass && !spec;
+  // one element offset per storage class: mass and w levels, x faces, y faces, and their 2-D fields
+  const int sjM = D.t2.sj, o = i + j * sjM + k * D.t2.sk;
+  const int oU = i + j * D.u2.sj + k * D.u2.sk, sjV = D.v2.sj, oV = i + j * sjV + k * D.v2.sk;
+  const int oU2 = i + j * D.muu.sj, oV2 = i + j * D.muv.sj;
 
-  if (mass)  // phase 1's inputs of the block's columns into L2 (a level above nz takes level 0: inside the field)
-    CB_LOOP(k, nz + 1) {
-      const int kh = k < nz ? k : 0;
-      pf_l2(&D.u2(i, j, kh));
-      pf_l2(&D.u2(i + 1, j, kh));
-      pf_l2(&D.u_save(i, j, kh));
-      pf_l2(&D.ru_m(i, j, kh));
-      if (D.do_y) {
-        pf_l2(&D.v2(i, j, kh));
-        pf_l2(&D.v2(i, j + 1, kh));
-        pf_l2(&D.v_save(i, j, kh));
-        pf_l2(&D.v_save(i, j + 1, kh));
-        pf_l2(&D.rv_m(i, j, kh));
-      }
-      pf_l2(&D.ww1(i, j, k));
-      pf_l2(&D.ww_m(i, j, k));
-      if (k < nz) {
-        pf_l2(&D.t2(i, j, k));
-        pf_l2(&D.t_tend(i, j, k));
-        pf_l2(&D.t_save(i, j, k));
-        if (D.do_y) {
-          pf_l2(&D.t_save(i, j - 1, k));
-          pf_l2(&D.t_save(i, j + 1, k));
-        }
-      }
-    }
-  {  // phase 1
-    if (col && D.spec_x && i == nx && j < ny)  // KSumEdge, east face (specified or open x)
-      CB_LOOP(k, nz) {
-        const R su = (first ? R(0) : D.ru_m(i, j, k)) + D.u2.ld(i, j, k);
-        const R cpl = (R(D.c1h[k]) * D.muu.ld(i, j, 0) + R(D.c2h[k])) * D.u_save.ld(i, j, k);
-        D.ru_m(i, j, k) = last ? su / rn + div_msf(cpl, D.msfuy(i, j)) : su;
-      }
-    if (col && D.spec_y && j == ny && i < nx)  // KSumEdge, north face (specified or open y)
-      CB_LOOP(k, nz) {
-        const R su = (first ? R(0) : D.rv_m(i, j, k)) + D.v2.ld(i, j, k);
-        const R cpl = (R(D.c1h[k]) * D.muv.ld(i, j, 0) + R(D.c2h[k])) * D.v_save.ld(i, j, k);
-        D.rv_m(i, j, k) = last ? su / rn + cpl * D.msfvx_inv(i, j) : su;
-      }
-    if (spec) {  // spec zone: sumflux of ww only; mu and mu_ts take dts mu_tend (LateralBC::update_mu_t :363-372)
-      CB_LOOP(k, nz + 1) {
-        const R sw = (first ? R(0) : D.ww_m(i, j, k)) + D.ww(i, j, k);
-        D.ww_m(i, j, k) = last ? sw / rn + D.ww1.ld(i, j, k) : sw;
-      }
-      if (w0) {
-        D.mu2(i, j, 0) += dts * D.mu_tend.ld(i, j, 0);
-        D.muts(i, j, 0) += dts * D.mu_tend.ld(i, j, 0);
-      }
-    }
-    if (mass)
-      CB_LOOP(k, nz) {  // dv of each level (KMuTDiv), the time sums of ru, rv (KMuTPoint), ww1 staged
-        const R c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
-        const R u_k = D.u2.ld(i, j, k), usv = D.u_save.ld(i, j, k), muu = D.muu.ld(i, j, 0), msfuy = D.msfuy(i, j);
-        const R rum = first ? R(0) : D.ru_m(i, j, k);
-        R v_k = 0, vsv = 0, muv = 0, mvxi = 0, rvm = 0;
-        if (D.do_y) {
-          v_k = D.v2.ld(i, j, k);
-          vsv = D.v_save.ld(i, j, k);
-          muv = D.muv.ld(i, j, 0);
-          mvxi = D.msfvx_inv(i, j);
-          rvm = first ? R(0) : D.rv_m(i, j, k);
-        }
-        if (dyn) {
-          const R u_ip = D.u2.ld(i + 1, j, k), usv_ip = D.u_save.ld(i + 1, j, k), muu_ip = D.muu.ld(i + 1, j, 0);
-          const R msfuy_ip = D.msfuy(i + 1, j);
-          R v_jp = 0, vsv_jp = 0, muv_jp = 0, mvxi_jp = 0;
-          if (D.do_y) {
-            v_jp = D.v2.ld(i, j + 1, k);
-            vsv_jp = D.v_save.ld(i, j + 1, k);
-            muv_jp = D.muv.ld(i, j + 1, 0);
-            mvxi_jp = D.msfvx_inv(i, j + 1);
-          }
-          if (k + 1 < nz) s2[(k + 1) * CX + lane] = A(D.ww1.ld(i, j, k + 1));
-          // KMuTDiv (small_step.cpp:194-206), the expression of mut_dv
-          const R fx = (u_ip + div_msf((c1h * muu_ip + c2h) * usv_ip, msfuy_ip)) - (u_k + div_msf((c1h * muu + c2h) * usv, msfuy));
-          R d = R(D.rdx) * fx;
-          if (D.do_y) d += R(D.rdy) * ((v_jp + (c1h * muv_jp + c2h) * vsv_jp * mvxi_jp) - (v_k + (c1h * muv + c2h) * vsv * mvxi));
-          const A dv = A(D.msftx(i, j) * D.msfty(i, j) * d);
-          s0[k * CX + lane] = dv;
-          s1[k * CX + lane] = D.dnw[k] * dv;  // the term of the column sum, for the serial sum below
-        }
-        const R su = rum + u_k;
-        D.ru_m(i, j, k) = last ? su / rn + div_msf((c1h * muu + c2h) * usv, msfuy) : su;
-        if (D.do_y) {
-          const R sv = rvm + v_k;
-          D.rv_m(i, j, k) = last ? sv / rn + (c1h * muv + c2h) * vsv * mvxi : sv;
-        }
-      }
-    __syncthreads();
-    if (mass)  // while warp 0 sums the column: phase 2's inputs into L2
-      CB_LOOP_W1(k, nz + 1) {
-        pf_l2(&D.ph_tend(i, j, k));
-        pf_l2(&D.w2(i, j, k));
-        pf_l2(&D.ph_save(i, j, k));
-        pf_l2(&D.ph2(i, j, k));
-        pf_l2(&D.rw_tend(i, j, k));
-        pf_l2(&D.a(i, j, k));
-        pf_l2(&D.alpha(i, j, k));
-        pf_l2(&D.gamma(i, j, k));
-        if (!D.flat) pf_l2(D.phb.p + (i * D.phb.si + j * D.phb.sj + k * D.phb.sk));
-        if (k < nz) {
-          pf_l2(&D.c2a(i, j, k));
-          pf_l2(&D.alt(i, j, k));
-          pf_l2(&D.pm1(i, j, k));
-          if (D.n_moist) pf_l2(&D.cqw(i, j, k));
-        }
-      }
-    if (dyn && w0) {  // the column mass tendency: sum over k in order
-      A dmdt = 0;
-#pragma unroll 4
-      for (int k = 0; k < nz; ++k) dmdt += s1[k * CX + lane];
-      const A mtend = A(D.mu_tend.ld(i, j, 0));
-      const A mu_old = A(D.mu2(i, j, 0));
-      const A mu_new = mu_old + A(dts) * (dmdt + mtend);
-      D.mu2(i, j, 0) = R(mu_new);
-      D.mudf(i, j, 0) = R(dmdt + mtend);
-      D.muts(i, j, 0) = D.mut.ld(i, j, 0) + R(mu_new);
-      D.muave(i, j, 0) = R(0.5) * ((R(1) + epssm) * R(mu_new) + (R(1) - epssm) * R(mu_old));
-      sc[0 * CX + lane] = dmdt;
-      sc[1 * CX + lane] = mtend;
-    }
-    __syncthreads();
-    if (dyn) {  // the decrement of the omega integral at each level
-      const A dmdt = sc[0 * CX + lane], mtend = sc[1 * CX + lane];
-      const A msfty = A(D.msfty(i, j));
-      CB_LOOP_SH(k, nz - 1) s1[k * CX + lane] = div_msf(D.dnw[k] * (D.c1h[k] * dmdt + s0[k * CX + lane] + D.c1h[k] * mtend), msfty);
-    }
-    __syncthreads();
-    if (dyn && w0) {  // ww'' by the running integral (ww1 of level k + 1 staged in s2[k + 1])
-      A ww_full = 0;
-      s2[0 * CX + lane] = 0;
-#pragma unroll 4
-      for (int k = 0; k < nz - 1; ++k) {
-        ww_full = ww_full - s1[k * CX + lane];
-        s2[(k + 1) * CX + lane] = A(R(ww_full - s2[(k + 1) * CX + lane]));
-      }
-      s2[nz * CX + lane] = 0;
-    }
-    __syncthreads();
-    if (mass) {
-      CB_LOOP(k, nz + 1) {  // ww'' and its time sum; theta'' (KMuTPoint), every load before the first store
-        R wpp = 0, wwm = 0, ww1 = 0;
-        if (dyn) {
-          wpp = R(s2[k * CX + lane]);
-          wwm = first ? R(0) : D.ww_m(i, j, k);
-          ww1 = D.ww1.ld(i, j, k);
-        }
-        R tk = 0, tnew = 0;
-        if (k < nz) {
-          tk = D.t2(i, j, k);
-          const R ttend = D.t_tend.ld(i, j, k);
-          if (spec) {  // theta'' of the spec zone (update_mu_t)
-            tnew = tk + dts * ttend;
-          } else {
-            const R u_k = D.u2.ld(i, j, k), u_ip = D.u2.ld(i + 1, j, k);
-            const R ts = D.t_save.ld(i, j, k), ts_ip = D.t_save.ld(i + 1, j, k), ts_im = D.t_save.ld(i - 1, j, k);
-            R v_k = 0, v_jp = 0, ts_jp = 0, ts_jm = 0;
-            if (D.do_y) {
-              v_k = D.v2.ld(i, j, k);
-              v_jp = D.v2.ld(i, j + 1, k);
-              ts_jp = D.t_save.ld(i, j + 1, k);
-              ts_jm = D.t_save.ld(i, j - 1, k);
-            }
-            const R ts_kp = k + 1 < nz ? D.t_save.ld(i, j, k + 1) : R(0), ts_km = k >= 1 ? D.t_save.ld(i, j, k - 1) : R(0);
-            const R msfty = D.msfty(i, j), msftx = D.msftx(i, j);
-            R hflux = R(0.5) * R(D.rdx) * (u_ip * (ts_ip + ts) - u_k * (ts + ts_im));
-            if (D.do_y) hflux += R(0.5) * R(D.rdy) * (v_jp * (ts_jp + ts) - v_k * (ts + ts_jm));
-            const R tn = tk + msfty * dts * ttend;
-            const R wd_kp = (k + 1 == nz) ? R(0) : R(s2[(k + 1) * CX + lane]) * (R(D.fnm[k + 1]) * ts_kp + R(D.fnp[k + 1]) * ts);
-            const R wd_k = (k == 0) ? R(0) : R(s2[k * CX + lane]) * (R(D.fnm[k]) * ts + R(D.fnp[k]) * ts_km);
-            tnew = tn - dts * msfty * (msftx * hflux + R(D.rdnw[k]) * (wd_kp - wd_k));
-          }
-        }
-        if (dyn) {
-          const R sw = wwm + (k == 0 ? R(0) : wpp);
-          D.ww(i, j, k) = wpp;
-          D.ww_m(i, j, k) = last ? sw / rn + ww1 : sw;
-        }
-        if (k < nz) {
-          s_t2s[k * CX + lane] = double(tk);  // t_2save: kept in shared memory for advance_w
-          D.t2(i, j, k) = tnew;
-        }
-      }
-    }
-    __syncthreads();
+  // KSumEdge: the east face (specified or open x) and the north face (specified or open y)
+  if (lm && i < ilim && D.spec_x && i == nx && j < ny) {
+    const R su = (first ? R(0) : D.ru_m.p[oU]) + __ldg(D.u2.p + oU);
+    const R cpl = (R(D.c1h[k]) * __ldg(D.muu.p + oU2) + R(D.c2h[k])) * __ldg(D.u_save.p + oU);
+    D.ru_m.p[oU] = last ? su / rn + div_msf(cpl, D.msfuy(i, j)) : su;
   }
-  {  // phase 2
-    // advance_w in double in both forms (the mixed form's fields are float; the explicit phi'' and w'' right-hand
-    // sides are differences of nearly equal pressure-gradient and buoyancy terms, kept in double). For the FP64
-    // form every conversion below is the identity and the operations are the reference's, in its order.
-    const A dtsA = rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound, eps = D.epssm;
-    const A ope = 1.0 + eps, ome = 1.0 - eps;
-    auto mhA = [&](int kk, A m) { return D.c1h[kk] * m + D.c2h[kk]; };
-    auto mfA = [&](int kk, A m) { return D.c1f[kk] * m + D.c2f[kk]; };
-    A mut = 0, muts = 0, mav = 0, msfty = 1;
-    double* s_a = cb_array(3, nz);
-    double* s_al = cb_array(4, nz);
-    double* s_ga = cb_array(5, nz);
-    if (spec) {  // phi'' of the spec zone (LateralBC::update_ph_w, KUpdatePh :374-386)
-      const R mts = D.muts(i, j, 0), mold = mts - dts * D.mu_tend.ld(i, j, 0);
-      CB_LOOP(k, nz + 1) {
-        const R m_old = R(D.c1f[k]) * mold + R(D.c2f[k]), m_new = R(D.c1f[k]) * mts + R(D.c2f[k]);
-        D.ph2(i, j, k) = D.ph2(i, j, k) * m_old / m_new + dts * D.ph_tend.ld(i, j, k) / m_new + D.ph_save.ld(i, j, k) * (m_old / m_new - R(1));
-      }
-    }
+  if (lm && i < ilim && D.spec_y && j == ny && i < nx) {
+    const R su = (first ? R(0) : D.rv_m.p[oV]) + __ldg(D.v2.p + oV);
+    const R cpl = (R(D.c1h[k]) * __ldg(D.muv.p + oV2) + R(D.c2h[k])) * __ldg(D.v_save.p + oV);
+    D.rv_m.p[oV] = last ? su / rn + cpl * D.msfvx_inv(i, j) : su;
+  }
+  if (mass) {
+    lc_copy(s_ph + x, D.ph2.p + o);
+    lc_copy(s_pht + x, D.ph_tend.p + o);
+    lc_copy(s_phs + x, D.ph_save.p + o);
     if (dyn) {
-      mut = A(D.mut.ld(i, j, 0));
-      muts = A(D.muts(i, j, 0));
-      mav = A(D.muave(i, j, 0));
-      msfty = A(D.msfty(i, j));
-      CB_LOOP_SH(k, nz + 1) {  // KWRhs: R (explicit phi'') and t_2ave
-        A r;
-        if (k == 0 || (D.top_lid && k == nz)) {
-          r = 0;
-        } else {
-          A rr = dtsA * (A(D.ph_tend.ld(i, j, k)) + 0.5 * k::g * (1.0 - eps) * A(D.w2(i, j, k)));
-          if (k < nz) {
-            auto wdwn = [&](int mm) {
-              return 0.5 * (A(D.ww(i, j, mm)) + A(D.ww(i, j, mm - 1))) * D.rdnw[mm - 1] *
-                     (A(D.ph_save.ld(i, j, mm)) - A(D.ph_save.ld(i, j, mm - 1)) + A(D.phb64(i, j, mm)) - A(D.phb64(i, j, mm - 1)));
-            };
-            rr -= dtsA * (D.fnm[k] * wdwn(k + 1) + D.fnp[k] * wdwn(k));
-          }
-          r = A(D.ph2(i, j, k)) + msfty * rr / mfA(k, mut);
-        }
-        s0[k * CX + lane] = r;
-        if (k < nz) {
-          const A tav = 0.5 * ((1.0 + eps) * A(D.t2(i, j, k)) + (1.0 - eps) * s_t2s[k * CX + lane]);
-          s1[k * CX + lane] = (tav + D.c1h[k] * mav * k::t0) / (mhA(k, muts) * (k::t0 + A(D.t_save.ld(i, j, k))));
-        }
-      }
+      lc_copy(s_phb + x, D.phb64.p + (i * D.phb64.si + j * D.phb64.sj + k * D.phb64.sk));
+      lc_copy(s_w + x, D.w2.p + o);
+      lc_copy(s_rwt + x, D.rw_tend.p + o);
+      lc_copy(s_a + x, D.a.p + o);
+      lc_copy(s_al + x, D.alpha.p + o);
+      lc_copy(s_ga + x, D.gamma.p + o);
+      if (D.n_moist > 0 && lm) lc_copy(s_cqw + x, D.cqw.p + o);
     }
-    __syncthreads();
+    if (lm) {
+      lc_copy(s_ts + x, D.t_save.p + o);
+      lc_copy(s_c2a + x, D.c2a.p + o);
+      lc_copy(s_alt + x, D.alt.p + o);
+      lc_copy(s_pm1 + x, D.pm1.p + o);
+    }
+  }
+  // dv (KMuTDiv, small_step.cpp:194-206), the time sums of ru, rv and theta's horizontal flux (KMuTPoint)
+  A dv = 0;
+  R tn = 0, tk = 0, hflux = 0, ww1k = 0, wwm = 0, msfty = 1, msftx = 1;
+  if (mass) {
+    if (k >= 1 && lm) ww1k = __ldg(D.ww1.p + o);
+    if (!first) wwm = D.ww_m.p[o];
     if (dyn) {
-      const A msft_inv = div_msf(1.0, msfty);
-      CB_LOOP_SH(k, nz + 1) {  // KWExpl: explicit w''
-        A wn;
-        if (k == 0) {
-          if (!D.flat) {
-            const A cf1 = D.cf1, cf2 = D.cf2, cf3 = D.cf3;
-            auto U = [&](int ii, int kk) { return A(D.u2.ld(ii, j, kk)); };
-            auto V = [&](int jj, int kk) { return A(D.v2.ld(i, jj, kk)); };
-            auto H = [&](int ii, int jj) { return A(D.ht(ii, jj)); };
-            A ws = A(D.msftx(i, j)) * 0.5 * D.rdx *
-                   ((H(i + 1, j) - H(i, j)) * (cf1 * U(i + 1, 0) + cf2 * U(i + 1, 1) + cf3 * U(i + 1, 2)) +
-                    (H(i, j) - H(i - 1, j)) * (cf1 * U(i, 0) + cf2 * U(i, 1) + cf3 * U(i, 2)));
-            if (D.do_y)
-              ws = msfty * 0.5 * D.rdy *
-                       ((H(i, j + 1) - H(i, j)) * (cf1 * V(j + 1, 0) + cf2 * V(j + 1, 1) + cf3 * V(j + 1, 2)) +
-                        (H(i, j) - H(i, j - 1)) * (cf1 * V(j, 0) + cf2 * V(j, 1) + cf3 * V(j, 2))) +
-                   ws;
-            wn = ws;
-          } else {
-            wn = 0;
-          }
-        } else {
-          const A r_k = s0[k * CX + lane], r_km1 = s0[(k - 1) * CX + lane];
-          const A ph_k = A(D.ph2(i, j, k)), ph_km1 = A(D.ph2(i, j, k - 1));
-          const A c2a_k1 = A(D.c2a.ld(i, j, k - 1)), alt_k1 = A(D.alt.ld(i, j, k - 1));
-          if (k < nz) {
-            const A r_kp1 = s0[(k + 1) * CX + lane], ph_kp1 = A(D.ph2(i, j, k + 1));
-            const A cq1 = 1.0 / (1.0 + A(cqw_(D, i, j, k)));
-            const A c2a_k = A(D.c2a.ld(i, j, k)), alt_k = A(D.alt.ld(i, j, k));
-            wn = A(D.w2(i, j, k)) + dtsA * A(D.rw_tend.ld(i, j, k)) +
-                 msft_inv * cq1 *
-                     (0.5 * dtsA * k::g * D.rdn[k] *
-                      (c2a_k * D.rdnw[k] / mhA(k, mut) * (ope * (r_kp1 - r_k) + ome * (ph_kp1 - ph_k)) -
-                       c2a_k1 * D.rdnw[k - 1] / mhA(k - 1, mut) * (ope * (r_k - r_km1) + ome * (ph_k - ph_km1)))) +
-                 dtsA * k::g * msft_inv *
-                     (D.rdn[k] * (c2a_k * alt_k * s1[k * CX + lane] - c2a_k1 * alt_k1 * s1[(k - 1) * CX + lane]) -
-                      D.c1f[k] * mav);
-          } else {
-            const int km = nz - 1;
-            wn = A(D.w2(i, j, k)) + dtsA * A(D.rw_tend.ld(i, j, k)) +
-                 msft_inv * (-0.5 * dtsA * k::g / mhA(km, mut) * (D.rdnw[km] * D.rdnw[km]) * 2.0 * c2a_k1 *
-                                 (ope * (r_k - r_km1) + ome * (ph_k - ph_km1)) -
-                             dtsA * k::g * (2.0 * D.rdnw[km] * c2a_k1 * alt_k1 * s1[km * CX + lane] + D.c1f[k] * mav));
-            if (D.top_lid) wn = 0;
-          }
-        }
-        s2[k * CX + lane] = wn;
-        s_a[k * CX + lane] = A(D.a.ld(i, j, k));
-        s_al[k * CX + lane] = A(D.alpha.ld(i, j, k));
-        s_ga[k * CX + lane] = A(D.gamma.ld(i, j, k));
-      }
+      msfty = D.msfty(i, j);
+      msftx = D.msftx(i, j);
     }
-    __syncthreads();
-    if (dyn && w0) {  // KWSolve: forward and backward sweeps
-      A wprev = s2[0 * CX + lane];
-#pragma unroll 4
-      for (int k = 1; k <= nz; ++k) {
-        wprev = (s2[k * CX + lane] - s_a[k * CX + lane] * wprev) * s_al[k * CX + lane];
-        s2[k * CX + lane] = wprev;
+    if (lm) {
+      const R c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
+      const R u_k = __ldg(D.u2.p + oU), usv = __ldg(D.u_save.p + oU), muu = __ldg(D.muu.p + oU2), msfuy = D.msfuy(i, j);
+      const R rum = first ? R(0) : D.ru_m.p[oU];
+      R v_k = 0, vsv = 0, muv = 0, mvxi = 0, rvm = 0;
+      if (D.do_y) {
+        v_k = __ldg(D.v2.p + oV);
+        vsv = __ldg(D.v_save.p + oV);
+        muv = __ldg(D.muv.p + oV2);
+        mvxi = D.msfvx_inv(i, j);
+        rvm = first ? R(0) : D.rv_m.p[oV];
       }
-      A wnext = wprev;
-#pragma unroll 4
-      for (int k = nz - 1; k >= 1; --k) {
-        wnext = s2[k * CX + lane] - s_ga[k * CX + lane] * wnext;
-        s2[k * CX + lane] = wnext;
-      }
-    }
-    __syncthreads();
-    if (D.damp_opt == 3) {  // damp_opt 3: implicit Rayleigh damping of w toward 0 near the top (KWSolve :393-404)
+      tk = D.t2.p[o];
+      const R ttend = __ldg(D.t_tend.p + o);
+      const R cu = div_msf((c1h * muu + c2h) * usv, msfuy);
+      const R cv = (c1h * muv + c2h) * vsv * mvxi;
       if (dyn) {
-        const R dampmag = dts * R(D.dampcoef), hdepth = R(D.zdamp), pi = R(0x1.921fb54442d18p+1);  // 4 atan(1)
-        const R htop = (D.ph_save.ld(i, j, nz) + D.phb(i, j, nz)) / R(k::g), hbot = htop - hdepth;
-        CB_LOOP_SH(k, nz + 1) {
-          if (k >= 1) {
-            const R hk = (D.ph_save.ld(i, j, k) + D.phb(i, j, k)) / R(k::g);
-            R dampwt = 0;
-            if (hk >= hbot) {
-              const R sn = R(cw_sin(double(R(0.5) * pi * (hk - hbot) / hdepth)));
-              dampwt = dampmag * sn * sn;
-            }
-            s2[k * CX + lane] = A(R((R(s2[k * CX + lane]) - dampwt * mf_(D, k, R(mut)) * D.w_save.ld(i, j, k)) / (R(1) + dampwt)));
-          }
+        const R u_ip = __ldg(D.u2.p + oU + 1), usv_ip = __ldg(D.u_save.p + oU + 1), muu_ip = __ldg(D.muu.p + oU2 + 1);
+        const R msfuy_ip = D.msfuy(i + 1, j);
+        const R* const pts = D.t_save.p + o;
+        const R ts = __ldg(pts), ts_ip = __ldg(pts + 1), ts_im = __ldg(pts - 1);
+        const R fx = (u_ip + div_msf((c1h * muu_ip + c2h) * usv_ip, msfuy_ip)) - (u_k + cu);
+        R d = R(D.rdx) * fx;
+        hflux = R(0.5) * R(D.rdx) * (u_ip * (ts_ip + ts) - u_k * (ts + ts_im));
+        if (D.do_y) {
+          const R v_jp = __ldg(D.v2.p + oV + sjV), vsv_jp = __ldg(D.v_save.p + oV + sjV);
+          const R muv_jp = __ldg(D.muv.p + oV2 + D.muv.sj), mvxi_jp = D.msfvx_inv(i, j + 1);
+          const R ts_jp = __ldg(pts + sjM), ts_jm = __ldg(pts - sjM);
+          d += R(D.rdy) * ((v_jp + (c1h * muv_jp + c2h) * vsv_jp * mvxi_jp) - (v_k + cv));
+          hflux += R(0.5) * R(D.rdy) * (v_jp * (ts_jp + ts) - v_k * (ts + ts_jm));
         }
+        dv = A(msftx * msfty * d);
+        s1[x] = D.dnw[k] * dv;  // the term of the column sum
+        tn = tk + msfty * dts * ttend;
+      } else {
+        tn = tk + dts * ttend;  // theta'' of the spec zone (update_mu_t)
       }
-      __syncthreads();  // the member's option: uniform over the block
+      const R su = rum + u_k;
+      D.ru_m.p[oU] = last ? su / rn + cu : su;
+      if (D.do_y) {
+        const R sv = rvm + v_k;
+        D.rv_m.p[oV] = last ? sv / rn + cv : sv;
+      }
     }
-    // w'' and phi'' (dyn columns), then calc_p_rho of the level (every mass column, phase 3) from the new
-    // phi'' of levels k and k + 1: recomputed from the shared terms here (the same expression as the store),
-    // read back for the spec zone (written before the last barriers) and for the unchanged level 0
-    auto ph_new = [&](int m) { return R(s0[m * CX + lane] + msfty * 0.5 * dtsA * k::g * ope * s2[m * CX + lane] / mfA(m, muts)); };
-    if (mass)
-      CB_LOOP(k, nz + 1) {
-        R wk = 0, phk = 0, phkp = 0;
-        if (dyn) {
-          wk = R(s2[k * CX + lane]);
-          phk = k >= 1 ? ph_new(k) : D.ph2(i, j, 0);
-          if (k < nz) phkp = ph_new(k + 1);
-        } else if (k < nz) {
-          phk = D.ph2(i, j, k);
-          phkp = D.ph2(i, j, k + 1);
-        }
-        if (dyn) {
-          D.w2(i, j, k) = wk;
-          if (k >= 1) D.ph2(i, j, k) = phk;
-        }
-        if (k < nz) p_rho_point_ph<true>(D, i, j, k, true, phk, phkp);
+    s2[x] = A(ww1k);  // (0 at the ground and the lid)
+  }
+  lc_bar();
+  lc_bar();  // the column's sum
+  if (dyn && k < nz - 1)  // the decrement of the omega integral at each level
+    s1[x] = div_msf(D.dnw[k] * (D.c1h[k] * sc[0] + dv + D.c1h[k] * sc[CB]), A(msfty));
+  lc_bar();
+  lc_wait();
+  lc_bar();  // ww''
+  const A msfA = A(msfty);
+  A phn = 0;  // the new phi'' (as stored)
+  R tnew = 0;
+  if (dyn) {  // ww'' and its time sum; theta'' (KMuTPoint); the terms of advance_w that other levels read
+    const R wpp = R(s2[x]);
+    const R sw = wwm + (k == 0 ? R(0) : wpp);
+    D.ww.p[o] = wpp;
+    D.ww_m.p[o] = last ? sw / rn + ww1k : sw;
+    if (lm) {
+      const R ts = s_ts[x];
+      const R wd_kp = (k + 1 == nz) ? R(0) : R(s2[x + CB]) * (R(D.fnm[k + 1]) * s_ts[x + CB] + R(D.fnp[k + 1]) * ts);
+      const R wd_k = (k == 0) ? R(0) : wpp * (R(D.fnm[k]) * ts + R(D.fnp[k]) * s_ts[x - CB]);
+      tnew = tn - dts * msfty * (msftx * hflux + R(D.rdnw[k]) * (wd_kp - wd_k));
+      D.t2.p[o] = tnew;
+      // t_2ave and the buoyancy term (advance_w in double in both forms: the explicit phi'' and w'' right-hand sides are
+      // differences of nearly equal terms; in the FP64 form every conversion is the identity)
+      const A tav = 0.5 * (ope * A(tnew) + ome * A(tk));
+      const A t2a = (tav + D.c1h[k] * sc[4 * CB] * k::t0) / ((D.c1h[k] * sc[3 * CB] + D.c2h[k]) * (k::t0 + A(ts)));
+      s1[x] = A(s_c2a[x]) * A(s_alt[x]) * t2a;
+      if (k == nz - 1) sc[6 * CB] = t2a;
+    }
+    if (k >= 1)  // wdwn of level k
+      s0[x] = 0.5 * (s2[x] + s2[x - CB]) * D.rdnw[k - 1] * (A(s_phs[x]) - A(s_phs[x - CB]) + s_phb[x] - s_phb[x - CB]);
+  } else if (spec) {
+    const R sw = wwm + D.ww.p[o];
+    D.ww_m.p[o] = last ? sw / rn + __ldg(D.ww1.p + o) : sw;
+    if (lm) {
+      tnew = tn;
+      D.t2.p[o] = tnew;
+    }
+    // phi'' (LateralBC::update_ph_w, KUpdatePh :374-386)
+    const R mts = R(sc[3 * CB]), mold = mts - dts * R(sc[CB]);
+    const R m_old = R(D.c1f[k]) * mold + R(D.c2f[k]), m_new = R(D.c1f[k]) * mts + R(D.c2f[k]);
+    const R pn = s_ph[x] * m_old / m_new + dts * s_pht[x] / m_new + s_phs[x] * (m_old / m_new - R(1));
+    D.ph2.p[o] = pn;
+    phn = A(pn);
+  }
+  lc_bar();
+  const A mut = dyn ? sc[5 * CB] : A(1);
+  A r = 0;
+  if (dyn) {  // KWRhs: R (explicit phi'')
+    if (k > 0 && !(D.top_lid && k == nz)) {
+      A rr = dtsA * (A(s_pht[x]) + 0.5 * k::g * (1.0 - eps) * A(s_w[x]));
+      if (lm) rr -= dtsA * (D.fnm[k] * s0[x + CB] + D.fnp[k] * s0[x]);
+      r = A(s_ph[x]) + msfA * rr / (D.c1f[k] * mut + D.c2f[k]);
+    }
+    s3[x] = r;
+  }
+  lc_bar();
+  if (dyn && lm)  // the pressure term of each layer
+    s0[x] = A(s_c2a[x]) * D.rdnw[k] / (D.c1h[k] * mut + D.c2h[k]) *
+            (ope * (s3[x + CB] - r) + ome * (A(s_ph[x + CB]) - A(s_ph[x])));
+  lc_bar();
+  if (dyn) {  // KWExpl: explicit w''
+    const A msft_inv = div_msf(1.0, msfA), mav = sc[4 * CB];
+    A wn;
+    if (k == 0) {
+      wn = sc[7 * CB];
+    } else if (lm) {
+      const A cq1 = 1.0 / (1.0 + (D.n_moist > 0 ? A(s_cqw[x]) : A(0)));
+      wn = A(s_w[x]) + dtsA * A(s_rwt[x]) + msft_inv * cq1 * (0.5 * dtsA * k::g * D.rdn[k] * (s0[x] - s0[x - CB])) +
+           dtsA * k::g * msft_inv * (D.rdn[k] * (s1[x] - s1[x - CB]) - D.c1f[k] * mav);
+    } else {
+      const int km = nz - 1;
+      const A c2a_k1 = A(s_c2a[x - CB]), alt_k1 = A(s_alt[x - CB]);
+      wn = A(s_w[x]) + dtsA * A(s_rwt[x]) +
+           msft_inv * (-0.5 * dtsA * k::g / (D.c1h[km] * mut + D.c2h[km]) * (D.rdnw[km] * D.rdnw[km]) * 2.0 * c2a_k1 *
+                           (ope * (r - s3[x - CB]) + ome * (A(s_ph[x]) - A(s_ph[x - CB]))) -
+                       dtsA * k::g * (2.0 * D.rdnw[km] * c2a_k1 * alt_k1 * sc[6 * CB] + D.c1f[k] * mav));
+      if (D.top_lid) wn = 0;
+    }
+    s2[x] = wn;
+  }
+  lc_bar();
+  lc_bar();  // the tridiagonal sweeps
+  if (dyn) {  // w'' and phi''
+    A ws = s2[x];
+    if (D.damp_opt == 3 && k >= 1) {  // implicit Rayleigh damping of w toward 0 near the top (KWSolve :393-404)
+      const R dampmag = dts * R(D.dampcoef), hdepth = R(D.zdamp), pi = R(0x1.921fb54442d18p+1);  // 4 atan(1)
+      const R htop = (D.ph_save.ld(i, j, nz) + D.phb(i, j, nz)) / R(k::g), hbot = htop - hdepth;
+      const R hk = (s_phs[x] + D.phb(i, j, k)) / R(k::g);
+      R dampwt = 0;
+      if (hk >= hbot) {
+        const R sn = R(cw_sin(double(R(0.5) * pi * (hk - hbot) / hdepth)));
+        dampwt = dampmag * sn * sn;
       }
+      ws = A(R((R(ws) - dampwt * mf_(D, k, R(mut)) * D.w_save.ld(i, j, k)) / (R(1) + dampwt)));
+    }
+    R pn = s_ph[x];
+    if (k >= 1) {
+      pn = R(r + msfA * 0.5 * dtsA * k::g * ope * ws / (D.c1f[k] * sc[3 * CB] + D.c2f[k]));
+      D.ph2.p[o] = pn;
+    }
+    phn = A(pn);
+    D.w2.p[o] = R(ws);
+  }
+  if (mass) s0[x] = phn;
+  lc_bar();
+  if (mass && lm) {  // calc_p_rho (p_rho_point, small_step.cpp:97-112) from the new values of the point
+    const A mu = sc[2 * CB], muts = sc[3 * CB], alt = A(s_alt[x]), tsA = A(s_ts[x]), c2a = A(s_c2a[x]);
+    const A m = D.c1h[k] * muts + A(D.c2h[k]);
+    const A a = -((1. / m) * (alt * (D.c1h[k] * mu) + A(D.rdnw[k]) * (s0[x + CB] - phn)));
+    A pp = c2a * (alt * (A(tnew) - D.c1h[k] * mu * tsA) / (m * (k::t0 + tsA)) - a);
+    const A ptmp = pp;
+    pp = pp + A(D.smdiv) * (pp - A(s_pm1[x]));
+    D.al.p[o] = R(a);
+    D.pm1.p[o] = R(ptmp);
+    D.p.p[o] = R(pp);
   }
 }
 

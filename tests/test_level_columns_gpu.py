@@ -1,0 +1,49 @@
+# SPDX-License-Identifier: GPL-3.0-or-later
+"""The column kernels that run one thread per column and level, at the sizes where their blocks change: level counts
+around whole warps, the smallest and the largest level counts (from nz = 124 on a block holds fewer columns), column
+counts around a block's width, and domains on both sides of the size from which the preparation and finish kernels run
+in blocks of whole rows. The FP64 form equals the oracle bit for bit; every autotuned shape gives the same bits."""
+import numpy as np
+import pytest
+
+from cppwrf_b200 import Domain, capi
+from cases import golden_config, ideal_case, lam_case
+from test_parity_gpu import compare_all, run_pair
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(7, 8, 3), (8, 7, 7), (15, 9, 30), (16, 8, 31), (17, 8, 32), (9, 8, 63),
+                                      (23, 7, 64), (12, 8, 123), (11, 9, 126)])
+def test_lam_levels_and_widths(nx, ny, nz):
+    case = lam_case(nx=nx, ny=ny, nz=nz, n_moist=2, n_scalars=2, seed=nx + nz)
+    dom, orc = run_pair(case, 2)
+    bad = compare_all(dom, orc, case, names=capi.STATE_FIELDS)
+    assert not bad, "\n".join(bad)
+
+
+@pytest.mark.parametrize("nx,nz", [(33, 100), (40, 124), (31, 126)])
+def test_ideal_tall_domains(nx, nz):
+    case = ideal_case(dict(golden_config("warm_bubble"), nx=nx, nz=nz, ztop=100.0 * nz))
+    dom, orc = run_pair(case, 2)
+    bad = compare_all(dom, orc, case, names=capi.STATE_FIELDS)
+    assert not bad, "\n".join(bad)
+
+
+@pytest.mark.parametrize("ny", [246, 252])
+def test_both_sides_of_the_whole_row_blocks(ny):
+    """31 columns (with their last face) are one block of whole rows per row: 247 and 253 of them."""
+    case = lam_case(nx=30, ny=ny, nz=8, n_moist=1, n_scalars=1, seed=2)
+    dom, orc = run_pair(case, 1)
+    bad = compare_all(dom, orc, case, names=capi.STATE_FIELDS)
+    assert not bad, "\n".join(bad)
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("nz", [20, 70, 126])
+def test_every_tuned_shape_gives_the_same_bits(nz, precision):
+    case = lam_case(nx=21, ny=11, nz=nz, n_moist=1, n_scalars=1, seed=nz, precision=precision)
+    a = Domain(case.g, case.o).upload_case(case).set_autotune(True).step(6)
+    b = Domain(case.g, case.o).upload_case(case).step(6)
+    for name in capi.STATE_FIELDS:
+        assert np.array_equal(a.field(name).view(np.uint64), b.field(name).view(np.uint64)), name
