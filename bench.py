@@ -653,8 +653,10 @@ def main():
                                        "k_q_scale_pd", "k_q_update_pd", "k_p_rho_phi")
                              if dom.autotune_choice(k) >= 0},
             "level_chunks": {k: [2, 1, 4][dom.autotune_choice(k)] for k in ("k_q_march",) if dom.autotune_choice(k) >= 0},
-            "column_warps": {k: [8, 16, 4][dom.autotune_choice(k)]
-                             for k in ("k_ls_prep", "k_ss_prep", "k_ac", "k_finish") if dom.autotune_choice(k) >= 0},
+            "column_shapes": {k: (["8 columns", "16 columns", "4 columns"] if k == "k_ac" else
+                                  ["32 columns, 8 warps", "32 columns, 16 warps", "8 columns, a thread per level"])
+                              [dom.autotune_choice(k)]
+                              for k in ("k_ls_prep", "k_ss_prep", "k_ac", "k_finish") if dom.autotune_choice(k) >= 0},
             "clocks": clocks, "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": ebytes,
                                       "d2h_bytes_per_step": ebytes, "steps": n_e2e},
             "gpu_launches": launches, "roofline": roofline, "step_roofline": step_roofline}

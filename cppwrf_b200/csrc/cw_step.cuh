@@ -209,12 +209,13 @@ struct Launcher {
     k_copy<<<unsigned((total + bs - 1) / bs), bs, 0, h->stream>>>(d, int(n), sd);
     check();
   }
-  // the block shape of a point kernel: the one being timed while tuning, else the tuned choice (0 by default)
+  // the block shape of a tunable kernel: the one being timed while tuning, else the tuned choice, else -1 (the launch's
+  // own rule)
   int shape_for(const char* name) const {
     if (h->tuning_shape >= 0) return h->tuning_shape;
     for (const auto& [n, sh] : h->shape_choice)
       if (n == name) return sh;
-    return 0;
+    return -1;
   }
   // a point kernel of fixed shape 0 over the index range kind, one launch per pack
   template <class R, int NM, class K, class... Args>
@@ -235,7 +236,8 @@ struct Launcher {
              Args... args) {
     flush();
     if (plan) return;
-    const int sh = shape_for(name);
+    int sh = shape_for(name);
+    if (sh < 0) sh = 0;
     for (size_t c = 0; c < ps.p.size(); ++c) {
       const int nb = ps.blocks[c][size_t(kind)][size_t(sh)];
       if (nb == 0 || nq == 0) continue;
@@ -250,7 +252,7 @@ struct Launcher {
   void run_q(const char* name, const std::array<K, kNumShapes>& kerns, const Packs<R, NM>& ps, Args... args) {
     flush();
     if (plan) return;
-    const int sh = shape_for(name);
+    const int sh = std::max(0, shape_for(name));
     const size_t smem = q_march_smem<R>(sh);
     CW_CUDA(cudaFuncSetAttribute(kerns[size_t(sh)], cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     for (size_t c = 0; c < ps.p.size(); ++c) {
@@ -268,15 +270,6 @@ struct Launcher {
     if (plan) return;
     static_assert(CX == 32, "a column block's lanes are one warp");
     launch_cb(name, kind, arrays, kern, CNW, ps, args...);
-  }
-  // the same with a tunable warp count (one instantiation per shape: cb_warps(shape) warps per column block)
-  template <class R, int NM, class K, class... Args>
-  void run_cbt(const char* name, int kind, int arrays, const std::array<K, kNumShapes>& kerns, const Packs<R, NM>& ps,
-               Args... args) {
-    flush();
-    if (plan) return;
-    const int sh = shape_for(name);
-    launch_cb(name, kind, arrays, kerns[size_t(sh)], cb_warps(sh), ps, args...);
   }
   template <class R, int NM, class K, class... Args>
   void launch_cb(const char* name, int kind, int arrays, K kern, int nw, const Packs<R, NM>& ps, Args... args) {
@@ -298,20 +291,41 @@ struct Launcher {
               const Packs<R, NM>& ps, Args... args) {
     flush();
     if (plan) return;
-    int sh = shape_for(name);
+    int sh = std::max(0, shape_for(name));
     if (lc_threads(sh, h->nzmax) > kLcMaxThreads) sh = 0;
     if (lc_threads(sh, h->nzmax) > kLcMaxThreads) sh = 2;
+    launch_lc(name, sh, arrays, fields, scalars, kerns[size_t(sh)], ps, args...);
+  }
+  template <class R, int NM, class K, class... Args>
+  void launch_lc(const char* name, int sh, int arrays, int fields, int scalars, K kern, const Packs<R, NM>& ps, Args... args) {
     const int cb = lc_cols(sh);
     const dim3 bs(unsigned(cb), unsigned(lc_threads(sh, h->nzmax) / cb));
     const size_t smem = (size_t(h->nzmax + 1) * (arrays * sizeof(double) + fields * sizeof(R)) + scalars * sizeof(double)) * cb;
-    CW_CUDA(cudaFuncSetAttribute(kerns[size_t(sh)], cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    CW_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     for (size_t c = 0; c < ps.p.size(); ++c) {
       const int nb = ps.blocks[c][size_t(RG_LCOLS_STAG)][size_t(sh)];
       if (nb == 0) continue;
       begin(name);
-      kerns[size_t(sh)]<<<nb, bs, smem, h->stream>>>(ps.p[c], args...);
+      kern<<<nb, bs, smem, h->stream>>>(ps.p[c], args...);
       check();
     }
+  }
+  // A column kernel in its two forms: column blocks of 32 columns x 8 or 16 warps (shapes 0, 1; `arrays` shared level
+  // arrays of doubles) and level-thread columns of 8 (shape 2; `lc_arrays`).
+  template <class R, int NM, class K, class K2, class... Args>
+  void run_col(const char* name, bool recurrence, int arrays, const std::array<K, 2>& wide, int lc_arrays, K2 lc,
+               const Packs<R, NM>& ps, Args... args) {
+    flush();
+    if (plan) return;
+    int sh = shape_for(name);
+    if (sh < 0) {
+      int nb = 0;
+      for (const auto& b : ps.blocks) nb += b[size_t(RG_COLS_STAG)][0];
+      sh = nb < kWideBlocks ? 2 : (recurrence && nb >= kWide16Blocks ? 1 : 0);
+    }
+    if (sh == 2 && lc_threads(0, h->nzmax) > kLcMaxThreads) sh = 1;
+    if (sh == 2) launch_lc(name, 0, lc_arrays, 0, 8, lc, ps, args...);
+    else launch_cb(name, RG_COLS_STAG, arrays, wide[size_t(sh)], cb_warps(sh), ps, args...);
   }
   // one block per member
   template <class R, int NM, class K>
@@ -331,9 +345,6 @@ struct Launcher {
 #define KV_OP(kern, op) std::array{kern<R, NM, 0, op>, kern<R, NM, 1, op>, kern<R, NM, 2, op>}
 // the same with the kernel's part (its fifth template argument)
 #define KV_OP2(kern, op, x) std::array{kern<R, NM, 0, op, x>, kern<R, NM, 1, op, x>, kern<R, NM, 2, op, x>}
-// the three warp-count instantiations of a tunable column kernel
-#define KC(kern) std::array{kern<R, NM, cb_warps(0)>, kern<R, NM, cb_warps(1)>, kern<R, NM, cb_warps(2)>}
-
 template <class R, int NM>
 void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
   const Member& M0 = h->m[0];
@@ -375,7 +386,7 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
     // fill would make them (only the scalars change in between), so only the first stage runs it (the fill merges
     // with the scalars' H_Q2 into one launch: fewer cells, not fewer launches)
     if (rk == 1) L.halo(cw_handle::H_PREP0);
-    L.run_cbt("k_ls_prep", RG_COLS_STAG, 1, KC(k_ls_prep), d);
+    L.run_col("k_ls_prep", true, 1, std::array{k_ls_prep<R, NM, cb_warps(0)>, k_ls_prep<R, NM, cb_warps(1)>}, kLsArrays, k_ls_prep_lc<R, NM, 0>, d);
     L.halo(cw_handle::H_PREP1);
     if (rk == 1 && (dampkm || smag)) {  // DiffusionDriver::prepare: km_opt 4's and damp_opt 1's eddy viscosities
       if (smag) L.run_t("k_smag", RG_MASS, 1, KV(k_smag), d);
@@ -397,7 +408,7 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
     }
     if (h->cfl_on) L.run_t("k_cfl", RG_MASS, 1, KV(k_cfl), d, rk);
     if (rk == 1) L.copy_list(h->zeros_d, h->zeros_start_d, h->zeros.size(), h->zeros_total);
-    L.run_cbt("k_ss_prep", RG_COLS_STAG, 3, KC(k_ss_prep), d, rk);
+    L.run_col("k_ss_prep", true, 3, std::array{k_ss_prep<R, NM, cb_warps(0)>, k_ss_prep<R, NM, cb_warps(1)>}, kSsArrays, k_ss_prep_lc<R, NM, 0>, d, rk);
     if (!spec_all) L.halo(cw_handle::H_SS0);
     for (int it = 1; it <= ns; ++it) {
       L.run_t("k_uv", RG_STAG, 1, KV(k_uv), d, rk);
@@ -407,7 +418,7 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
       if (!spec_all) L.halo(cw_handle::H_AC);
     }
     L.halo(cw_handle::H_POST);
-    L.run_cbt("k_finish", RG_COLS_STAG, 0, KC(k_finish), d, rk, ns);
+    L.run_col("k_finish", false, 0, std::array{k_finish<R, NM, cb_warps(0)>, k_finish<R, NM, cb_warps(1)>}, 1, k_finish_lc<R, NM, 0>, d, rk, ns);
     L.halo(cw_handle::H_FIN);
     if (scalars) {
       if (rk == 1) L.run_t("k_q_tendf_rk1", RG_MASS, nq, KV(k_q_tendf_rk1), d);

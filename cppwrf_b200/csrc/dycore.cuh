@@ -164,17 +164,25 @@ constexpr int PX = 128, PY = 1;
 __host__ __device__ constexpr int shape_x(int s) { return s == 0 ? PX : (s == 1 ? PX / 2 : PX / 4); }
 __host__ __device__ constexpr int shape_y(int s) { return PX / shape_x(s); }
 constexpr int CX = 32, CNW = 8;
-// the column kernels' warp counts the autotuner chooses from (shape s: cb_warps(s) warps; the fewest blocks per SM
-// their launch bound asks for keeps 3 x 256, 2 x 512 and 6 x 128 threads resident)
-__host__ __device__ constexpr int cb_warps(int s) { return s == 0 ? CNW : (s == 1 ? 2 * CNW : CNW / 2); }
-__host__ __device__ constexpr int cb_minblocks(int nw) { return nw == CNW ? 3 : (nw > CNW ? 2 : 6); }
+// a column block's warps (shape s; the fewest blocks per SM their launch bound asks for keeps 3 x 256 and 2 x 512
+// threads resident)
+__host__ __device__ constexpr int cb_warps(int s) { return s == 0 ? CNW : 2 * CNW; }
+__host__ __device__ constexpr int cb_minblocks(int nw) { return nw == CNW ? 3 : 2; }
 // the level-thread column kernels: lc_cols(s) columns per block in shape s; a thread per column and w level (whole warps)
 // and one warp for the columns' recurrences, kLcMaxThreads in all (a narrower shape where nz does not fit)
 __host__ __device__ constexpr int lc_cols(int s) { return s == 0 ? 8 : (s == 1 ? 16 : 4); }
 __host__ __device__ constexpr int lc_threads(int s, int nz) { return (lc_cols(s) * (nz + 1) + 31) / 32 * 32 + 32; }
 constexpr int kLcMaxThreads = 1024;
-// k_ac's shared memory: level arrays of doubles and of the fields' type, per-column scalars
-constexpr int kAcArrays = 5, kAcFields = 13, kAcScalars = 8;
+// Where the preparation and finish kernels change form, in blocks of 32 columns over the launch's rows. Below kWideBlocks
+// (under two such blocks per SM) the latency of a column's levels in turn is what they take, and a thread per level is
+// faster: k_ls_prep, k_ss_prep, k_finish 33 / 49 / 57 -> 11 / 19 / 15 us at 200 x 100 (7 blocks), 17 / 27 / 30 -> 15 / 23
+// / 19 us at 65 x 63 x 40 (192). Above it, their loads and stores are what they take, and rows of 32 columns are: 35 / 41
+// / 47 against 43 / 58 / 43 us at 119 x 89 x 44 (360 blocks), 129 / 185 / 190 against 172 / 248 / 188 at 200 x 200 x 60.
+// From kWide16Blocks on, 16 warps a block instead of 8: 129 against 153 and 185 against 203 us at 200 x 200 x 60.
+constexpr int kWideBlocks = 250, kWide16Blocks = 1000;
+// their shared memory: k_ac's level arrays of doubles and of the fields' type and its per-column scalars, the others'
+// level arrays of doubles
+constexpr int kAcArrays = 5, kAcFields = 13, kAcScalars = 8, kLsArrays = 2, kSsArrays = 5;
 constexpr int kCbArrays = 6;  // shared-memory level arrays of the acoustic column block: kCbArrays x (nz + 2) x CX doubles
 __host__ __device__ __forceinline__ int cdiv(int a, int b) { return (a + b - 1) / b; }
 

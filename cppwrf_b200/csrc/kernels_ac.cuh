@@ -148,28 +148,32 @@ __device__ __forceinline__ double hypso_log(double x) {
   if constexpr (sizeof(R) == 4) return ::log(x);
   else return cw_log(x);
 }
+// from the column masses muts and mu'', phi'' of levels k and k + 1 and theta at the point
 template <class R>
-__device__ __forceinline__ void p_rho_phi_point(const Dom<R>& D, int i, int j, int k) {
+__device__ __forceinline__ void p_rho_phi_val(const Dom<R>& D, int i, int j, int k, R muts, R mu, R ph_k, R ph_kp, R t2) {
   R a;
   if (D.hypsometric_opt == 2) {
     // log-linear in pressure: the total inverse density of the layer is its geopotential thickness over
     // p_mid log(p_bottom / p_top), the dry pressures from the hybrid coefficients; in double in both forms (the
     // perturbation is a small difference of totals)
-    const double m = double(D.muts(i, j, 0)), ptop = D.p_top;
+    const double m = double(muts), ptop = D.p_top;
     const double pfu = D.c3f[k + 1] * m + D.c4f[k + 1] + ptop, pfd = D.c3f[k] * m + D.c4f[k] + ptop;
     const double phm = D.c3h[k] * m + D.c4h[k] + ptop;
-    a = R((double(D.ph2(i, j, k + 1)) - double(D.ph2(i, j, k)) + D.phb64(i, j, k + 1) - D.phb64(i, j, k)) /
-              phm / hypso_log<R>(pfd / pfu) -
+    a = R((double(ph_kp) - double(ph_k) + D.phb64(i, j, k + 1) - D.phb64(i, j, k)) / phm / hypso_log<R>(pfd / pfu) -
           D.alb64(i, j, k));
   } else {
-    a = R(-1) / (R(D.c1h[k]) * D.muts(i, j, 0) + R(D.c2h[k])) *
-        (D.alb(i, j, k) * (R(D.c1h[k]) * D.mu2(i, j, 0)) + R(D.rdnw[k]) * (D.ph2(i, j, k + 1) - D.ph2(i, j, k)));
+    a = R(-1) / (R(D.c1h[k]) * muts + R(D.c2h[k])) * (D.alb(i, j, k) * (R(D.c1h[k]) * mu) + R(D.rdnw[k]) * (ph_kp - ph_k));
   }
-  D.al(i, j, k) = a;
   // the equation of state in double in both forms: p'' is a small difference of totals of ~1e5 Pa (in float the
   // rounding of the total's base, 6e-8, would be ~1e-4 of p'') -- for the FP64 form the same operations
-  const double base = k::r_d * (k::t0 + double(D.t2(i, j, k))) / (k::p1000mb * (double(a) + D.alb64(i, j, k)));
-  D.p(i, j, k) = R(k::p1000mb * eos_pow<R>(base) - D.pb64(i, j, k));
+  const double base = k::r_d * (k::t0 + double(t2)) / (k::p1000mb * (double(a) + D.alb64(i, j, k)));
+  const R p = R(k::p1000mb * eos_pow<R>(base) - D.pb64(i, j, k));
+  D.al(i, j, k) = a;
+  D.p(i, j, k) = p;
+}
+template <class R>
+__device__ __forceinline__ void p_rho_phi_point(const Dom<R>& D, int i, int j, int k) {
+  p_rho_phi_val(D, i, j, k, D.muts(i, j, 0), D.mu2(i, j, 0), D.ph2(i, j, k), D.ph2(i, j, k + 1), D.t2(i, j, k));
 }
 // mode 0: every mass point; 1: calc_p_rho_phi_interior (after spec_bdy_final); 2: after the microphysics, only in
 // the members that have it, on the interior where the member has boundary data (rk3.cpp:146-158)

@@ -18,12 +18,6 @@ namespace cw {
 // the next level can still be issued early)
 #define CB_LOOP_U2(k, n) _Pragma("unroll 2") for (int k = int(threadIdx.y); k < (n); k += NW)
 
-
-// a hint that brings the line of a into L2 (no register, no wait): the column blocks' level loops then meet L2
-// instead of DRAM latency
-__device__ __forceinline__ void pf_l2(const void* a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
-// the levels of a loop split over warps 1 .. NW - 1 (warp 0 runs a recurrence meanwhile)
-#define CB_LOOP_W1(k, n) for (int k = int(threadIdx.y) - 1; threadIdx.y > 0 && k < (n); k += NW - 1)
 // block -> (member, column i of this lane, row j)
 // (ilim: the end of the member's column range along i; the lanes at or past it have no column)
 template <class R, int NM>
@@ -43,70 +37,6 @@ __device__ __forceinline__ const Dom<R>& cb_member(const Pack<R, NM>& P, int kin
 __device__ __forceinline__ double* cb_array(int a, int nz) {
   extern __shared__ double cb_smem[];
   return cb_smem + size_t(a) * (nz + 2) * CX;
-}
-
-// ---- level-thread column kernels: a block holds lc_cols(SH) neighbouring columns along i and one thread per column and
-// w level (threadIdx.x the column, threadIdx.y the level), so that a column's levels are all in flight at once
-template <int SH, class R, int NM>
-__device__ __forceinline__ const Dom<R>& lc_member(const Pack<R, NM>& P, int& i, int& j, int& ilim) {
-  constexpr int CB = lc_cols(SH);
-  const int b = blockIdx.x;
-  const int m = member_of(P, RG_LCOLS_STAG, SH, b);
-  const Dom<R>& D = P.d[m];
-  const Range r = range_of(RG_LCOLS_STAG, D);
-  const int bx = cdiv(r.i1 - r.i0, CB);
-  const int local = b - P.start(RG_LCOLS_STAG, SH, m);
-  i = r.i0 + (local % bx) * CB + int(threadIdx.x);
-  j = r.j0 + local / bx;
-  ilim = r.i1;
-  return D;
-}
-// A column's recurrence over n levels on one thread: step(e, v) in order, e = 0, S, 2 S, ... the element's offset from the
-// arrays' first one and v[a] the element of array a (S = CB upwards, -CB downwards). The values of the next kLcAhead levels
-// are read while the present ones are stepped through, ahead of the stores that the steps make (the compiler may not move
-// a load across those): the chain is then its arithmetic, and not a shared-memory load a level as well. The last
-// read-ahead runs up to 2 kLcAhead - 1 levels past the arrays' last element: the callers' arrays have others of the
-// block's shared memory there.
-constexpr int kLcAhead = 4;
-template <int S, class F, class... T>
-__device__ __forceinline__ void lc_serial(int n, F step, const T*... a) {
-  constexpr int NA = sizeof...(T);
-  double nxt[kLcAhead][NA];
-  auto read = [&](int e) {
-#pragma unroll
-    for (int u = 0; u < kLcAhead; ++u) {
-      int m = 0;
-      ((nxt[u][m++] = double(a[e + u * S])), ...);
-    }
-  };
-  read(0);
-  int e = 0, left = n;
-  for (; left >= kLcAhead; left -= kLcAhead) {
-    double v[kLcAhead][NA];
-#pragma unroll
-    for (int u = 0; u < kLcAhead; ++u)
-#pragma unroll
-      for (int m = 0; m < NA; ++m) v[u][m] = nxt[u][m];
-    read(e + kLcAhead * S);
-#pragma unroll
-    for (int u = 0; u < kLcAhead; ++u) step(e + u * S, v[u]);
-    e += kLcAhead * S;
-  }
-#pragma unroll
-  for (int u = 0; u < kLcAhead - 1; ++u)
-    if (u < left) step(e + u * S, nxt[u]);
-}
-// one element from global to shared memory without a register in between (lc_wait: this thread's copies are done)
-template <class T>
-__device__ __forceinline__ void lc_copy(T* dst, const T* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(sizeof(T)) : "memory");
-}
-__device__ __forceinline__ void lc_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// the block's barrier, reached by its point warps and its column warp at different places of the code
-__device__ __forceinline__ void lc_bar() { asm volatile("bar.sync 0;" ::: "memory"); }
-__device__ __forceinline__ double* lc_smem() {
-  extern __shared__ double cb_smem[];
-  return cb_smem;
 }
 
 // rk_step_prep: KMu (large_step.cpp:49-66), KPrep3 (:68-81), KWW (:83-108), KCq (:127-148)
@@ -334,6 +264,406 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_ss_prep(const __g
     }
     D.alpha(i, j, nz) = R(1. / (s_b[nz * CX + lane] - s_a[nz * CX + lane] * gprev));
     D.gamma(i, j, nz) = 0;
+  }
+}
+
+// small_step_finish (KFinish :419-444, KFinishMu :446-453) + calc_p_rho_phi (KPRhoPhi :456-477)
+template <class R, int NM, int NW = CNW>
+__global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __grid_constant__ Pack<R, NM> P, int rk, int nsmall) {
+  int i, j, ilim;
+  const Dom<R>& D = cb_member(P, RG_COLS_STAG, i, j, ilim);
+  const int nx = D.nx, ny = D.ny, nz = D.nz, nyv = D.nyv;
+  const bool col = i < ilim;  // a column of the member (its faces' range)
+  const bool mass = col && i < nx && j < ny;
+  const R dts = R(rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound);
+  const R hd_dt = (rk == 3 && D.n_moist > 0) ? dts * R(nsmall) : R(0);
+  if (col) {
+    CB_LOOP(k, nz + 1) {  // every load of a level before its first store
+      const bool has_u = j < ny && k < nz, has_v = i < nx && j < nyv && k < nz;
+      const R c1h = k < nz ? R(D.c1h[k]) : R(0), c2h = k < nz ? R(D.c2h[k]) : R(0);
+      R u2 = 0, usv = 0, msfuy = 0, muu = 0, mts_u0 = 0, mts_u1 = 0;
+      if (has_u) {
+        u2 = D.u2(i, j, k);
+        usv = D.u_save.ld(i, j, k);
+        msfuy = D.msfuy(i, j);
+        muu = D.muu.ld(i, j, 0);
+        mts_u0 = D.muts.ld(i, j, 0);
+        mts_u1 = D.muts.ld(i - 1, j, 0);
+      }
+      R v2 = 0, vsv = 0, msfvx = 0, muv = 0, mts_v0 = 0, mts_v1 = 0;
+      if (has_v) {
+        v2 = D.v2(i, j, k);
+        vsv = D.v_save.ld(i, j, k);
+        msfvx = D.msfvx(i, j);
+        muv = D.muv.ld(i, j, 0);
+        mts_v0 = D.muts.ld(i, j, 0);
+        mts_v1 = D.muts.ld(i, j - 1, 0);
+      }
+      R m = 0, mts = 0, w2 = 0, wsv = 0, msfty = 0, ph2 = 0, phsv = 0, ww = 0, ww1 = 0, t2 = 0, tsv = 0, hd = 0;
+      if (mass) {
+        m = D.mut.ld(i, j, 0);
+        mts = D.muts.ld(i, j, 0);
+        w2 = D.w2(i, j, k);
+        wsv = D.w_save.ld(i, j, k);
+        msfty = D.msfty(i, j);
+        ph2 = D.ph2(i, j, k);
+        phsv = D.ph_save.ld(i, j, k);
+        ww = D.ww(i, j, k);
+        ww1 = D.ww1.ld(i, j, k);
+        if (k < nz) {
+          t2 = D.t2(i, j, k);
+          tsv = D.t_save.ld(i, j, k);
+          if (hd_dt != R(0)) hd = D.hd.ld(i, j, k);
+        }
+      }
+      if (has_u) {
+        const R mus_u = R(0.5) * (mts_u0 + mts_u1);
+        D.u2(i, j, k) = (msfuy * u2 + usv * (c1h * muu + c2h)) / (c1h * mus_u + c2h);
+      }
+      if (has_v) {
+        const R mus_v = R(0.5) * (mts_v0 + mts_v1);
+        D.v2(i, j, k) = (msfvx * v2 + vsv * (c1h * muv + c2h)) / (c1h * mus_v + c2h);
+      }
+      if (mass) {
+        D.w2(i, j, k) = (msfty * w2 + wsv * (R(D.c1f[k]) * m + R(D.c2f[k]))) / (R(D.c1f[k]) * mts + R(D.c2f[k]));
+        D.ph2(i, j, k) = ph2 + phsv;
+        D.ww(i, j, k) = ww + ww1;
+        if (k < nz)
+          D.t2(i, j, k) = (t2 - (hd_dt != R(0) ? hd_dt * (c1h * m + c2h) * hd : R(0)) + tsv * (c1h * m + c2h)) / (c1h * mts + c2h);
+      }
+    }
+    if (threadIdx.y == 0) {
+      if (mass) D.mu2(i, j, 0) = D.mu2(i, j, 0) + D.mu_save(i, j, 0);
+      if (j < ny) D.muus(i, j, 0) = R(0.5) * (D.muts.ld(i, j, 0) + D.muts.ld(i - 1, j, 0));
+      if (i < nx && j < nyv) D.muvs(i, j, 0) = R(0.5) * (D.muts.ld(i, j, 0) + D.muts.ld(i, j - 1, 0));
+    }
+  }
+  __syncthreads();
+  if (mass) CB_LOOP(k, nz) p_rho_phi_point(D, i, j, k);
+}
+
+// ---- level-thread column kernels: a block holds lc_cols(SH) neighbouring columns along i and one thread per column and
+// w level (threadIdx.x the column, threadIdx.y the level), so that a column's levels are all in flight at once
+template <int SH, class R, int NM>
+__device__ __forceinline__ const Dom<R>& lc_member(const Pack<R, NM>& P, int& i, int& j, int& ilim) {
+  constexpr int CB = lc_cols(SH);
+  const int b = blockIdx.x;
+  const int m = member_of(P, RG_LCOLS_STAG, SH, b);
+  const Dom<R>& D = P.d[m];
+  const Range r = range_of(RG_LCOLS_STAG, D);
+  const int bx = cdiv(r.i1 - r.i0, CB);
+  const int local = b - P.start(RG_LCOLS_STAG, SH, m);
+  i = r.i0 + (local % bx) * CB + int(threadIdx.x);
+  j = r.j0 + local / bx;
+  ilim = r.i1;
+  return D;
+}
+// A column's recurrence over n levels on one thread: step(e, v) in order, e = 0, S, 2 S, ... the element's offset from the
+// arrays' first one and v[a] the element of array a (S = CB upwards, -CB downwards). The values of the next kLcAhead levels
+// are read while the present ones are stepped through, ahead of the stores that the steps make (the compiler may not move
+// a load across those): the chain is then its arithmetic, and not a shared-memory load a level as well. The last
+// read-ahead runs up to 2 kLcAhead - 1 levels past the arrays' last element: the callers' arrays have others of the
+// block's shared memory there.
+constexpr int kLcAhead = 4;
+template <int S, class F, class... T>
+__device__ __forceinline__ void lc_serial(int n, F step, const T*... a) {
+  constexpr int NA = sizeof...(T);
+  double nxt[kLcAhead][NA];
+  auto read = [&](int e) {
+#pragma unroll
+    for (int u = 0; u < kLcAhead; ++u) {
+      int m = 0;
+      ((nxt[u][m++] = double(a[e + u * S])), ...);
+    }
+  };
+  read(0);
+  int e = 0, left = n;
+  for (; left >= kLcAhead; left -= kLcAhead) {
+    double v[kLcAhead][NA];
+#pragma unroll
+    for (int u = 0; u < kLcAhead; ++u)
+#pragma unroll
+      for (int m = 0; m < NA; ++m) v[u][m] = nxt[u][m];
+    read(e + kLcAhead * S);
+#pragma unroll
+    for (int u = 0; u < kLcAhead; ++u) step(e + u * S, v[u]);
+    e += kLcAhead * S;
+  }
+#pragma unroll
+  for (int u = 0; u < kLcAhead - 1; ++u)
+    if (u < left) step(e + u * S, nxt[u]);
+}
+// one element from global to shared memory without a register in between (lc_wait: this thread's copies are done)
+template <class T>
+__device__ __forceinline__ void lc_copy(T* dst, const T* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(sizeof(T)) : "memory");
+}
+__device__ __forceinline__ void lc_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// the block's barrier, reached by its point warps and its column warp at different places of the code
+__device__ __forceinline__ void lc_bar() { asm volatile("bar.sync 0;" ::: "memory"); }
+__device__ __forceinline__ double* lc_smem() {
+  extern __shared__ double cb_smem[];
+  return cb_smem;
+}
+
+// k_ls_prep as level-thread columns; the column warp runs KWW's column integral and running sum, in the reference's order
+template <class R, int NM, int SH>
+__global__ void __maxnreg__(64) k_ls_prep_lc(const __grid_constant__ Pack<R, NM> P) {
+  constexpr int CB = lc_cols(SH);
+  int i, j, ilim;
+  const Dom<R>& D = lc_member<SH>(P, i, j, ilim);
+  const int c = threadIdx.x, k = threadIdx.y;
+  const int nx = D.nx, ny = D.ny, nz = D.nz, nyv = D.nyv;
+  const int ns = (nz + 1) * CB, x = k * CB + c;
+  double* const s_div = lc_smem();  // the layer's divergence term, then ww of the level above
+  double* const s_c = s_div + ns;   // dnw c1h
+  const bool cell = i < nx && i < ilim && j < ny;
+  if (k >= int(blockDim.y) - 32 / CB) {  // the column warp
+    const bool on = x - (int(blockDim.y) - 32 / CB) * CB < CB && cell;
+    lc_bar();
+    if (on) {  // the column integral, then the running sum: ww of level k + 1 into the slot of the divergence it consumed
+      R dmdt = 0, w = 0;
+      lc_serial<CB>(nz, [&](int, const double* v) { dmdt += R(v[0]); }, s_div + c);
+      double* const d = s_div + c;
+      lc_serial<CB>(nz - 1, [&](int e, const double* v) {
+        w = w - R(v[1]) * dmdt - R(v[0]);
+        d[e] = double(w);
+      }, d, s_c + c);
+    }
+    lc_bar();
+    return;
+  }
+  const bool col = i < ilim && k <= nz, lm = k < nz;  // a column of the member (its faces' range)
+  const bool has_u = col && j < ny && lm, has_v = col && i < nx && j < nyv && lm, has_w = col && cell, has_m = has_w && lm;
+  const int spx = D.spec_x, spy = D.spec_y;
+  const int o = i + j * D.t2.sj + k * D.t2.sk, oU = i + j * D.u2.sj + k * D.u2.sk, oV = i + j * D.v2.sj + k * D.v2.sk;
+  const int o2 = i + j * D.mu2.sj, sj2 = D.mu2.sj;
+  R muu = 0, muv = 0, mut = 0;
+  if (col) {
+    const R* const pm = D.mu2.p + o2;
+    if (cell) mut = __ldg(pm) + D.mub(i, j);
+    if (j < ny) {
+      if (spx && i == 0) muu = R(0.5) * (D.mu2.ld(0, j, 0) + D.mu2.ld(0, j, 0) + D.mub(0, j) + D.mub(0, j));
+      else if (spx && i == nx)
+        muu = R(0.5) * (D.mu2.ld(nx - 1, j, 0) + D.mu2.ld(nx - 1, j, 0) + D.mub(nx - 1, j) + D.mub(nx - 1, j));
+      else muu = R(0.5) * (__ldg(pm) + __ldg(pm - 1) + D.mub(i, j) + D.mub(i - 1, j));
+    }
+    if (i < nx && j < nyv) {
+      if (spy && j == 0) muv = R(0.5) * (D.mu2.ld(i, 0, 0) + D.mu2.ld(i, 0, 0) + D.mub(i, 0) + D.mub(i, 0));
+      else if (spy && j == ny)
+        muv = R(0.5) * (D.mu2.ld(i, ny - 1, 0) + D.mu2.ld(i, ny - 1, 0) + D.mub(i, ny - 1) + D.mub(i, ny - 1));
+      else muv = R(0.5) * (__ldg(pm) + __ldg(pm - sj2) + D.mub(i, j) + D.mub(i, j - 1));
+    }
+    if (k == 0) {
+      if (cell) D.mut.p[o2] = mut;
+      if (j < ny) D.muu.p[i + j * D.muu.sj] = muu;
+      if (i < nx && j < nyv) D.muv.p[i + j * D.muv.sj] = muv;
+    }
+  }
+  if (has_m) {
+    s_div[x] = double(ww_divv(D, i, j, k, ww_mu_u(D, i + 1, j), ww_mu_u(D, i, j), ww_mu_v(D, i, j + 1), ww_mu_v(D, i, j)));
+    s_c[x] = double(R(D.dnw[k]) * R(D.c1h[k]));
+  }
+  lc_bar();
+  // KPrep3 while the column warp integrates (every load of a point before its first store)
+  {
+    const R u2 = has_u ? __ldg(D.u2.p + oU) : R(0), msfuy = has_u ? D.msfuy(i, j) : R(1);
+    const R v2 = has_v ? __ldg(D.v2.p + oV) : R(0), mvxi = has_v ? D.msfvx_inv(i, j) : R(0);
+    const R w2 = has_w ? __ldg(D.w2.p + o) : R(0), msfty = has_w ? D.msfty(i, j) : R(1);
+    R al = 0, alb = 0, phb0 = 0, phb1 = 0, ph0 = 0, ph1 = 0;
+    if (has_m) {
+      al = __ldg(D.al.p + o);
+      alb = D.alb(i, j, k);
+      phb0 = D.phb(i, j, k);
+      phb1 = D.phb(i, j, k + 1);
+      ph0 = __ldg(D.ph2.p + o);
+      ph1 = __ldg(D.ph2.p + o + D.ph2.sk);
+    }
+    if (has_u) D.ru.p[oU] = div_msf(u2 * (R(D.c1h[k]) * muu + R(D.c2h[k])), msfuy);
+    if (has_v) D.rv.p[oV] = v2 * (R(D.c1h[k]) * muv + R(D.c2h[k])) * mvxi;
+    if (has_w) D.rw.p[o] = div_msf(w2 * (R(D.c1f[k]) * mut + R(D.c2f[k])), msfty);
+    if (has_m) {
+      D.alt.p[o] = al + alb;
+      D.php.p[o] = R(0.5) * (phb0 + phb1 + ph0 + ph1);
+    }
+  }
+  if (D.n_moist > 0 && col && lm) {  // KCq: the three sums over species first, then the stores
+    const bool has_q = has_w && k >= 1;
+    R tu = 0, tv = 0, tw = 0;
+    const int sj = D.t2.sj, sk = D.t2.sk;
+    for (int s = 0; s < D.n_moist; ++s) {
+      const R* const q = D.q2[s].p + o;
+      const R q0 = __ldg(q);
+      if (has_u) tu = tu + q0 + __ldg(q - 1);
+      if (has_v) tv = tv + q0 + __ldg(q - sj);
+      if (has_q) tw = tw + q0 + __ldg(q - sk);
+    }
+    if (has_u) D.cqu.p[oU] = R(1) / (R(1) + R(0.5) * tu);
+    if (has_v) D.cqv.p[oV] = R(1) / (R(1) + R(0.5) * tv);
+    if (has_q) D.cqw.p[o] = R(0.5) * tw;
+  }
+  lc_bar();
+  if (has_w) D.ww.p[o] = (k == 0 || k == nz) ? R(0) : R(s_div[x - CB]);
+}
+
+// k_ss_prep as level-thread columns; the column warp runs the forward-elimination factors, a recurrence with a division a level
+template <class R, int NM, int SH>
+__global__ void __maxnreg__(64) k_ss_prep_lc(const __grid_constant__ Pack<R, NM> P, int rk) {
+  using A = double;
+  constexpr int CB = lc_cols(SH);
+  int i, j, ilim;
+  const Dom<R>& D = lc_member<SH>(P, i, j, ilim);
+  const int c = threadIdx.x, k = threadIdx.y;
+  const int nx = D.nx, ny = D.ny, nz = D.nz, nyv = D.nyv;
+  const int ns = (nz + 1) * CB, x = k * CB + c;
+  double* const s_a = lc_smem();     // the coefficients a, b, c of calc_coef_w
+  double* const s_b = s_a + ns;
+  double* const s_c = s_b + ns;
+  double* const s_c2a = s_c + ns;
+  double* const s_ph = s_c2a + ns;  // the new phi''
+  const bool cell = i < nx && i < ilim && j < ny;
+  if (k >= int(blockDim.y) - 32 / CB) {  // the column warp
+    const bool on = x - (int(blockDim.y) - 32 / CB) * CB < CB && cell;
+    lc_bar();
+    lc_bar();
+    if (on) {
+      const int o2 = i + j * D.alpha.sj, sk = D.alpha.sk;
+      R* const pal = D.alpha.p + o2;
+      R* const pga = D.gamma.p + o2;
+      pal[0] = 0;
+      pga[0] = 0;
+      A gprev = 0;
+      int kk = 1;
+      lc_serial<CB>(nz - 1, [&](int, const double* v) {
+        const A al = 1. / (v[1] - v[0] * gprev);
+        pal[kk * sk] = R(al);
+        gprev = A(R(v[2] * A(R(al))));
+        pga[kk * sk] = R(gprev);
+        ++kk;
+      }, s_a + CB + c, s_b + CB + c, s_c + CB + c);
+      pal[nz * sk] = R(1. / (s_b[nz * CB + c] - s_a[nz * CB + c] * gprev));
+      pga[nz * sk] = 0;
+    }
+    return;
+  }
+  const bool col = i < ilim && k <= nz, lm = k < nz, mass = col && cell, first = rk == 1;
+  const bool has_u = col && j < ny && lm, has_v = col && i < nx && j < nyv && lm;
+  const int o = i + j * D.t2.sj + k * D.t2.sk, oU = i + j * D.u2.sj + k * D.u2.sk, oV = i + j * D.v2.sj + k * D.v2.sk;
+  const int o2 = i + j * D.mu2.sj;
+  R mts = 0, mus_u = 0, mus_v = 0, mut = 0, mu_new = 0;
+  R c2a = 0, alt = 1, tnew = 0, ts = 0;
+  A ph_new = 0;
+  if (col) {
+    const R* const pm1 = D.mu1.p + o2;
+    mts = D.mub(i, j) + __ldg(pm1);
+    mus_u = first ? D.muu.ld(i, j, 0) : R(0.5) * (mts + D.mub(i - 1, j) + __ldg(pm1 - 1));
+    mus_v = first ? D.muv.ld(i, j, 0) : R(0.5) * (mts + D.mub(i, j - 1) + __ldg(pm1 - D.mu2.sj));
+    if (mass) {
+      mut = D.mut.ld(i, j, 0);
+      const R mu = D.mu2.p[o2];
+      mu_new = __ldg(pm1) - mu;
+      if (k == 0) D.mu_save.p[o2] = mu;
+    }
+    // KPrep (every load of a point before its first store)
+    const R c1h = lm ? R(D.c1h[k]) : R(0), c2h = lm ? R(D.c2h[k]) : R(0);
+    R ui = 0, u1 = 0, muu = 0, msfuy = 1, vi = 0, v1 = 0, muv = 0, mvxi = 0;
+    if (has_u) {
+      ui = D.u2.p[oU];
+      u1 = __ldg(D.u1.p + oU);
+      muu = D.muu.ld(i, j, 0);
+      msfuy = D.msfuy(i, j);
+    }
+    if (has_v) {
+      vi = D.v2.p[oV];
+      v1 = __ldg(D.v1.p + oV);
+      muv = D.muv.ld(i, j, 0);
+      mvxi = D.msfvx_inv(i, j);
+    }
+    R ti = 0, t1 = 0, pb = 0, pp = 0, wi = 0, w1 = 0, msfty = 1, phi = 0, ph1 = 0, ww = 0;
+    if (mass) {
+      if (lm) {
+        ti = D.t2.p[o];
+        t1 = __ldg(D.t1.p + o);
+        pb = D.pb(i, j, k);
+        pp = D.p.p[o];
+        alt = __ldg(D.alt.p + o);
+      }
+      wi = D.w2.p[o];
+      w1 = __ldg(D.w1.p + o);
+      msfty = D.msfty(i, j);
+      phi = D.ph2.p[o];
+      ph1 = __ldg(D.ph1.p + o);
+      ww = (k == 0 || k == nz) ? R(0) : __ldg(D.ww.p + o);
+    }
+    if (has_u) {
+      D.u_save.p[oU] = ui;
+      D.u2.p[oU] = div_msf(((c1h * mus_u + c2h) * u1 - (c1h * muu + c2h) * ui), msfuy);
+    }
+    if (has_v) {
+      D.v_save.p[oV] = vi;
+      D.v2.p[oV] = ((c1h * mus_v + c2h) * v1 - (c1h * muv + c2h) * vi) * mvxi;
+    }
+    if (mass) {
+      if (lm) {
+        ts = ti;
+        tnew = (c1h * mts + c2h) * t1 - (c1h * mut + c2h) * ti;
+        c2a = R(k::cpovcv) * (pb + pp) / alt;
+        D.t_save.p[o] = ti;
+        D.t2.p[o] = tnew;
+        D.c2a.p[o] = c2a;
+        s_c2a[x] = A(c2a);
+      }
+      const R pn = ph1 - phi;
+      ph_new = A(pn);
+      s_ph[x] = ph_new;
+      D.w_save.p[o] = wi;
+      D.w2.p[o] = div_msf(((R(D.c1f[k]) * mts + R(D.c2f[k])) * w1 - (R(D.c1f[k]) * mut + R(D.c2f[k])) * wi), msfty);
+      D.ph_save.p[o] = phi;
+      D.ph2.p[o] = pn;
+      D.ww1.p[o] = ww;
+    }
+  }
+  lc_bar();
+  if (col && k == 0) {  // after every thread of the column has read mu_2
+    if (mass) {
+      D.muts.p[o2] = mts;
+      D.mu2.p[o2] = mu_new;
+    }
+    if (j < ny) D.muus(i, j, 0) = mus_u;
+    if (i < nx && j < nyv) D.muvs(i, j, 0) = mus_v;
+  }
+  if (mass) {  // calc_coef_w: the coefficients a, b, c of the level
+    const A dts = rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound;
+    const A cof_h = 0.5 * A(R(dts)) * k::g * (1.0 + A(R(D.epssm)));
+    const A cof = A(R(cof_h * cof_h));
+    const A m = A(mut);
+    auto mh = [&](int kk) { return D.c1h[kk] * m + D.c2h[kk]; };
+    auto mf = [&](int kk) { return D.c1f[kk] * m + D.c2f[kk]; };
+    A a = 0, b = 0, cc = 0;
+    if (k == nz) {
+      const A c2a1 = s_c2a[x - CB];
+      a = -2. * cof * (D.rdnw[nz - 1] * D.rdnw[nz - 1]) * c2a1 * (D.top_lid ? 0.0 : 1.0) / (mh(nz - 1) * mf(nz - 1));
+      b = 1. + 2. * cof * (D.rdnw[nz - 1] * D.rdnw[nz - 1]) * c2a1 / (mh(nz - 1) * mf(nz));
+    } else if (k >= 1) {
+      const A c2a1 = s_c2a[x - CB], q1 = A(R(1) / (R(1) + cqw_(D, i, j, k)));
+      if (k >= 2) a = -q1 * cof * D.rdn[k] * D.rdnw[k - 1] * c2a1 / (mh(k - 1) * mf(k - 1));
+      b = 1. + q1 * cof * D.rdn[k] * (D.rdnw[k] * A(c2a) / (mh(k) * mf(k)) + D.rdnw[k - 1] * c2a1 / (mh(k - 1) * mf(k)));
+      cc = -q1 * cof * D.rdn[k] * D.rdnw[k] * A(c2a) / (mh(k) * mf(k + 1));
+    }
+    s_a[x] = A(R(a));
+    s_b[x] = b;
+    s_c[x] = cc;
+    D.a.p[o] = R(a);
+  }
+  lc_bar();
+  if (mass && lm) {  // calc_p_rho (p_rho_point, small_step.cpp:97-112) while the column warp eliminates
+    const A c1h = D.c1h[k], mu = A(mu_new), altA = A(alt), tsA = A(ts);
+    const A m = c1h * A(mts) + A(D.c2h[k]);
+    const A a = -((1. / m) * (altA * (c1h * mu) + A(D.rdnw[k]) * (s_ph[x + CB] - ph_new)));
+    const A pp = A(c2a) * (altA * (A(tnew) - c1h * mu * tsA) / (m * (k::t0 + tsA)) - a);
+    D.al.p[o] = R(a);
+    D.pm1.p[o] = R(pp);
+    D.p.p[o] = R(pp);
   }
 }
 
@@ -687,79 +1017,87 @@ __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int 
   }
 }
 
-// small_step_finish (KFinish :419-444, KFinishMu :446-453) + calc_p_rho_phi (KPRhoPhi :456-477)
-template <class R, int NM, int NW = CNW>
-__global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __grid_constant__ Pack<R, NM> P, int rk, int nsmall) {
+// k_finish as level-thread columns, without recurrences (the column warp is idle); the new phi'' of the level above
+// through shared memory
+template <class R, int NM, int SH>
+__global__ void __maxnreg__(64) k_finish_lc(const __grid_constant__ Pack<R, NM> P, int rk, int nsmall) {
+  constexpr int CB = lc_cols(SH);
   int i, j, ilim;
-  const Dom<R>& D = cb_member(P, RG_COLS_STAG, i, j, ilim);
+  const Dom<R>& D = lc_member<SH>(P, i, j, ilim);
+  const int k = threadIdx.y, x = k * CB + int(threadIdx.x);
   const int nx = D.nx, ny = D.ny, nz = D.nz, nyv = D.nyv;
-  const bool col = i < ilim;  // a column of the member (its faces' range)
-  const bool mass = col && i < nx && j < ny;
+  double* const s_ph = lc_smem();
+  const bool col = i < ilim && k <= nz, lm = k < nz;  // a column of the member (its faces' range)
+  const bool mass = col && i < nx && j < ny, has_u = col && j < ny && lm, has_v = col && i < nx && j < nyv && lm;
   const R dts = R(rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound);
   const R hd_dt = (rk == 3 && D.n_moist > 0) ? dts * R(nsmall) : R(0);
-  if (col) {
-    CB_LOOP(k, nz + 1) {  // every load of a level before its first store
-      const bool has_u = j < ny && k < nz, has_v = i < nx && j < nyv && k < nz;
-      const R c1h = k < nz ? R(D.c1h[k]) : R(0), c2h = k < nz ? R(D.c2h[k]) : R(0);
-      R u2 = 0, usv = 0, msfuy = 0, muu = 0, mts_u0 = 0, mts_u1 = 0;
-      if (has_u) {
-        u2 = D.u2(i, j, k);
-        usv = D.u_save.ld(i, j, k);
-        msfuy = D.msfuy(i, j);
-        muu = D.muu.ld(i, j, 0);
-        mts_u0 = D.muts.ld(i, j, 0);
-        mts_u1 = D.muts.ld(i - 1, j, 0);
-      }
-      R v2 = 0, vsv = 0, msfvx = 0, muv = 0, mts_v0 = 0, mts_v1 = 0;
-      if (has_v) {
-        v2 = D.v2(i, j, k);
-        vsv = D.v_save.ld(i, j, k);
-        msfvx = D.msfvx(i, j);
-        muv = D.muv.ld(i, j, 0);
-        mts_v0 = D.muts.ld(i, j, 0);
-        mts_v1 = D.muts.ld(i, j - 1, 0);
-      }
-      R m = 0, mts = 0, w2 = 0, wsv = 0, msfty = 0, ph2 = 0, phsv = 0, ww = 0, ww1 = 0, t2 = 0, tsv = 0, hd = 0;
-      if (mass) {
-        m = D.mut.ld(i, j, 0);
-        mts = D.muts.ld(i, j, 0);
-        w2 = D.w2(i, j, k);
-        wsv = D.w_save.ld(i, j, k);
-        msfty = D.msfty(i, j);
-        ph2 = D.ph2(i, j, k);
-        phsv = D.ph_save.ld(i, j, k);
-        ww = D.ww(i, j, k);
-        ww1 = D.ww1.ld(i, j, k);
-        if (k < nz) {
-          t2 = D.t2(i, j, k);
-          tsv = D.t_save.ld(i, j, k);
-          if (hd_dt != R(0)) hd = D.hd.ld(i, j, k);
-        }
-      }
-      if (has_u) {
-        const R mus_u = R(0.5) * (mts_u0 + mts_u1);
-        D.u2(i, j, k) = (msfuy * u2 + usv * (c1h * muu + c2h)) / (c1h * mus_u + c2h);
-      }
-      if (has_v) {
-        const R mus_v = R(0.5) * (mts_v0 + mts_v1);
-        D.v2(i, j, k) = (msfvx * v2 + vsv * (c1h * muv + c2h)) / (c1h * mus_v + c2h);
-      }
-      if (mass) {
-        D.w2(i, j, k) = (msfty * w2 + wsv * (R(D.c1f[k]) * m + R(D.c2f[k]))) / (R(D.c1f[k]) * mts + R(D.c2f[k]));
-        D.ph2(i, j, k) = ph2 + phsv;
-        D.ww(i, j, k) = ww + ww1;
-        if (k < nz)
-          D.t2(i, j, k) = (t2 - (hd_dt != R(0) ? hd_dt * (c1h * m + c2h) * hd : R(0)) + tsv * (c1h * m + c2h)) / (c1h * mts + c2h);
+  const int o = i + j * D.t2.sj + k * D.t2.sk, oU = i + j * D.u2.sj + k * D.u2.sk, oV = i + j * D.v2.sj + k * D.v2.sk;
+  const int o2 = i + j * D.mu2.sj;
+  const R* const pms = D.muts.p + o2;
+  R mts = 0, mu_new = 0, tnew = 0, pn = 0;
+  if (col) {  // every load of a point before its first store
+    const R c1h = lm ? R(D.c1h[k]) : R(0), c2h = lm ? R(D.c2h[k]) : R(0);
+    mts = __ldg(pms);
+    R u2 = 0, usv = 0, msfuy = 0, muu = 0, mts_im = 0;
+    if (has_u) {
+      u2 = D.u2.p[oU];
+      usv = __ldg(D.u_save.p + oU);
+      msfuy = D.msfuy(i, j);
+      muu = D.muu.ld(i, j, 0);
+      mts_im = __ldg(pms - 1);
+    }
+    R v2 = 0, vsv = 0, msfvx = 0, muv = 0, mts_jm = 0;
+    if (has_v) {
+      v2 = D.v2.p[oV];
+      vsv = __ldg(D.v_save.p + oV);
+      msfvx = D.msfvx(i, j);
+      muv = D.muv.ld(i, j, 0);
+      mts_jm = __ldg(pms - D.mu2.sj);
+    }
+    R m = 0, w2 = 0, wsv = 0, msfty = 0, ph2 = 0, phsv = 0, ww = 0, ww1 = 0, t2 = 0, tsv = 0, hd = 0;
+    if (mass) {
+      m = D.mut.ld(i, j, 0);
+      mu_new = D.mu2.p[o2] + __ldg(D.mu_save.p + o2);
+      w2 = D.w2.p[o];
+      wsv = __ldg(D.w_save.p + o);
+      msfty = D.msfty(i, j);
+      ph2 = D.ph2.p[o];
+      phsv = __ldg(D.ph_save.p + o);
+      ww = D.ww.p[o];
+      ww1 = __ldg(D.ww1.p + o);
+      if (lm) {
+        t2 = D.t2.p[o];
+        tsv = __ldg(D.t_save.p + o);
+        if (hd_dt != R(0)) hd = __ldg(D.hd.p + o);
       }
     }
-    if (threadIdx.y == 0) {
-      if (mass) D.mu2(i, j, 0) = D.mu2(i, j, 0) + D.mu_save(i, j, 0);
-      if (j < ny) D.muus(i, j, 0) = R(0.5) * (D.muts.ld(i, j, 0) + D.muts.ld(i - 1, j, 0));
-      if (i < nx && j < nyv) D.muvs(i, j, 0) = R(0.5) * (D.muts.ld(i, j, 0) + D.muts.ld(i, j - 1, 0));
+    if (has_u) {
+      const R mus_u = R(0.5) * (mts + mts_im);
+      D.u2.p[oU] = (msfuy * u2 + usv * (c1h * muu + c2h)) / (c1h * mus_u + c2h);
+    }
+    if (has_v) {
+      const R mus_v = R(0.5) * (mts + mts_jm);
+      D.v2.p[oV] = (msfvx * v2 + vsv * (c1h * muv + c2h)) / (c1h * mus_v + c2h);
+    }
+    if (mass) {
+      D.w2.p[o] = (msfty * w2 + wsv * (R(D.c1f[k]) * m + R(D.c2f[k]))) / (R(D.c1f[k]) * mts + R(D.c2f[k]));
+      pn = ph2 + phsv;
+      D.ph2.p[o] = pn;
+      s_ph[x] = double(pn);
+      D.ww.p[o] = ww + ww1;
+      if (lm) {
+        tnew = (t2 - (hd_dt != R(0) ? hd_dt * (c1h * m + c2h) * hd : R(0)) + tsv * (c1h * m + c2h)) / (c1h * mts + c2h);
+        D.t2.p[o] = tnew;
+      }
+    }
+    if (k == 0) {
+      if (j < ny) D.muus(i, j, 0) = R(0.5) * (mts + __ldg(pms - 1));
+      if (i < nx && j < nyv) D.muvs(i, j, 0) = R(0.5) * (mts + __ldg(pms - D.mu2.sj));
     }
   }
   __syncthreads();
-  if (mass) CB_LOOP(k, nz) p_rho_phi_point(D, i, j, k);
+  if (mass && k == 0) D.mu2.p[o2] = mu_new;  // after every thread of the column has read it
+  if (mass && lm) p_rho_phi_val(D, i, j, k, mts, mu_new, pn, R(s_ph[x + CB]), tnew);
 }
 
 // DiffusionDriver::prepare with damp_opt 1 (diffusion_driver.cpp:114-130): the horizontal eddy viscosities start at
