@@ -363,12 +363,13 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
   const Member& M0 = h->m[0];
   bool lbc = false, terrain = false, scalars = false, any_pd = false, mp = false, open = false, dampkm = false,
        smag = false, any_plain = false;
-  // every member specified on all four sides: the acoustic substeps read no halo cell of the fields the
-  // per-substep fills (H_SS0, H_UV, H_AC) would refresh (the faces next to the boundary are the spec
-  // zone's, updated from the boundary data), and the fills after the substeps (H_POST, H_FIN) refresh them
-  // before anything reads them; those fills, and the spec zone's zero-gradient w of every substep but the
-  // last (overwritten by the next one, read only after the substeps), are left out
-  bool spec_all = h->decomp_px * h->decomp_py <= 1;  // a decomposed domain takes every fill: its patches read each other's points
+  // The acoustic substeps take the points past a domain's edge from the domain itself (edge_lo, edge_hi, face_hi, edge_col),
+  // so the fills before and between them (H_SS0, H_UV, H_AC) are left out and the fills after them (H_POST, H_FIN) refresh
+  // those halos before anything reads them. A decomposed domain runs them: its patches read each other's points there.
+  const bool dec = h->decomp_px * h->decomp_py > 1;
+  // every member specified on all four sides: the spec zone's zero-gradient w of every substep but the last (overwritten by
+  // the next one, read only after the substeps) is left out
+  bool spec_all = !dec;
   int nq = 0;  // the most species of a member
   for (const Member& M : h->m) {
     spec_all &= M.o.lbc != 0 && flat_x(M.g) && flat_y(M.g) && !two_d(M.g);
@@ -422,16 +423,19 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
     if (h->cfl_on) L.run_t("k_cfl", RG_MASS, 1, KV(k_cfl), d, rk);
     if (rk == 1) L.copy_list(h->zeros_d, h->zeros_start_d, h->zeros.size(), h->zeros_total);
     L.run_col("k_ss_prep", true, 3, std::array{k_ss_prep<R, NM, cb_warps(0)>, k_ss_prep<R, NM, cb_warps(1)>}, kSsArrays, k_ss_prep_lc<R, NM, 0>, d, rk);
-    if (!spec_all) L.halo(cw_handle::H_SS0);
+    if (dec) L.halo(cw_handle::H_SS0);
     for (int it = 1; it <= ns; ++it) {
       L.run_t("k_uv", RG_STAG, 1, KV(k_uv), d, rk);
-      if (!spec_all) L.halo(cw_handle::H_UV);
+      if (dec) L.halo(cw_handle::H_UV);
       L.run_lc("k_ac", kAcArrays, kAcFields, kAcScalars, KV(k_ac), d, rk, it, ns);
       if (lbc && (!spec_all || it == ns)) L.run("k_ring", RG_RING, k_ring<R, NM>, d, int(RO_ZERO_GRAD_W), rk);
-      if (!spec_all) L.halo(cw_handle::H_AC);
+      if (dec) L.halo(cw_handle::H_AC);
     }
-    L.halo(cw_handle::H_POST);
+    // (k_finish reads mu_ts past the edge as the substeps do: elsewhere than on specified domains its fill waits for the
+    // one after it, in one launch)
+    if (dec || spec_all) L.halo(cw_handle::H_POST);
     L.run_col("k_finish", false, 0, std::array{k_finish<R, NM, cb_warps(0)>, k_finish<R, NM, cb_warps(1)>}, 1, k_finish_lc<R, NM, 0>, d, rk, ns);
+    if (!dec && !spec_all) L.halo(cw_handle::H_POST);
     L.halo(cw_handle::H_FIN);
     if (scalars) {
       if (rk == 1) L.run_t("k_q_tendf_rk1", RG_MASS, nq, KV(k_q_tendf_rk1), d);

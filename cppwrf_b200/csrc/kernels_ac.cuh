@@ -58,82 +58,120 @@ __device__ __forceinline__ void p_rho_point(const Dom<R>& D, int i, int j, int k
   p_rho_point_ph<RO>(D, i, j, k, damp, D.ph2(i, j, k), D.ph2(i, j, k + 1));
 }
 
-// advance_uv (KUV :151-190): the faces i, j of cells i, j
-template <class R, int DI, int DJ>
-__device__ __forceinline__ R uv_dpn(const Dom<R>& D, int i, int j, int k) {
-  auto ps = [&](int kk) { return D.p.ld(i, j, kk) + D.p.ld(i - DI, j - DJ, kk); };
-  const int nz = D.nz;
-  if (k == 0) return R(0.5) * (R(D.cf1) * ps(0) + R(D.cf2) * ps(1) + R(D.cf3) * ps(2));
-  if (k == nz) return D.top_lid ? R(0.5) * (R(D.cf1) * ps(nz - 1) + R(D.cf2) * ps(nz - 2) + R(D.cf3) * ps(nz - 3)) : R(0);
-  return R(0.5) * (R(D.fnm[k]) * ps(k) + R(D.fnp[k]) * ps(k - 1));
+// The acoustic substeps read the fields that they advance at most one point away, so at the domain's edges they take the
+// point that a halo fill would copy instead of running the fill: the element offset from mass point 0 (n - 1) to the
+// point before (after) it -- the wrapped point of a periodic side, the outermost point itself of a symmetric, specified or
+// open one -- and from face n - 1 to face n.
+__device__ __forceinline__ int edge_lo(int i, int n, int bc) { return i > 0 ? -1 : (bc == CW_BC_PERIODIC ? n - 1 : 0); }
+__device__ __forceinline__ int edge_hi(int i, int n, int bc) { return i < n - 1 ? 1 : (bc == CW_BC_PERIODIC ? 1 - n : 0); }
+// the column of the domain whose value a halo fill copies to column i of an even mass field (n <= i < n + 1, i = -1)
+__device__ __forceinline__ int edge_col(int i, int n, int bc) {
+  return i < 0 ? (bc == CW_BC_PERIODIC ? n - 1 : 0) : (i < n ? i : (bc == CW_BC_PERIODIC ? 0 : n - 1));
 }
-template <class R, int DI, int DJ>
-__device__ __forceinline__ R uv_dp(const Dom<R>& D, int i, int j, int k, R mface, R rd, R rm) {
-  const R c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
+__device__ __forceinline__ int face_hi(int i, int n, int bc) { return i < n - 1 || bc != CW_BC_PERIODIC ? 1 : 1 - n; }
+
+// advance_uv (KUV :151-190): the horizontal pressure gradient force between the point's column and the one before it.
+// C: the point's own values; om, o2m: the neighbour's element in 3-D and 2-D mass fields; alts, dpb, dphp: the sum of alt
+// and the differences of pb and php, whose halos are current throughout the substeps
+template <class R>
+struct UvPoint {
+  int o, k, sk;
+  R p0, pm, pp, ph0, ph1, al, mu;  // p of levels k, k - 1, k + 1; phi'' of levels k, k + 1
+  __device__ __forceinline__ UvPoint(const Dom<R>& D, int o_, int o2, int k_) : o(o_), k(k_), sk(D.t2.sk) {
+    const R* const q = D.p.p + o;
+    p0 = __ldg(q);
+    pm = k > 0 ? __ldg(q - sk) : R(0);
+    pp = k + 1 < D.nz ? __ldg(q + sk) : R(0);
+    ph0 = __ldg(D.ph2.p + o);
+    ph1 = __ldg(D.ph2.p + o + sk);
+    al = __ldg(D.al.p + o);
+    mu = __ldg(D.mu2.p + o2);
+  }
+};
+template <class R>
+__device__ __forceinline__ R uv_dp(const Dom<R>& D, const UvPoint<R>& C, int om, int o2m, R alts, R dpb, R dphp, R mface,
+                                   R rd, R rm, R c1h, R c2h) {
+  const int k = C.k, nz = D.nz;
+  const R* const q = D.p.p + om;
+  const R p0 = __ldg(q), ph0 = __ldg(D.ph2.p + om), ph1 = __ldg(D.ph2.p + om + C.sk), al = __ldg(D.al.p + om);
+  const R mu = __ldg(D.mu2.p + o2m);
+  const R ps = C.p0 + p0;
+  const R psm = k > 0 ? C.pm + __ldg(q - C.sk) : R(0), psp = k + 1 < nz ? C.pp + __ldg(q + C.sk) : R(0);
   R d = rm * R(0.5) * rd * (c1h * mface + c2h) *
-        (((D.ph2.ld(i, j, k + 1) - D.ph2.ld(i - DI, j - DJ, k + 1)) + (D.ph2.ld(i, j, k) - D.ph2.ld(i - DI, j - DJ, k))) +
-         (D.alt.ld(i, j, k) + D.alt.ld(i - DI, j - DJ, k)) * (D.p.ld(i, j, k) - D.p.ld(i - DI, j - DJ, k)) +
-         (D.al.ld(i, j, k) + D.al.ld(i - DI, j - DJ, k)) * (D.pb(i, j, k) - D.pb(i - DI, j - DJ, k)));
-  d += rm * rd * (D.php.ld(i, j, k) - D.php.ld(i - DI, j - DJ, k)) *
-       (R(D.rdnw[k]) * (uv_dpn<R, DI, DJ>(D, i, j, k + 1) - uv_dpn<R, DI, DJ>(D, i, j, k)) -
-        R(0.5) * (c1h * D.mu2.ld(i - DI, j - DJ, 0) + c1h * D.mu2.ld(i, j, 0)));
+        (((C.ph1 - ph1) + (C.ph0 - ph0)) + alts * (C.p0 - p0) + (C.al + al) * dpb);
+  R lo, hi;  // p'' at w levels k and k + 1
+  if (k == 0) {
+    lo = R(0.5) * (R(D.cf1) * ps + R(D.cf2) * psp + R(D.cf3) * (__ldg(D.p.p + C.o + 2 * C.sk) + __ldg(q + 2 * C.sk)));
+  } else {
+    lo = R(0.5) * (R(D.fnm[k]) * ps + R(D.fnp[k]) * psm);
+  }
+  if (k + 1 == nz) {
+    hi = R(0);
+    if (D.top_lid)
+      hi = R(0.5) * (R(D.cf1) * ps + R(D.cf2) * psm + R(D.cf3) * (__ldg(D.p.p + C.o - 2 * C.sk) + __ldg(q - 2 * C.sk)));
+  } else {
+    hi = R(0.5) * (R(D.fnm[k + 1]) * psp + R(D.fnp[k + 1]) * ps);
+  }
+  d += rm * rd * dphp * (R(D.rdnw[k]) * (hi - lo) - R(0.5) * (c1h * mu + c1h * C.mu));
   return d;
 }
 // over the staggered index range; with lateral boundaries the spec zone's faces take
 // u += dts ru_tend (LateralBC::update_uv, lateral_bc.cpp:353-361) instead, and so do the faces of open boundaries
-// (no pressure gradient or divergence damping on them, :175-184)
+// (no pressure gradient or divergence damping on them, :175-184). Bound by the latency of its loads: every value that the
+// two faces share is loaded once, from one offset per storage class. Registers: 64 in double (at 48 it spills: 36.7
+// against 31.9 us at 119 x 89 x 44, where the form that indexed each field for itself took 31.3), 48 in float (22.3 us; 26.0
+// before; 300 x 300 x 60: 221 -> 175 us).
 template <class R, int NM, int SH>
-__global__ void __launch_bounds__(PX, 10) k_uv(const __grid_constant__ Pack<R, NM> P, int rk) {
+__global__ void __launch_bounds__(PX, sizeof(R) == 8 ? 8 : 10) k_uv(const __grid_constant__ Pack<R, NM> P, int rk) {
   const Dom<R>* Dp;
   int i, j, k;
   if (!thread_index<SH>(P, RG_STAG, Dp, i, j, k)) return;
   const Dom<R>& D = *Dp;
+  const int nx = D.nx, ny = D.ny;
   if (k >= D.nz) return;
   const R dts = R(rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound);
-  // both new values are computed before either store (the stores cannot alias the loads then)
-  bool su = false, sv = false;
-  R un = 0, vn = 0;
+  const int oU = i + j * D.u2.sj + k * D.u2.sk, oV = i + j * D.v2.sj + k * D.v2.sk;
+  // the faces of the spec zone and of open sides; the faces that the pressure gradient moves
+  bool hu = false, hv = false;
   if (D.lbc) {
     int sl, pos;
-    if (spec_at(ring_for(D.nx, D.ny, 'u'), i, j, sl, pos)) {
-      un = D.u2(i, j, k) + dts * D.ru_tend.ld(i, j, k);
-      su = true;
-    }
-    if (spec_at(ring_for(D.nx, D.ny, 'v'), i, j, sl, pos)) {
-      vn = D.v2(i, j, k) + dts * D.rv_tend.ld(i, j, k);
-      sv = true;
-    }
+    hu = spec_at(ring_for(nx, ny, 'u'), i, j, sl, pos);
+    hv = spec_at(ring_for(nx, ny, 'v'), i, j, sl, pos);
   }
-  if (D.open_x && (i == 0 || i == D.nx) && j < D.ny) {
-    un = D.u2(i, j, k) + dts * D.ru_tend.ld(i, j, k);
-    su = true;
-  }
-  if (D.do_y && D.open_y && (j == 0 || j == D.ny) && i < D.nx) {
-    vn = D.v2(i, j, k) + dts * D.rv_tend.ld(i, j, k);
-    sv = true;
-  }
-  if (i < D.nx && j < D.ny) {
-    const int ui0 = D.bc_x != CW_BC_PERIODIC ? 1 : 0, ui1 = D.nx;
-    const int vj0 = (D.bc_y != CW_BC_PERIODIC && D.do_y) ? 1 : 0, vj1 = D.ny;
-    const R emdx = R(D.emdiv) * (R(1.) / R(D.rdx)), emdy = D.do_y ? R(D.emdiv) * (R(1.) / R(D.rdy)) : R(0);
-    const R c1h = R(D.c1h[k]);
-    if (i >= ui0 && i < ui1 && !edge_uface(D, i, j)) {
-      const R mudf_x = div_msf(-emdx * (D.mudf.ld(i, j, 0) - D.mudf.ld(i - 1, j, 0)), D.msfuy(i, j));
-      un = D.u2(i, j, k) + dts * D.ru_tend.ld(i, j, k) -
-           dts * cqu_(D, i, j, k) * uv_dp<R, 1, 0>(D, i, j, k, D.muu.ld(i, j, 0), R(D.rdx), div_msf(D.msfux(i, j), D.msfuy(i, j))) +
-           c1h * mudf_x;
-      su = true;
+  if (D.open_x && (i == 0 || i == nx) && j < ny) hu = true;
+  if (D.do_y && D.open_y && (j == 0 || j == ny) && i < nx) hv = true;
+  const bool cell = i < nx && j < ny;
+  const bool gu = cell && (i > 0 || D.bc_x == CW_BC_PERIODIC) && !edge_uface(D, i, j);
+  const bool gv = cell && D.do_y && (j > 0 || D.bc_y == CW_BC_PERIODIC) && !edge_vface(D, i, j);
+  // both new values are computed before either store (the stores cannot alias the loads then)
+  R un = 0, vn = 0;
+  if (hu || gu) un = D.u2.p[oU] + dts * __ldg(D.ru_tend.p + oU);
+  if (hv || gv) vn = D.v2.p[oV] + dts * __ldg(D.rv_tend.p + oV);
+  if (gu || gv) {
+    const int sj = D.t2.sj, o = i + j * sj + k * D.t2.sk, o2 = i + j * sj;
+    const R c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
+    const UvPoint<R> C(D, o, o2, k);
+    const R alt = __ldg(D.alt.p + o), php = __ldg(D.php.p + o), pb = D.pb(i, j, k), mudf = __ldg(D.mudf.p + o2);
+    if (gu) {
+      const int m = edge_lo(i, nx, D.bc_x);
+      const R msfuy = D.msfuy(i, j);
+      const R emdx = R(D.emdiv) * (R(1.) / R(D.rdx));
+      const R mudf_x = div_msf(-emdx * (mudf - __ldg(D.mudf.p + o2 + m)), msfuy);
+      const R dp = uv_dp(D, C, o + m, o2 + m, alt + __ldg(D.alt.p + o - 1), pb - D.pb(i - 1, j, k),
+                         php - __ldg(D.php.p + o - 1), D.muu.ld(i, j, 0), R(D.rdx), div_msf(D.msfux(i, j), msfuy), c1h, c2h);
+      un = un - dts * (D.n_moist > 0 ? __ldg(D.cqu.p + oU) : R(1)) * dp + c1h * mudf_x;
     }
-    if (D.do_y && j >= vj0 && j < vj1 && !edge_vface(D, i, j)) {
-      const R mudf_y = -emdy * (D.mudf.ld(i, j, 0) - D.mudf.ld(i, j - 1, 0)) * D.msfvx_inv(i, j);
-      vn = D.v2(i, j, k) + dts * D.rv_tend.ld(i, j, k) -
-           dts * cqv_(D, i, j, k) * uv_dp<R, 0, 1>(D, i, j, k, D.muv.ld(i, j, 0), R(D.rdy), div_msf(D.msfvy(i, j), D.msfvx(i, j))) +
-           c1h * mudf_y;
-      sv = true;
+    if (gv) {
+      const int m = edge_lo(j, ny, D.bc_y) * sj;
+      const R emdy = R(D.emdiv) * (R(1.) / R(D.rdy));
+      const R mudf_y = -emdy * (mudf - __ldg(D.mudf.p + o2 + m)) * D.msfvx_inv(i, j);
+      const R dp = uv_dp(D, C, o + m, o2 + m, alt + __ldg(D.alt.p + o - sj), pb - D.pb(i, j - 1, k),
+                         php - __ldg(D.php.p + o - sj), D.muv.ld(i, j, 0), R(D.rdy), div_msf(D.msfvy(i, j), D.msfvx(i, j)), c1h, c2h);
+      vn = vn - dts * (D.n_moist > 0 ? __ldg(D.cqv.p + oV) : R(1)) * dp + c1h * mudf_y;
     }
   }
-  if (su) D.u2(i, j, k) = un;
-  if (sv) D.v2(i, j, k) = vn;
+  if (hu || gu) D.u2.p[oU] = un;
+  if (hv || gv) D.v2.p[oV] = vn;
 }
 
 // calc_p_rho_phi (KPRhoPhi :456-477) at (i, j, k); pow and log in double: cw_pow / cw_log in the FP64 form

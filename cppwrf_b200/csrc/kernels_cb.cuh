@@ -277,6 +277,8 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __gr
   const bool mass = col && i < nx && j < ny;
   const R dts = R(rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound);
   const R hd_dt = (rk == 3 && D.n_moist > 0) ? dts * R(nsmall) : R(0);
+  // mu_ts of the neighbour columns: past the domain's edge the column that a halo fill would copy
+  auto mts_at = [&](int ii, int jj) { return D.muts.ld(edge_col(ii, nx, D.bc_x), edge_col(jj, ny, D.bc_y), 0); };
   if (col) {
     CB_LOOP(k, nz + 1) {  // every load of a level before its first store
       const bool has_u = j < ny && k < nz, has_v = i < nx && j < nyv && k < nz;
@@ -287,8 +289,8 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __gr
         usv = D.u_save.ld(i, j, k);
         msfuy = D.msfuy(i, j);
         muu = D.muu.ld(i, j, 0);
-        mts_u0 = D.muts.ld(i, j, 0);
-        mts_u1 = D.muts.ld(i - 1, j, 0);
+        mts_u0 = mts_at(i, j);
+        mts_u1 = mts_at(i - 1, j);
       }
       R v2 = 0, vsv = 0, msfvx = 0, muv = 0, mts_v0 = 0, mts_v1 = 0;
       if (has_v) {
@@ -296,8 +298,8 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __gr
         vsv = D.v_save.ld(i, j, k);
         msfvx = D.msfvx(i, j);
         muv = D.muv.ld(i, j, 0);
-        mts_v0 = D.muts.ld(i, j, 0);
-        mts_v1 = D.muts.ld(i, j - 1, 0);
+        mts_v0 = mts_at(i, j);
+        mts_v1 = mts_at(i, j - 1);
       }
       R m = 0, mts = 0, w2 = 0, wsv = 0, msfty = 0, ph2 = 0, phsv = 0, ww = 0, ww1 = 0, t2 = 0, tsv = 0, hd = 0;
       if (mass) {
@@ -334,8 +336,8 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __gr
     }
     if (threadIdx.y == 0) {
       if (mass) D.mu2(i, j, 0) = D.mu2(i, j, 0) + D.mu_save(i, j, 0);
-      if (j < ny) D.muus(i, j, 0) = R(0.5) * (D.muts.ld(i, j, 0) + D.muts.ld(i - 1, j, 0));
-      if (i < nx && j < nyv) D.muvs(i, j, 0) = R(0.5) * (D.muts.ld(i, j, 0) + D.muts.ld(i, j - 1, 0));
+      if (j < ny) D.muus(i, j, 0) = R(0.5) * (mts_at(i, j) + mts_at(i - 1, j));
+      if (i < nx && j < nyv) D.muvs(i, j, 0) = R(0.5) * (mts_at(i, j) + mts_at(i, j - 1));
     }
   }
   __syncthreads();
@@ -729,8 +731,8 @@ __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int 
       A ws = 0;
       if (!D.flat) {
         const A cf1 = D.cf1, cf2 = D.cf2, cf3 = D.cf3;
-        auto U = [&](int ii, int kk) { return A(D.u2.ld(ii, j, kk)); };
-        auto V = [&](int jj, int kk) { return A(D.v2.ld(i, jj, kk)); };
+        auto U = [&](int ii, int kk) { return A(D.u2.ld(ii > i ? i + face_hi(i, nx, D.bc_x) : i, j, kk)); };
+        auto V = [&](int jj, int kk) { return A(D.v2.ld(i, jj > j ? j + face_hi(j, ny, D.bc_y) : j, kk)); };
         auto H = [&](int ii, int jj) { return A(D.ht(ii, jj)); };
         ws = A(D.msftx(i, j)) * 0.5 * D.rdx *
              ((H(i + 1, j) - H(i, j)) * (cf1 * U(i + 1, 0) + cf2 * U(i + 1, 1) + cf3 * U(i + 1, 2)) +
@@ -870,17 +872,17 @@ __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int 
       const R cu = div_msf((c1h * muu + c2h) * usv, msfuy);
       const R cv = (c1h * muv + c2h) * vsv * mvxi;
       if (dyn) {
-        const R u_ip = __ldg(D.u2.p + oU + 1), usv_ip = __ldg(D.u_save.p + oU + 1), muu_ip = __ldg(D.muu.p + oU2 + 1);
+        const R u_ip = __ldg(D.u2.p + oU + face_hi(i, nx, D.bc_x)), usv_ip = __ldg(D.u_save.p + oU + 1), muu_ip = __ldg(D.muu.p + oU2 + 1);
         const R msfuy_ip = D.msfuy(i + 1, j);
         const R* const pts = D.t_save.p + o;
-        const R ts = __ldg(pts), ts_ip = __ldg(pts + 1), ts_im = __ldg(pts - 1);
+        const R ts = __ldg(pts), ts_ip = __ldg(pts + edge_hi(i, nx, D.bc_x)), ts_im = __ldg(pts + edge_lo(i, nx, D.bc_x));
         const R fx = (u_ip + div_msf((c1h * muu_ip + c2h) * usv_ip, msfuy_ip)) - (u_k + cu);
         R d = R(D.rdx) * fx;
         hflux = R(0.5) * R(D.rdx) * (u_ip * (ts_ip + ts) - u_k * (ts + ts_im));
         if (D.do_y) {
-          const R v_jp = __ldg(D.v2.p + oV + sjV), vsv_jp = __ldg(D.v_save.p + oV + sjV);
+          const R v_jp = __ldg(D.v2.p + oV + face_hi(j, ny, D.bc_y) * sjV), vsv_jp = __ldg(D.v_save.p + oV + sjV);
           const R muv_jp = __ldg(D.muv.p + oV2 + D.muv.sj), mvxi_jp = D.msfvx_inv(i, j + 1);
-          const R ts_jp = __ldg(pts + sjM), ts_jm = __ldg(pts - sjM);
+          const R ts_jp = __ldg(pts + edge_hi(j, ny, D.bc_y) * sjM), ts_jm = __ldg(pts + edge_lo(j, ny, D.bc_y) * sjM);
           d += R(D.rdy) * ((v_jp + (c1h * muv_jp + c2h) * vsv_jp * mvxi_jp) - (v_k + cv));
           hflux += R(0.5) * R(D.rdy) * (v_jp * (ts_jp + ts) - v_k * (ts + ts_jm));
         }
@@ -1033,18 +1035,19 @@ __global__ void __maxnreg__(64) k_finish_lc(const __grid_constant__ Pack<R, NM> 
   const R hd_dt = (rk == 3 && D.n_moist > 0) ? dts * R(nsmall) : R(0);
   const int o = i + j * D.t2.sj + k * D.t2.sk, oU = i + j * D.u2.sj + k * D.u2.sk, oV = i + j * D.v2.sj + k * D.v2.sk;
   const int o2 = i + j * D.mu2.sj;
-  const R* const pms = D.muts.p + o2;
+  // mu_ts of the neighbour columns: past the domain's edge the column that a halo fill would copy
+  auto mts_at = [&](int ii, int jj) { return D.muts.ld(edge_col(ii, nx, D.bc_x), edge_col(jj, ny, D.bc_y), 0); };
   R mts = 0, mu_new = 0, tnew = 0, pn = 0;
   if (col) {  // every load of a point before its first store
     const R c1h = lm ? R(D.c1h[k]) : R(0), c2h = lm ? R(D.c2h[k]) : R(0);
-    mts = __ldg(pms);
+    mts = mts_at(i, j);
     R u2 = 0, usv = 0, msfuy = 0, muu = 0, mts_im = 0;
     if (has_u) {
       u2 = D.u2.p[oU];
       usv = __ldg(D.u_save.p + oU);
       msfuy = D.msfuy(i, j);
       muu = D.muu.ld(i, j, 0);
-      mts_im = __ldg(pms - 1);
+      mts_im = mts_at(i - 1, j);
     }
     R v2 = 0, vsv = 0, msfvx = 0, muv = 0, mts_jm = 0;
     if (has_v) {
@@ -1052,7 +1055,7 @@ __global__ void __maxnreg__(64) k_finish_lc(const __grid_constant__ Pack<R, NM> 
       vsv = __ldg(D.v_save.p + oV);
       msfvx = D.msfvx(i, j);
       muv = D.muv.ld(i, j, 0);
-      mts_jm = __ldg(pms - D.mu2.sj);
+      mts_jm = mts_at(i, j - 1);
     }
     R m = 0, w2 = 0, wsv = 0, msfty = 0, ph2 = 0, phsv = 0, ww = 0, ww1 = 0, t2 = 0, tsv = 0, hd = 0;
     if (mass) {
@@ -1091,8 +1094,8 @@ __global__ void __maxnreg__(64) k_finish_lc(const __grid_constant__ Pack<R, NM> 
       }
     }
     if (k == 0) {
-      if (j < ny) D.muus(i, j, 0) = R(0.5) * (mts + __ldg(pms - 1));
-      if (i < nx && j < nyv) D.muvs(i, j, 0) = R(0.5) * (mts + __ldg(pms - D.mu2.sj));
+      if (j < ny) D.muus(i, j, 0) = R(0.5) * (mts + mts_at(i - 1, j));
+      if (i < nx && j < nyv) D.muvs(i, j, 0) = R(0.5) * (mts + mts_at(i, j - 1));
     }
   }
   __syncthreads();
