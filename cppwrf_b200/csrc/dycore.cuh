@@ -148,6 +148,25 @@ __device__ __forceinline__ int member_of(const Pack<R, NM>& P, int kind, int sha
   }
 }
 
+// The member of a column kernel's block: a single domain's descriptor stays in the constant bank; a batch's is copied into
+// the block's shared memory, from where no store of the kernel makes the compiler load it again (an ensemble of five
+// members, 2.7 M points, mixed: k_ac 402 -> 350 us, k_ss_prep 238 -> 219, k_finish 202 -> 175). Not in the point kernels,
+// whose blocks are too short for the copy (k_q_tendf_rk1 227 -> 278 us). Called by every thread of the block.
+template <class R, int NM>
+__device__ __forceinline__ const Dom<R>& dom_of(const Pack<R, NM>& P, int m) {
+  if constexpr (NM == 1) {
+    return P.d[0];
+  } else {
+    __shared__ __align__(16) unsigned char sd[sizeof(Dom<R>)];
+    static_assert(sizeof(Dom<R>) % 8 == 0);
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(P.d + m);
+    const int nt = blockDim.x * blockDim.y, t = threadIdx.y * blockDim.x + threadIdx.x;
+    for (int n = t; n < int(sizeof(Dom<R>) / 8); n += nt) reinterpret_cast<unsigned long long*>(sd)[n] = __ldg(src + n);
+    __syncthreads();
+    return *reinterpret_cast<const Dom<R>*>(sd);
+  }
+}
+
 // x / m for a map factor m. In IEEE arithmetic x / 1 is x exactly, so the division is skipped when m == 1 with the
 // same bits as its result: an unmapped domain's map factors are all 1, and its divisions by them cost a compare.
 template <class X>

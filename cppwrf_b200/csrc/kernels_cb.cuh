@@ -24,7 +24,7 @@ template <class R, int NM>
 __device__ __forceinline__ const Dom<R>& cb_member(const Pack<R, NM>& P, int kind, int& i, int& j, int& ilim) {
   const int b = blockIdx.x;
   const int m = member_of(P, kind, 0, b);
-  const Dom<R>& D = P.d[m];
+  const Dom<R>& D = dom_of(P, m);
   const Range r = range_of(kind, D);
   const int bx = cdiv(r.i1 - r.i0, CX);
   const int local = b - P.start(kind, 0, m);
@@ -351,7 +351,7 @@ __device__ __forceinline__ const Dom<R>& lc_member(const Pack<R, NM>& P, int& i,
   constexpr int CB = lc_cols(SH);
   const int b = blockIdx.x;
   const int m = member_of(P, RG_LCOLS_STAG, SH, b);
-  const Dom<R>& D = P.d[m];
+  const Dom<R>& D = dom_of(P, m);
   const Range r = range_of(RG_LCOLS_STAG, D);
   const int bx = cdiv(r.i1 - r.i0, CB);
   const int local = b - P.start(RG_LCOLS_STAG, SH, m);
