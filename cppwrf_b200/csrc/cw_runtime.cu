@@ -89,7 +89,8 @@ Plan plan_member(Member& M) {
     for (int n = 0; n < M.o.n_scalars; ++n)
       for (int f = 0; f < 6; ++f) P.qpd.push_back(take(field_bytes(M.Lpd[f / 2], M.esz)));
   }
-  P.vert = take(24 * size_t(M.g.nz + 2) * sizeof(double));
+  // the vertical arrays in double and, in the mixed form, after them in float
+  P.vert = take(24 * size_t(M.g.nz + 2) * (sizeof(double) + (M.esz == 4 ? sizeof(float) : 0)));
   for (int v = 0; v < 5; ++v) {
     size_t n = 0;
     if (M.o.lbc)
@@ -197,6 +198,22 @@ Dom<R> make_dom(cw_handle* h, size_t mi, V3<R>* qtab_d, Slabs<R>* lbcq_d) {
   D.znu = va(VA_ZNU); D.znw = va(VA_ZNW); D.dnw = va(VA_DNW); D.dn = va(VA_DN); D.rdnw = va(VA_RDNW); D.rdn = va(VA_RDN);
   D.fnm = va(VA_FNM); D.fnp = va(VA_FNP); D.c1h = va(VA_C1H); D.c2h = va(VA_C2H); D.c1f = va(VA_C1F); D.c2f = va(VA_C2F);
   D.u_base = va(VA_UB); D.v_base = va(VA_VB); D.fcx = va(VA_FCX); D.gcx = va(VA_GCX);
+  {  // the constants in the fields' type
+    const R* vr;
+    if constexpr (sizeof(R) == 8) vr = v;
+    else vr = reinterpret_cast<const R*>(v + 24 * size_t(g.nz + 2));
+    auto vf = [&](int a) { return vr + M.vert_off[a]; };
+    D.dt3 = g.dt / 3.0;
+    D.dtsn = g.dt / M.n_sound;
+    Consts<R>& r = D.r;
+    r.dnw = vf(VA_DNW); r.rdnw = vf(VA_RDNW); r.rdn = vf(VA_RDN); r.fnm = vf(VA_FNM); r.fnp = vf(VA_FNP);
+    r.c1h = vf(VA_C1H); r.c2h = vf(VA_C2H); r.c1f = vf(VA_C1F); r.c2f = vf(VA_C2F);
+    r.rdx = R(D.rdx); r.rdy = R(D.rdy); r.cf1 = R(D.cf1); r.cf2 = R(D.cf2); r.cf3 = R(D.cf3); r.cfn = R(D.cfn); r.cfn1 = R(D.cfn1);
+    r.hup = R(D.hup); r.vup = R(D.vup); r.epssm = R(D.epssm);
+    r.emdx = R(D.emdiv) * (R(1.) / r.rdx);
+    r.emdy = D.do_y ? R(D.emdiv) * (R(1.) / r.rdy) : R(0);
+    r.dt = R(D.dt); r.dt2 = R(0.5 * D.dt); r.dt3 = R(D.dt3); r.dts = R(D.dtsn);
+  }
   D.t_base = va(VA_TB); D.z_base = va(VA_ZB);
   D.c3h = va(VA_C3H); D.c4h = va(VA_C4H); D.c3f = va(VA_C3F); D.c4f = va(VA_C4F);
   D.hypsometric_opt = o.hypsometric_opt; D.p_top = g.p_top;
@@ -1646,6 +1663,11 @@ int cw_member_set_vertical(cw_handle* h, int mi, const cw_vertical* v) {
       }
     }
     CW_CUDA(cudaMemcpyAsync(M.vert, buf.data(), buf.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    std::vector<float> bf;
+    if (M.esz == 4) {
+      bf.assign(buf.begin(), buf.end());
+      CW_CUDA(cudaMemcpyAsync(M.vert + buf.size(), bf.data(), bf.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+    }
     CW_CUDA(cudaStreamSynchronize(h->stream));
     M.cf1 = v->cf1; M.cf2 = v->cf2; M.cf3 = v->cf3; M.cfn = v->cfn; M.cfn1 = v->cfn1; M.rdx = v->rdx; M.rdy = v->rdy;
     M.g.p_top = v->p_top;

@@ -35,6 +35,26 @@ struct VB {  // BView3 / BView2 (field.hpp:35-44): si = sj = 0 for horizontally 
   __device__ __forceinline__ T operator()(int i, int j) const { return __ldg(p + (i * si + j * sj)); }
 };
 
+// A 1-D array over levels that no kernel writes: read through the read-only path
+template <class T>
+struct Lev {
+  const T* p;
+  Lev() = default;
+  Lev(const T* q) : p(q) {}
+  __device__ __forceinline__ T operator[](int k) const { return __ldg(p + k); }
+  __host__ __device__ operator const T*() const { return p; }
+};
+// The vertical arrays, grid constants and time steps in the fields' own type R, rounded once on the host: in the mixed form
+// a conversion from double in the kernels, an eighth of an instruction's rate each, is otherwise made by every point of
+// every launch (k_uv made 38, and a division of the time step in double). The same values: the FP64 form's are the doubles.
+template <class R>
+struct Consts {
+  Lev<R> dnw, rdnw, rdn, fnm, fnp, c1h, c2h, c1f, c2f;
+  R rdx, rdy, cf1, cf2, cf3, cfn, cfn1, hup, vup, epssm;
+  R emdx, emdy;          // emdiv / rdx, emdiv / rdy as emdiv (1 / rdx)
+  R dt, dt2, dt3, dts;   // the time step, a half and a third of it, the acoustic one
+};
+
 // Lateral boundary slabs of one variable: 4 sides of values then 4 of tendencies, (pos, k, b) pos fastest
 template <class T>
 struct Slabs {
@@ -47,6 +67,7 @@ struct Slabs {
 
 template <class T>
 struct Dom {
+  using R = T;
   // grid and options
   int nx, ny, nz, nyv, two_d, do_y;
   // the mass points this member computes, pi0 <= i < pi1, pj0 <= j < pj1, in the domain's indices: the whole domain,
@@ -69,7 +90,10 @@ struct Dom {
   double* dtbc;  // device scalar: time since the boundary data (LateralBC::dtbc), advanced on the device
   unsigned long long* cfl;  // per RK stage: the vertical and horizontal CFL maxima (bits of positive doubles)
   double rdx, rdy, cf1, cf2, cf3, cfn, cfn1;
-  const double *znu, *znw, *dnw, *dn, *rdnw, *rdn, *fnm, *fnp, *c1h, *c2h, *c1f, *c2f, *u_base, *v_base;
+  double dt3, dtsn;  // dt / 3, dt / n_sound
+  Consts<R> r;
+  const double *znu, *znw, *dn, *u_base, *v_base;
+  Lev<double> dnw, rdnw, rdn, fnm, fnp, c1h, c2h, c1f, c2f;
   const double *fcx, *gcx;  // relaxation weights per row (LateralBC::set_dt)
   const double *t_base, *z_base;  // BaseState 1-D profiles (damp_opt 2's base state)
   const double *c3h, *c4h, *c3f, *c4f;  // hybrid coefficients of the dry pressure (hypsometric_opt 2)

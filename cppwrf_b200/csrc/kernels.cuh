@@ -264,10 +264,10 @@ __device__ __forceinline__ R ww_mu_v(const Dom<R>& D, int i, int j) {
 }
 template <class R>
 __device__ __forceinline__ R ww_divv(const Dom<R>& D, int i, int j, int k, R mu1, R mu0, R mv1, R mv0) {
-  const R c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
-  return D.msftx(i, j) * R(D.dnw[k]) *
-         (R(D.rdx) * (div_msf((c1h * mu1 + c2h) * D.u2.ld(i + 1, j, k), D.msfuy(i + 1, j)) - div_msf((c1h * mu0 + c2h) * D.u2.ld(i, j, k), D.msfuy(i, j))) +
-          R(D.rdy) * ((c1h * mv1 + c2h) * D.v2.ld(i, j + 1, k) * D.msfvx_inv(i, j + 1) -
+  const R c1h = D.r.c1h[k], c2h = D.r.c2h[k];
+  return D.msftx(i, j) * D.r.dnw[k] *
+         (D.r.rdx * (div_msf((c1h * mu1 + c2h) * D.u2.ld(i + 1, j, k), D.msfuy(i + 1, j)) - div_msf((c1h * mu0 + c2h) * D.u2.ld(i, j, k), D.msfuy(i, j))) +
+          D.r.rdy * ((c1h * mv1 + c2h) * D.v2.ld(i, j + 1, k) * D.msfvx_inv(i, j + 1) -
                       (c1h * mv0 + c2h) * D.v2.ld(i, j, k) * D.msfvx_inv(i, j)));
 }
 
@@ -284,8 +284,8 @@ __device__ __forceinline__ R cqw_(const Dom<R>& D, int i, int j, int k) { return
 // MapC::vxgm (large_step.cpp:121-124): the curvature factor at mass point (i, j, k) from u, v and the map factors
 template <class R>
 __device__ __forceinline__ R vxgm(const Dom<R>& D, int i, int j, int k) {
-  return R(0.5) * (D.u2.ld(i, j, k) + D.u2.ld(i + 1, j, k)) * (D.msfvx(i, j + 1) - D.msfvx(i, j)) * R(D.rdy) -
-         R(0.5) * (D.v2.ld(i, j, k) + D.v2.ld(i, j + 1, k)) * (D.msfuy(i + 1, j) - D.msfuy(i, j)) * R(D.rdx);
+  return R(0.5) * (D.u2.ld(i, j, k) + D.u2.ld(i + 1, j, k)) * (D.msfvx(i, j + 1) - D.msfvx(i, j)) * D.r.rdy -
+         R(0.5) * (D.v2.ld(i, j, k) + D.v2.ld(i, j + 1, k)) * (D.msfuy(i + 1, j) - D.msfuy(i, j)) * D.r.rdx;
 }
 // KTendU (large_step.cpp:152-264)
 template <class R>
@@ -300,40 +300,40 @@ __device__ R tu_fx(const Dom<R>& D, int i, int j, int k) {
     return R(0.25) * (D.ru.ld(i, j, k) + D.ru.ld(i - 1, j, k)) * (D.u2.ld(i - 1, j, k) + ub);
   }
   const R vel = R(0.5) * (D.ru.ld(i, j, k) + D.ru.ld(i - 1, j, k));
-  if (o == 3) return vel * flux3(D.u2.ld(i - 2, j, k), D.u2.ld(i - 1, j, k), D.u2.ld(i, j, k), D.u2.ld(i + 1, j, k), vel, R(D.hup));
+  if (o == 3) return vel * flux3(D.u2.ld(i - 2, j, k), D.u2.ld(i - 1, j, k), D.u2.ld(i, j, k), D.u2.ld(i + 1, j, k), vel, D.r.hup);
   return vel * flux5(D.u2.ld(i - 3, j, k), D.u2.ld(i - 2, j, k), D.u2.ld(i - 1, j, k), D.u2.ld(i, j, k), D.u2.ld(i + 1, j, k),
-                     D.u2.ld(i + 2, j, k), vel, R(D.hup));
+                     D.u2.ld(i + 2, j, k), vel, D.r.hup);
 }
 template <class R>
 __device__ R tu_fy(const Dom<R>& D, int i, int j, int k) {
   const int o = ord_face(j, D.ny, D.spec_y);
   if (o == 2) return R(0.25) * (D.rv.ld(i, j, k) + D.rv.ld(i - 1, j, k)) * (D.u2.ld(i, j, k) + D.u2.ld(i, j - 1, k));
   const R vel = R(0.5) * (D.rv.ld(i, j, k) + D.rv.ld(i - 1, j, k));
-  if (o == 3) return vel * flux3(D.u2.ld(i, j - 2, k), D.u2.ld(i, j - 1, k), D.u2.ld(i, j, k), D.u2.ld(i, j + 1, k), vel, R(D.hup));
+  if (o == 3) return vel * flux3(D.u2.ld(i, j - 2, k), D.u2.ld(i, j - 1, k), D.u2.ld(i, j, k), D.u2.ld(i, j + 1, k), vel, D.r.hup);
   return vel * flux5(D.u2.ld(i, j - 3, k), D.u2.ld(i, j - 2, k), D.u2.ld(i, j - 1, k), D.u2.ld(i, j, k), D.u2.ld(i, j + 1, k),
-                     D.u2.ld(i, j + 2, k), vel, R(D.hup));
+                     D.u2.ld(i, j + 2, k), vel, D.r.hup);
 }
 template <class R>
 __device__ R tu_fz(const Dom<R>& D, int i, int j, int k) {
   if (k == 0 || k == D.nz) return 0;
   const R vel = R(0.5) * (D.ww.ld(i - 1, j, k) + D.ww.ld(i, j, k));
-  if (k == 1 || k == D.nz - 1) return vel * (R(D.fnm[k]) * D.u2.ld(i, j, k) + R(D.fnp[k]) * D.u2.ld(i, j, k - 1));
-  return vel * flux3(D.u2.ld(i, j, k - 2), D.u2.ld(i, j, k - 1), D.u2.ld(i, j, k), D.u2.ld(i, j, k + 1), -vel, R(D.vup));
+  if (k == 1 || k == D.nz - 1) return vel * (D.r.fnm[k] * D.u2.ld(i, j, k) + D.r.fnp[k] * D.u2.ld(i, j, k - 1));
+  return vel * flux3(D.u2.ld(i, j, k - 2), D.u2.ld(i, j, k - 1), D.u2.ld(i, j, k), D.u2.ld(i, j, k + 1), -vel, D.r.vup);
 }
 template <class R, int DI, int DJ>
 __device__ __forceinline__ R pgf_dpn(const Dom<R>& D, int i, int j, int k) {  // p' at w level k, face column
   auto ps = [&](int kk) { return D.p.ld(i - DI, j - DJ, kk) + D.p.ld(i, j, kk); };
   const int nz = D.nz;
-  if (k == 0) return R(0.5) * (R(D.cf1) * ps(0) + R(D.cf2) * ps(1) + R(D.cf3) * ps(2));
-  if (k == nz) return D.top_lid ? R(0.5) * (R(D.cfn) * ps(nz - 1) + R(D.cfn1) * ps(nz - 2)) : R(0);
-  return R(0.5) * (R(D.fnm[k]) * ps(k) + R(D.fnp[k]) * ps(k - 1));
+  if (k == 0) return R(0.5) * (D.r.cf1 * ps(0) + D.r.cf2 * ps(1) + D.r.cf3 * ps(2));
+  if (k == nz) return D.top_lid ? R(0.5) * (D.r.cfn * ps(nz - 1) + D.r.cfn1 * ps(nz - 2)) : R(0);
+  return R(0.5) * (D.r.fnm[k] * ps(k) + D.r.fnp[k] * ps(k - 1));
 }
 // advect_u open_ys / open_ye (KTendU::open_y_term, :193-208): the v-flux terms of the outermost rows
 template <class R>
 __device__ R tu_open_y(const Dom<R>& D, int i, int j, int k) {
   const int imin = 0, imax = D.nx - 1;
   const int ip = i < imax ? i : imax, im = i - 1 > imin ? i - 1 : imin;
-  const R mrdy = D.msfux(i, j) * R(D.rdy);
+  const R mrdy = D.msfux(i, j) * D.r.rdy;
   if (j == 0) {
     const R vw = R(0.5) * (D.rv.ld(ip, 0, k) + D.rv.ld(im, 0, k));
     const R vb = vw < R(0) ? vw : R(0);
@@ -350,7 +350,7 @@ __device__ R tu_open_y(const Dom<R>& D, int i, int j, int k) {
 // unless y is open too, and the held tendency
 template <class R>
 __device__ R tend_u_open_face(const Dom<R>& D, int i, int j, int k, bool use_tendf) {
-  const R rdx = R(D.rdx), c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
+  const R rdx = D.r.rdx, c1h = D.r.c1h[k], c2h = D.r.c2h[k];
   R t;
   if (i == 0) {
     R ub = D.ru.ld(0, j, k) - R(k::cb) * (c1h * D.mut.ld(0, j, 0) + c2h);
@@ -361,28 +361,28 @@ __device__ R tend_u_open_face(const Dom<R>& D, int i, int j, int k, bool use_ten
     ub = ub > R(0) ? ub : R(0);
     t = R(0) - rdx * ub * (D.u2.ld(i, j, k) - D.u2.ld(i - 1, j, k));
   }
-  if (!D.open_y) t -= R(D.rdnw[k]) * (tu_fz(D, i, j, k + 1) - tu_fz(D, i, j, k));
+  if (!D.open_y) t -= D.r.rdnw[k] * (tu_fz(D, i, j, k + 1) - tu_fz(D, i, j, k));
   if (use_tendf) t += div_msf(D.ru_tendf.ld(i, j, k), D.msfuy(i, j));
   return t;
 }
 // OP: the kernel variant for packs with an open boundary (the checks compile away in the other)
 template <bool OP, class R>
 __device__ R tend_u(const Dom<R>& D, int i, int j, int k, bool use_tendf, R fx0, R fx1, R fy0, R fy1) {
-  const R rdx = R(D.rdx), rdy = R(D.rdy);
-  const R c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
+  const R rdx = D.r.rdx, rdy = D.r.rdy;
+  const R c1h = D.r.c1h[k], c2h = D.r.c2h[k];
   R t = -(D.msfux(i, j) * rdx) * (fx1 - fx0);
   if (D.do_y) {  // open_ys / ye: the outermost rows take the open terms instead of the y flux divergence
     if (!(OP && D.open_y && (j == 0 || j == D.ny - 1))) t -= (D.msfux(i, j) * rdy) * (fy1 - fy0);
     else t -= tu_open_y(D, i, j, k);
   }
-  if (!(OP && D.open_y && D.spec_x && (i == 0 || i == D.nx))) t -= R(D.rdnw[k]) * (tu_fz(D, i, j, k + 1) - tu_fz(D, i, j, k));
+  if (!(OP && D.open_y && D.spec_x && (i == 0 || i == D.nx))) t -= D.r.rdnw[k] * (tu_fz(D, i, j, k + 1) - tu_fz(D, i, j, k));
   const R rm = div_msf(D.msfux(i, j), D.msfuy(i, j));
   R dpx = rm * R(0.5) * rdx * (c1h * D.muu.ld(i, j, 0) + c2h) *
           ((D.ph2.ld(i, j, k + 1) - D.ph2.ld(i - 1, j, k + 1) + D.ph2.ld(i, j, k) - D.ph2.ld(i - 1, j, k)) +
            (D.alt.ld(i, j, k) + D.alt.ld(i - 1, j, k)) * (D.p.ld(i, j, k) - D.p.ld(i - 1, j, k)) +
            (D.al.ld(i, j, k) + D.al.ld(i - 1, j, k)) * (D.pb(i, j, k) - D.pb(i - 1, j, k)));
   dpx += rm * rdx * (D.php.ld(i, j, k) - D.php.ld(i - 1, j, k)) *
-         (R(D.rdnw[k]) * (pgf_dpn<R, 1, 0>(D, i, j, k + 1) - pgf_dpn<R, 1, 0>(D, i, j, k)) -
+         (D.r.rdnw[k] * (pgf_dpn<R, 1, 0>(D, i, j, k + 1) - pgf_dpn<R, 1, 0>(D, i, j, k)) -
           R(0.5) * (c1h * D.mu2.ld(i - 1, j, 0) + c1h * D.mu2.ld(i, j, 0)));
   t -= cqu_(D, i, j, k) * dpx;
   const R rw4 = R(0.25) * (D.rw.ld(i - 1, j, k + 1) + D.rw.ld(i - 1, j, k) + D.rw.ld(i, j, k + 1) + D.rw.ld(i, j, k));
@@ -405,9 +405,9 @@ __device__ R tv_fx(const Dom<R>& D, int i, int j, int k) {
   const int o = ord_face(i, D.nx, D.spec_x);
   if (o == 2) return R(0.25) * (D.ru.ld(i, j, k) + D.ru.ld(i, j - 1, k)) * (D.v2.ld(i, j, k) + D.v2.ld(i - 1, j, k));
   const R vel = R(0.5) * (D.ru.ld(i, j, k) + D.ru.ld(i, j - 1, k));
-  if (o == 3) return vel * flux3(D.v2.ld(i - 2, j, k), D.v2.ld(i - 1, j, k), D.v2.ld(i, j, k), D.v2.ld(i + 1, j, k), vel, R(D.hup));
+  if (o == 3) return vel * flux3(D.v2.ld(i - 2, j, k), D.v2.ld(i - 1, j, k), D.v2.ld(i, j, k), D.v2.ld(i + 1, j, k), vel, D.r.hup);
   return vel * flux5(D.v2.ld(i - 3, j, k), D.v2.ld(i - 2, j, k), D.v2.ld(i - 1, j, k), D.v2.ld(i, j, k), D.v2.ld(i + 1, j, k),
-                     D.v2.ld(i + 2, j, k), vel, R(D.hup));
+                     D.v2.ld(i + 2, j, k), vel, D.r.hup);
 }
 template <class R>
 __device__ R tv_fy(const Dom<R>& D, int i, int j, int k) {
@@ -421,16 +421,16 @@ __device__ R tv_fy(const Dom<R>& D, int i, int j, int k) {
     return R(0.25) * (D.rv.ld(i, j, k) + D.rv.ld(i, j - 1, k)) * (vb + D.v2.ld(i, j - 1, k));
   }
   const R vel = R(0.5) * (D.rv.ld(i, j, k) + D.rv.ld(i, j - 1, k));
-  if (o == 3) return vel * flux3(D.v2.ld(i, j - 2, k), D.v2.ld(i, j - 1, k), D.v2.ld(i, j, k), D.v2.ld(i, j + 1, k), vel, R(D.hup));
+  if (o == 3) return vel * flux3(D.v2.ld(i, j - 2, k), D.v2.ld(i, j - 1, k), D.v2.ld(i, j, k), D.v2.ld(i, j + 1, k), vel, D.r.hup);
   return vel * flux5(D.v2.ld(i, j - 3, k), D.v2.ld(i, j - 2, k), D.v2.ld(i, j - 1, k), D.v2.ld(i, j, k), D.v2.ld(i, j + 1, k),
-                     D.v2.ld(i, j + 2, k), vel, R(D.hup));
+                     D.v2.ld(i, j + 2, k), vel, D.r.hup);
 }
 template <class R>
 __device__ R tv_fz(const Dom<R>& D, int i, int j, int k) {
   if (k == 0 || k == D.nz) return 0;
   const R vel = R(0.5) * (D.ww.ld(i, j - 1, k) + D.ww.ld(i, j, k));
-  if (k == 1 || k == D.nz - 1) return vel * (R(D.fnm[k]) * D.v2.ld(i, j, k) + R(D.fnp[k]) * D.v2.ld(i, j, k - 1));
-  return vel * flux3(D.v2.ld(i, j, k - 2), D.v2.ld(i, j, k - 1), D.v2.ld(i, j, k), D.v2.ld(i, j, k + 1), -vel, R(D.vup));
+  if (k == 1 || k == D.nz - 1) return vel * (D.r.fnm[k] * D.v2.ld(i, j, k) + D.r.fnp[k] * D.v2.ld(i, j, k - 1));
+  return vel * flux3(D.v2.ld(i, j, k - 2), D.v2.ld(i, j, k - 1), D.v2.ld(i, j, k), D.v2.ld(i, j, k + 1), -vel, D.r.vup);
 }
 // advect_v open_xs / open_xe (KTendV::open_x_term, :307-323): the u-flux terms of the outermost columns
 template <class R>
@@ -438,14 +438,14 @@ __device__ R tv_open_x(const Dom<R>& D, int i, int j, int k) {
   const int jmin = 0, jmax = D.ny - 1;
   const int jp = j < jmax ? j : jmax, jm = j - 1 > jmin ? j - 1 : jmin;
   if (i == 0) {
-    const R mrdx = D.msfvy(0, j) * R(D.rdx);
+    const R mrdx = D.msfvy(0, j) * D.r.rdx;
     const R uw = R(0.5) * (D.ru.ld(0, jp, k) + D.ru.ld(0, jm, k));
     const R ub = uw < R(0) ? uw : R(0);
     const R dup = D.ru.ld(1, jp, k) - D.ru.ld(0, jp, k), dum = D.ru.ld(1, jm, k) - D.ru.ld(0, jm, k);
     return mrdx * (ub * (D.v2.ld(1, j, k) - D.v2.ld(0, j, k)) + R(0.5) * D.v2.ld(0, j, k) * (dup + dum));
   }
   const int ie = D.nx;
-  const R mrdx = D.msfvy(ie - 1, j) * R(D.rdx);
+  const R mrdx = D.msfvy(ie - 1, j) * D.r.rdx;
   const R uw = R(0.5) * (D.ru.ld(ie, jp, k) + D.ru.ld(ie, jm, k));
   const R ub = uw > R(0) ? uw : R(0);
   const R dup = D.ru.ld(ie, jp, k) - D.ru.ld(ie - 1, jp, k), dum = D.ru.ld(ie, jm, k) - D.ru.ld(ie - 1, jm, k);
@@ -454,7 +454,7 @@ __device__ R tv_open_x(const Dom<R>& D, int i, int j, int k) {
 // an open y boundary face of v (:327-340): the radiation condition only, and the held tendency
 template <class R>
 __device__ R tend_v_open_face(const Dom<R>& D, int i, int j, int k, bool use_tendf) {
-  const R rdy = R(D.rdy), c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
+  const R rdy = D.r.rdy, c1h = D.r.c1h[k], c2h = D.r.c2h[k];
   R t;
   if (j == 0) {
     R vb = D.rv.ld(i, 0, k) - R(k::cb) * (c1h * D.mut.ld(i, 0, 0) + c2h);
@@ -470,8 +470,8 @@ __device__ R tend_v_open_face(const Dom<R>& D, int i, int j, int k, bool use_ten
 }
 template <bool OP, class R>
 __device__ R tend_v(const Dom<R>& D, int i, int j, int k, bool use_tendf, R fx0, R fx1, R fy0, R fy1) {
-  const R rdx = R(D.rdx), rdy = R(D.rdy);
-  const R c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
+  const R rdx = D.r.rdx, rdy = D.r.rdy;
+  const R c1h = D.r.c1h[k], c2h = D.r.c2h[k];
   const R rm = div_msf(D.msfvy(i, j), D.msfvx(i, j));
   R t;
   if (OP && D.open_x && (i == 0 || i == D.nx - 1)) {  // open x: the y flux, then the open term instead of the x flux
@@ -481,13 +481,13 @@ __device__ R tend_v(const Dom<R>& D, int i, int j, int k, bool use_tendf, R fx0,
     t = -(D.msfvy(i, j) * rdx) * (fx1 - fx0);
     t -= (D.msfvy(i, j) * rdy) * (fy1 - fy0);
   }
-  t -= rm * R(D.rdnw[k]) * (tv_fz(D, i, j, k + 1) - tv_fz(D, i, j, k));
+  t -= rm * D.r.rdnw[k] * (tv_fz(D, i, j, k + 1) - tv_fz(D, i, j, k));
   R dpy = rm * R(0.5) * rdy * (c1h * D.muv.ld(i, j, 0) + c2h) *
           ((D.ph2.ld(i, j, k + 1) - D.ph2.ld(i, j - 1, k + 1) + D.ph2.ld(i, j, k) - D.ph2.ld(i, j - 1, k)) +
            (D.alt.ld(i, j, k) + D.alt.ld(i, j - 1, k)) * (D.p.ld(i, j, k) - D.p.ld(i, j - 1, k)) +
            (D.al.ld(i, j, k) + D.al.ld(i, j - 1, k)) * (D.pb(i, j, k) - D.pb(i, j - 1, k)));
   dpy += rm * rdy * (D.php.ld(i, j, k) - D.php.ld(i, j - 1, k)) *
-         (R(D.rdnw[k]) * (pgf_dpn<R, 0, 1>(D, i, j, k + 1) - pgf_dpn<R, 0, 1>(D, i, j, k)) -
+         (D.r.rdnw[k] * (pgf_dpn<R, 0, 1>(D, i, j, k + 1) - pgf_dpn<R, 0, 1>(D, i, j, k)) -
           R(0.5) * (c1h * D.mu2.ld(i, j - 1, 0) + c1h * D.mu2.ld(i, j, 0)));
   t -= cqv_(D, i, j, k) * dpy;
   const R rw4 = R(0.25) * (D.rw.ld(i, j - 1, k + 1) + D.rw.ld(i, j - 1, k) + D.rw.ld(i, j, k + 1) + D.rw.ld(i, j, k));
@@ -508,39 +508,39 @@ __device__ R tend_v(const Dom<R>& D, int i, int j, int k, bool use_tendf, R fx0,
 template <class R>
 __device__ __forceinline__ R tw_rux(const Dom<R>& D, int i, int j, int k) {
   const int nz = D.nz;
-  if (k < nz) return R(D.fnm[k]) * D.ru.ld(i, j, k) + R(D.fnp[k]) * D.ru.ld(i, j, k - 1);
-  return (R(2) - R(D.fnm[nz - 1])) * D.ru.ld(i, j, nz - 1) - R(D.fnp[nz - 1]) * D.ru.ld(i, j, nz - 2);
+  if (k < nz) return D.r.fnm[k] * D.ru.ld(i, j, k) + D.r.fnp[k] * D.ru.ld(i, j, k - 1);
+  return (R(2) - D.r.fnm[nz - 1]) * D.ru.ld(i, j, nz - 1) - D.r.fnp[nz - 1] * D.ru.ld(i, j, nz - 2);
 }
 template <class R>
 __device__ __forceinline__ R tw_rvy(const Dom<R>& D, int i, int j, int k) {
   const int nz = D.nz;
-  if (k < nz) return R(D.fnm[k]) * D.rv.ld(i, j, k) + R(D.fnp[k]) * D.rv.ld(i, j, k - 1);
-  return (R(2) - R(D.fnm[nz - 1])) * D.rv.ld(i, j, nz - 1) - R(D.fnp[nz - 1]) * D.rv.ld(i, j, nz - 2);
+  if (k < nz) return D.r.fnm[k] * D.rv.ld(i, j, k) + D.r.fnp[k] * D.rv.ld(i, j, k - 1);
+  return (R(2) - D.r.fnm[nz - 1]) * D.rv.ld(i, j, nz - 1) - D.r.fnp[nz - 1] * D.rv.ld(i, j, nz - 2);
 }
 template <class R>
 __device__ R tw_fx(const Dom<R>& D, int i, int j, int k) {
   const R vel = tw_rux(D, i, j, k);
   const int o = ord_face(i, D.nx, D.spec_x);
   if (o == 2) return R(0.5) * vel * (D.w2.ld(i, j, k) + D.w2.ld(i - 1, j, k));
-  if (o == 3) return vel * flux3(D.w2.ld(i - 2, j, k), D.w2.ld(i - 1, j, k), D.w2.ld(i, j, k), D.w2.ld(i + 1, j, k), vel, R(D.hup));
+  if (o == 3) return vel * flux3(D.w2.ld(i - 2, j, k), D.w2.ld(i - 1, j, k), D.w2.ld(i, j, k), D.w2.ld(i + 1, j, k), vel, D.r.hup);
   return vel * flux5(D.w2.ld(i - 3, j, k), D.w2.ld(i - 2, j, k), D.w2.ld(i - 1, j, k), D.w2.ld(i, j, k), D.w2.ld(i + 1, j, k),
-                     D.w2.ld(i + 2, j, k), vel, R(D.hup));
+                     D.w2.ld(i + 2, j, k), vel, D.r.hup);
 }
 template <class R>
 __device__ R tw_fy(const Dom<R>& D, int i, int j, int k) {
   const R vel = tw_rvy(D, i, j, k);
   const int o = ord_face(j, D.ny, D.spec_y);
   if (o == 2) return R(0.5) * vel * (D.w2.ld(i, j, k) + D.w2.ld(i, j - 1, k));
-  if (o == 3) return vel * flux3(D.w2.ld(i, j - 2, k), D.w2.ld(i, j - 1, k), D.w2.ld(i, j, k), D.w2.ld(i, j + 1, k), vel, R(D.hup));
+  if (o == 3) return vel * flux3(D.w2.ld(i, j - 2, k), D.w2.ld(i, j - 1, k), D.w2.ld(i, j, k), D.w2.ld(i, j + 1, k), vel, D.r.hup);
   return vel * flux5(D.w2.ld(i, j - 3, k), D.w2.ld(i, j - 2, k), D.w2.ld(i, j - 1, k), D.w2.ld(i, j, k), D.w2.ld(i, j + 1, k),
-                     D.w2.ld(i, j + 2, k), vel, R(D.hup));
+                     D.w2.ld(i, j + 2, k), vel, D.r.hup);
 }
 template <class R>
 __device__ R tw_fz(const Dom<R>& D, int i, int j, int m) {
   if (m == 0 || m == D.nz - 1)
     return R(0.25) * (D.ww.ld(i, j, m + 1) + D.ww.ld(i, j, m)) * (D.w2.ld(i, j, m + 1) + D.w2.ld(i, j, m));
   const R vel = R(0.5) * (D.ww.ld(i, j, m + 1) + D.ww.ld(i, j, m));
-  return vel * flux3(D.w2.ld(i, j, m - 1), D.w2.ld(i, j, m), D.w2.ld(i, j, m + 1), D.w2.ld(i, j, m + 2), -vel, R(D.vup));
+  return vel * flux3(D.w2.ld(i, j, m - 1), D.w2.ld(i, j, m), D.w2.ld(i, j, m + 1), D.w2.ld(i, j, m + 2), -vel, D.r.vup);
 }
 // advect_w open_xs/xe (open_ys/ye) terms of the outermost columns (rows) (KTendW::open_x_term / open_y_term,
 // :416-453): DI = 1 for x, 0 for y; the normal mass flux fnm/fnp-interpolated to the w level, extrapolated at the lid
@@ -554,15 +554,15 @@ __device__ R tw_open(const Dom<R>& D, int i, int j, int k) {
   auto Wv = [&](int f) { return DI ? D.w2.ld(f, j, k) : D.w2.ld(i, f, k); };
   R uw, dru;
   if (k < nz) {
-    const R fnm = R(D.fnm[k]), fnp = R(D.fnp[k]);
+    const R fnm = D.r.fnm[k], fnp = D.r.fnp[k];
     uw = R(0.5) * (fnm * (RF(a, k) + RF(b, k)) + fnp * (RF(a, k - 1) + RF(b, k - 1)));
     dru = fnm * (RF(b, k) - RF(a, k)) + fnp * (RF(b, k - 1) - RF(a, k - 1));
   } else {
-    const R fm = R(2) - R(D.fnm[nz - 1]), fp = R(D.fnp[nz - 1]);
+    const R fm = R(2) - D.r.fnm[nz - 1], fp = D.r.fnp[nz - 1];
     uw = R(0.5) * (fm * (RF(a, nz - 1) + RF(b, nz - 1)) - fp * (RF(a, nz - 2) + RF(b, nz - 2)));
     dru = fm * (RF(b, nz - 1) - RF(a, nz - 1)) - fp * (RF(b, nz - 2) - RF(a, nz - 2));
   }
-  const R rd = DI ? R(D.rdx) : R(D.rdy);
+  const R rd = DI ? D.r.rdx : D.r.rdy;
   if (c == 0) {
     const R ub = uw < R(0) ? uw : R(0);
     return rd * (ub * (Wv(1) - Wv(0)) + Wv(0) * dru);
@@ -573,7 +573,7 @@ __device__ R tw_open(const Dom<R>& D, int i, int j, int k) {
 template <bool OP, class R>
 __device__ R tend_w(const Dom<R>& D, int i, int j, int k, bool use_tendf, R fx0, R fx1, R fy0, R fy1) {
   const int nz = D.nz;
-  const R rdx = R(D.rdx), rdy = R(D.rdy);
+  const R rdx = D.r.rdx, rdy = D.r.rdy;
   R t;
   const bool ocol = OP && D.open_x && (i == 0 || i == D.nx - 1), orow = OP && D.open_y && (j == 0 || j == D.ny - 1);
   if (ocol || orow) {  // the reference's order: y flux, x flux, open x terms, open y terms
@@ -588,19 +588,19 @@ __device__ R tend_w(const Dom<R>& D, int i, int j, int k, bool use_tendf, R fx0,
   }
   const R rmsft = div_msf(R(1), D.msfty(i, j));
   if (k < nz) {
-    t -= R(D.rdn[k]) * (tw_fz(D, i, j, k) - tw_fz(D, i, j, k - 1));
+    t -= D.r.rdn[k] * (tw_fz(D, i, j, k) - tw_fz(D, i, j, k - 1));
     const R cqw = cqw_(D, i, j, k), cq1 = R(1) / (R(1) + cqw), cq2 = cqw * cq1;
     t += rmsft * R(k::g) *
-         (cq1 * R(D.rdn[k]) * (D.p.ld(i, j, k) - D.p.ld(i, j, k - 1)) - R(D.c1f[k]) * D.mu2.ld(i, j, 0) -
-          cq2 * (R(D.c1f[k]) * D.mub(i, j) + R(D.c2f[k])));
+         (cq1 * D.r.rdn[k] * (D.p.ld(i, j, k) - D.p.ld(i, j, k - 1)) - D.r.c1f[k] * D.mu2.ld(i, j, 0) -
+          cq2 * (D.r.c1f[k] * D.mub(i, j) + D.r.c2f[k]));
     if (D.w_damping) {  // w_damp, wd_dt = dt
       const R wd_dt = R(D.dt);
-      const R muf = R(D.c1f[k]) * D.mut.ld(i, j, 0) + R(D.c2f[k]);
-      R cfl = D.ww.ld(i, j, k) / muf * R(D.rdnw[k]) * wd_dt;
+      const R muf = D.r.c1f[k] * D.mut.ld(i, j, 0) + D.r.c2f[k];
+      R cfl = D.ww.ld(i, j, k) / muf * D.r.rdnw[k] * wd_dt;
       cfl = cfl < R(0) ? -cfl : cfl;
       if (cfl > R(1)) t = t - (D.w2.ld(i, j, k) < R(0) ? R(-1) : R(1)) * R(0.3) * (cfl - R(D.w_crit_cfl)) * muf;
     }
-    const R fnm = R(D.fnm[k]), fnp = R(D.fnp[k]);
+    const R fnm = D.r.fnm[k], fnp = D.r.fnp[k];
     const R ruw = R(0.5) * (fnm * (D.ru.ld(i, j, k) + D.ru.ld(i + 1, j, k)) + fnp * (D.ru.ld(i, j, k - 1) + D.ru.ld(i + 1, j, k - 1)));
     const R rvw = R(0.5) * (fnm * (D.rv.ld(i, j, k) + D.rv.ld(i, j + 1, k)) + fnp * (D.rv.ld(i, j, k - 1) + D.rv.ld(i, j + 1, k - 1)));
     const R rmt = div_msf(D.msftx(i, j), D.msfty(i, j));
@@ -609,11 +609,11 @@ __device__ R tend_w(const Dom<R>& D, int i, int j, int k, bool use_tendf, R fx0,
     const R vw = R(0.5) * (fnm * (D.v2.ld(i, j, k) + D.v2.ld(i, j + 1, k)) + fnp * (D.v2.ld(i, j, k - 1) + D.v2.ld(i, j + 1, k - 1)));
     t = t + R(k::reradius) * (ruw * uw + rmt * rvw * vw);
   } else {
-    t += R(2) * R(D.rdn[nz - 1]) * tw_fz(D, i, j, nz - 1);
+    t += R(2) * D.r.rdn[nz - 1] * tw_fz(D, i, j, nz - 1);
     const R cqw = cqw_(D, i, j, nz - 1), cq1 = R(1) / (R(1) + cqw), cq2 = cqw * cq1;
     t += rmsft * R(k::g) *
-         (cq1 * R(2) * R(D.rdnw[nz - 1]) * (-D.p.ld(i, j, nz - 1)) - R(D.c1f[nz]) * D.mu2.ld(i, j, 0) -
-          cq2 * (R(D.c1f[nz]) * D.mub(i, j) + R(D.c2f[nz])));
+         (cq1 * R(2) * D.r.rdnw[nz - 1] * (-D.p.ld(i, j, nz - 1)) - D.r.c1f[nz] * D.mu2.ld(i, j, 0) -
+          cq2 * (D.r.c1f[nz] * D.mub(i, j) + D.r.c2f[nz]));
   }
   if (use_tendf) t += div_msf(D.rw_tendf.ld(i, j, k), D.msfty(i, j));
   return t;
@@ -627,12 +627,12 @@ __device__ R sc_fx(const Dom<R>& D, const QV& q, const V3<R>& ruf, int i, int j,
   const int o = ord_face(i, D.nx, D.spec_x);
   if (o == 2) return R(0.5) * vel * (q.ld(i, j, k) + q.ld(i - 1, j, k));
   if (o == 3) {
-    if (pd) return vel * flux3_pd(q.ld(i - 2, j, k), q.ld(i - 1, j, k), q.ld(i, j, k), q.ld(i + 1, j, k), vel, R(D.hup));
-    return vel * flux3(q.ld(i - 2, j, k), q.ld(i - 1, j, k), q.ld(i, j, k), q.ld(i + 1, j, k), vel, R(D.hup));
+    if (pd) return vel * flux3_pd(q.ld(i - 2, j, k), q.ld(i - 1, j, k), q.ld(i, j, k), q.ld(i + 1, j, k), vel, D.r.hup);
+    return vel * flux3(q.ld(i - 2, j, k), q.ld(i - 1, j, k), q.ld(i, j, k), q.ld(i + 1, j, k), vel, D.r.hup);
   }
   if (pd)
-    return vel * flux5_pd(q.ld(i - 3, j, k), q.ld(i - 2, j, k), q.ld(i - 1, j, k), q.ld(i, j, k), q.ld(i + 1, j, k), q.ld(i + 2, j, k), vel, R(D.hup));
-  return vel * flux5(q.ld(i - 3, j, k), q.ld(i - 2, j, k), q.ld(i - 1, j, k), q.ld(i, j, k), q.ld(i + 1, j, k), q.ld(i + 2, j, k), vel, R(D.hup));
+    return vel * flux5_pd(q.ld(i - 3, j, k), q.ld(i - 2, j, k), q.ld(i - 1, j, k), q.ld(i, j, k), q.ld(i + 1, j, k), q.ld(i + 2, j, k), vel, D.r.hup);
+  return vel * flux5(q.ld(i - 3, j, k), q.ld(i - 2, j, k), q.ld(i - 1, j, k), q.ld(i, j, k), q.ld(i + 1, j, k), q.ld(i + 2, j, k), vel, D.r.hup);
 }
 template <class R, class QV>
 __device__ R sc_fy(const Dom<R>& D, const QV& q, const V3<R>& rvf, int i, int j, int k, bool pd) {
@@ -640,20 +640,20 @@ __device__ R sc_fy(const Dom<R>& D, const QV& q, const V3<R>& rvf, int i, int j,
   const int o = ord_face(j, D.ny, D.spec_y);
   if (o == 2) return R(0.5) * vel * (q.ld(i, j, k) + q.ld(i, j - 1, k));
   if (o == 3) {
-    if (pd) return vel * flux3_pd(q.ld(i, j - 2, k), q.ld(i, j - 1, k), q.ld(i, j, k), q.ld(i, j + 1, k), vel, R(D.hup));
-    return vel * flux3(q.ld(i, j - 2, k), q.ld(i, j - 1, k), q.ld(i, j, k), q.ld(i, j + 1, k), vel, R(D.hup));
+    if (pd) return vel * flux3_pd(q.ld(i, j - 2, k), q.ld(i, j - 1, k), q.ld(i, j, k), q.ld(i, j + 1, k), vel, D.r.hup);
+    return vel * flux3(q.ld(i, j - 2, k), q.ld(i, j - 1, k), q.ld(i, j, k), q.ld(i, j + 1, k), vel, D.r.hup);
   }
   if (pd)
-    return vel * flux5_pd(q.ld(i, j - 3, k), q.ld(i, j - 2, k), q.ld(i, j - 1, k), q.ld(i, j, k), q.ld(i, j + 1, k), q.ld(i, j + 2, k), vel, R(D.hup));
-  return vel * flux5(q.ld(i, j - 3, k), q.ld(i, j - 2, k), q.ld(i, j - 1, k), q.ld(i, j, k), q.ld(i, j + 1, k), q.ld(i, j + 2, k), vel, R(D.hup));
+    return vel * flux5_pd(q.ld(i, j - 3, k), q.ld(i, j - 2, k), q.ld(i, j - 1, k), q.ld(i, j, k), q.ld(i, j + 1, k), q.ld(i, j + 2, k), vel, D.r.hup);
+  return vel * flux5(q.ld(i, j - 3, k), q.ld(i, j - 2, k), q.ld(i, j - 1, k), q.ld(i, j, k), q.ld(i, j + 1, k), q.ld(i, j + 2, k), vel, D.r.hup);
 }
 template <class R, class QV>
 __device__ R sc_fz(const Dom<R>& D, const QV& q, const V3<R>& wwf, int i, int j, int k, bool pd) {
   if (k == 0 || k == D.nz) return 0;
   const R vel = wwf.ld(i, j, k);
-  if (k == 1 || k == D.nz - 1) return vel * (R(D.fnm[k]) * q.ld(i, j, k) + R(D.fnp[k]) * q.ld(i, j, k - 1));
-  if (pd) return vel * flux3_pd(q.ld(i, j, k - 2), q.ld(i, j, k - 1), q.ld(i, j, k), q.ld(i, j, k + 1), -vel, R(D.vup));
-  return vel * flux3(q.ld(i, j, k - 2), q.ld(i, j, k - 1), q.ld(i, j, k), q.ld(i, j, k + 1), -vel, R(D.vup));
+  if (k == 1 || k == D.nz - 1) return vel * (D.r.fnm[k] * q.ld(i, j, k) + D.r.fnp[k] * q.ld(i, j, k - 1));
+  if (pd) return vel * flux3_pd(q.ld(i, j, k - 2), q.ld(i, j, k - 1), q.ld(i, j, k), q.ld(i, j, k + 1), -vel, D.r.vup);
+  return vel * flux3(q.ld(i, j, k - 2), q.ld(i, j, k - 1), q.ld(i, j, k), q.ld(i, j, k + 1), -vel, D.r.vup);
 }
 // open boundaries of advect_scalar / advect_scalar_pd (kern::open_x_scalar / open_y_scalar, kernels_common.hpp:61-84):
 // the outermost column (row) takes rd (ub (qo(inner) - qo(outer)) + q (f(b) - f(a))) with the inflow mean normal
@@ -663,7 +663,7 @@ __device__ R open_scalar(const Dom<R>& D, const V3<R>& q, const V3<R>& qo, const
   auto M = [&](int f) { return DI ? mf.ld(f, j, k) : mf.ld(i, f, k); };
   auto Q = [&](const V3<R>& a, int f) { return DI ? a.ld(f, j, k) : a.ld(i, f, k); };
   const int c = DI ? i : j, n = DI ? D.nx : D.ny;
-  const R rd = DI ? R(D.rdx) : R(D.rdy);
+  const R rd = DI ? D.r.rdx : D.r.rdy;
   if (c == 0) {
     R ub = R(0.5) * (M(0) + M(1));
     ub = ub < R(0) ? ub : R(0);
@@ -679,24 +679,24 @@ __device__ R tend_t(const Dom<R>& D, int i, int j, int k, bool use_tendf, bool u
   const bool ocol = OP && D.open_x && (i == 0 || i == D.nx - 1), orow = OP && D.open_y && (j == 0 || j == D.ny - 1);
   if (ocol || orow) {  // open boundary (:535-541): y flux, x flux, open x terms, open y terms, then the vertical
     r = R(0);
-    if (D.do_y && !orow) r = r - (D.msftx(i, j) * R(D.rdy)) * (fy1 - fy0);
-    if (!ocol) r = r - (D.msftx(i, j) * R(D.rdx)) * (fx1 - fx0);
+    if (D.do_y && !orow) r = r - (D.msftx(i, j) * D.r.rdy) * (fy1 - fy0);
+    if (!ocol) r = r - (D.msftx(i, j) * D.r.rdx) * (fx1 - fx0);
     if (ocol) r = r - open_scalar<R, 1>(D, D.t2, D.t2, D.ru, i, j, k);
     if (orow) r = r - open_scalar<R, 0>(D, D.t2, D.t2, D.rv, i, j, k);
   } else {
-    r = -(D.msftx(i, j) * R(D.rdx)) * (fx1 - fx0);
-    if (D.do_y) r -= (D.msftx(i, j) * R(D.rdy)) * (fy1 - fy0);
+    r = -(D.msftx(i, j) * D.r.rdx) * (fx1 - fx0);
+    if (D.do_y) r -= (D.msftx(i, j) * D.r.rdy) * (fy1 - fy0);
   }
-  r -= R(D.rdnw[k]) * (sc_fz(D, D.t2, D.ww, i, j, k + 1, false) - sc_fz(D, D.t2, D.ww, i, j, k, false));
+  r -= D.r.rdnw[k] * (sc_fz(D, D.t2, D.ww, i, j, k + 1, false) - sc_fz(D, D.t2, D.ww, i, j, k, false));
   if (use_tendf) r += div_msf(D.t_tendf.ld(i, j, k), D.msfty(i, j));
-  if (use_hd) r += div_msf((R(D.c1h[k]) * D.mut.ld(i, j, 0) + R(D.c2h[k])) * D.hd.ld(i, j, k), D.msfty(i, j));
+  if (use_hd) r += div_msf((D.r.c1h[k] * D.mut.ld(i, j, 0) + D.r.c2h[k]) * D.hd.ld(i, j, k), D.msfty(i, j));
   return r;
 }
 
 // KTendPh (:570-668)
 template <class R>
 __device__ __forceinline__ R tph_wdwn(const Dom<R>& D, int i, int j, int m) {
-  return R(0.5) * (D.ww.ld(i, j, m + 1) + D.ww.ld(i, j, m)) * R(D.rdnw[m]) *
+  return R(0.5) * (D.ww.ld(i, j, m + 1) + D.ww.ld(i, j, m)) * D.r.rdnw[m] *
          (D.ph2.ld(i, j, m + 1) - D.ph2.ld(i, j, m) + D.phb(i, j, m + 1) - D.phb(i, j, m));
 }
 template <class R, int DI, int DJ>
@@ -729,16 +729,16 @@ __device__ __forceinline__ int ph_horder(int i, int n, int on, int is_x, int ope
 template <bool OP, class R>
 __device__ R tend_ph(const Dom<R>& D, int i, int j, int k, bool use_tendf) {
   const int nz = D.nz;
-  const R c1f = R(D.c1f[k]), c2f = R(D.c2f[k]);
+  const R c1f = D.r.c1f[k], c2f = D.r.c2f[k];
   R t = 0;
-  if (k < nz) t = t - (R(D.fnm[k]) * tph_wdwn(D, i, j, k) + R(D.fnp[k]) * tph_wdwn(D, i, j, k - 1));
+  if (k < nz) t = t - (D.r.fnm[k] * tph_wdwn(D, i, j, k) + D.r.fnp[k] * tph_wdwn(D, i, j, k - 1));
   t = t + div_msf((c1f * D.mut.ld(i, j, 0) + c2f) * R(k::g) * D.w2.ld(i, j, k), D.msfty(i, j));
   const R r60 = R(1) / R(60), r12 = R(1) / R(12);
   if (D.do_y) {
     const R mvp = c1f * D.muv.ld(i, j + 1, 0) + c2f, mvm = c1f * D.muv.ld(i, j, 0) + c2f;
-    const R vp = k < nz ? D.v2.ld(i, j + 1, k) + D.v2.ld(i, j + 1, k - 1) : R(D.cfn) * D.v2.ld(i, j + 1, nz - 1) + R(D.cfn1) * D.v2.ld(i, j + 1, nz - 2);
-    const R vm = k < nz ? D.v2.ld(i, j, k) + D.v2.ld(i, j, k - 1) : R(D.cfn) * D.v2.ld(i, j, nz - 1) + R(D.cfn1) * D.v2.ld(i, j, nz - 2);
-    const R cy = div_msf((k < nz ? R(0.25) : R(0.5)) * R(D.rdy), D.msfty(i, j));
+    const R vp = k < nz ? D.v2.ld(i, j + 1, k) + D.v2.ld(i, j + 1, k - 1) : D.r.cfn * D.v2.ld(i, j + 1, nz - 1) + D.r.cfn1 * D.v2.ld(i, j + 1, nz - 2);
+    const R vm = k < nz ? D.v2.ld(i, j, k) + D.v2.ld(i, j, k - 1) : D.r.cfn * D.v2.ld(i, j, nz - 1) + D.r.cfn1 * D.v2.ld(i, j, nz - 2);
+    const R cy = div_msf((k < nz ? R(0.25) : R(0.5)) * D.r.rdy, D.msfty(i, j));
     const int o = ph_horder(j, D.ny, D.spec_y, 0, OP && D.open_x);
     if (o == 6) t = t - cy * ((mvp * vp * D.msfvy(i, j + 1) + mvm * vm * D.msfvy(i, j)) * r60 * grad6<R, 0, 1>(D, i, j, k));
     else if (o == 4) t = t - cy * ((mvp * vp * D.msfvy(i, j + 1) + mvm * vm * D.msfvy(i, j)) * r12 * grad4<R, 0, 1>(D, i, j, k));
@@ -746,9 +746,9 @@ __device__ R tend_ph(const Dom<R>& D, int i, int j, int k, bool use_tendf) {
       t = t - cy * (mvp * vp * D.msfvy(i, j + 1) * dfwd<R, 0, 1>(D, i, j, k) + mvm * vm * D.msfvy(i, j) * dfwd<R, 0, 1>(D, i, j - 1, k));
   }
   const R mup = c1f * D.muu.ld(i + 1, j, 0) + c2f, mum = c1f * D.muu.ld(i, j, 0) + c2f;
-  const R up = k < nz ? D.u2.ld(i + 1, j, k) + D.u2.ld(i + 1, j, k - 1) : R(D.cfn) * D.u2.ld(i + 1, j, nz - 1) + R(D.cfn1) * D.u2.ld(i + 1, j, nz - 2);
-  const R um = k < nz ? D.u2.ld(i, j, k) + D.u2.ld(i, j, k - 1) : R(D.cfn) * D.u2.ld(i, j, nz - 1) + R(D.cfn1) * D.u2.ld(i, j, nz - 2);
-  const R cx = div_msf((k < nz ? R(0.25) : R(0.5)) * R(D.rdx), D.msfty(i, j));
+  const R up = k < nz ? D.u2.ld(i + 1, j, k) + D.u2.ld(i + 1, j, k - 1) : D.r.cfn * D.u2.ld(i + 1, j, nz - 1) + D.r.cfn1 * D.u2.ld(i + 1, j, nz - 2);
+  const R um = k < nz ? D.u2.ld(i, j, k) + D.u2.ld(i, j, k - 1) : D.r.cfn * D.u2.ld(i, j, nz - 1) + D.r.cfn1 * D.u2.ld(i, j, nz - 2);
+  const R cx = div_msf((k < nz ? R(0.25) : R(0.5)) * D.r.rdx, D.msfty(i, j));
   const int o = ph_horder(i, D.nx, D.spec_x, 1, OP && D.open_x);
   if (o == 6) t = t - cx * ((mup * up * D.msfux(i + 1, j) + mum * um * D.msfux(i, j)) * r60 * grad6<R, 1, 0>(D, i, j, k));
   else if (o == 2)
@@ -759,29 +759,29 @@ __device__ R tend_ph(const Dom<R>& D, int i, int j, int k, bool use_tendf) {
   if (OP && D.open_y && (j == 0 || j == D.ny - 1)) {
     const int kz = k < nz - 1 ? k : nz - 1;
     const int a = j == 0 ? 0 : D.ny - 1, b = j == 0 ? 1 : D.ny;
-    const R vb = R(0.5) * (R(D.fnm[kz]) * (D.v2.ld(i, b, kz) + D.v2.ld(i, a, kz)) +
-                           R(D.fnp[kz]) * (D.v2.ld(i, b, kz - 1) + D.v2.ld(i, a, kz - 1)));
+    const R vb = R(0.5) * (D.r.fnm[kz] * (D.v2.ld(i, b, kz) + D.v2.ld(i, a, kz)) +
+                           D.r.fnp[kz] * (D.v2.ld(i, b, kz - 1) + D.v2.ld(i, a, kz - 1)));
     const R muf = c1f * D.mut.ld(i, j, 0) + c2f;
     if (j == 0) {
       const R vl = vb < R(0) ? vb : R(0);
-      t = t - R(D.rdy) * muf * (vl * (D.ph2.ld(i, 1, k) - D.ph2.ld(i, 0, k)));
+      t = t - D.r.rdy * muf * (vl * (D.ph2.ld(i, 1, k) - D.ph2.ld(i, 0, k)));
     } else {
       const R vr = vb > R(0) ? vb : R(0);
-      t = t - R(D.rdy) * muf * (vr * (D.ph2.ld(i, j, k) - D.ph2.ld(i, j - 1, k)));
+      t = t - D.r.rdy * muf * (vr * (D.ph2.ld(i, j, k) - D.ph2.ld(i, j - 1, k)));
     }
   }
   if (OP && D.open_x && (i == 0 || i == D.nx - 1) && !(i == 0 && k == nz)) {
     const int kz = k < nz ? k : nz - 1;
     const int a = i == 0 ? 0 : D.nx - 1, b = i == 0 ? 1 : D.nx;
-    const R ub = R(0.5) * (R(D.fnm[kz]) * (D.u2.ld(b, j, kz) + D.u2.ld(a, j, kz)) +
-                           R(D.fnp[kz]) * (D.u2.ld(b, j, kz - 1) + D.u2.ld(a, j, kz - 1)));
+    const R ub = R(0.5) * (D.r.fnm[kz] * (D.u2.ld(b, j, kz) + D.u2.ld(a, j, kz)) +
+                           D.r.fnp[kz] * (D.u2.ld(b, j, kz - 1) + D.u2.ld(a, j, kz - 1)));
     const R muf = c1f * D.mut.ld(i, j, 0) + c2f;
     if (i == 0) {
       const R ul = ub < R(0) ? ub : R(0);
-      t = t - (div_msf(D.msftx(i, j), D.msfty(i, j))) * R(D.rdx) * muf * (ul * (D.ph2.ld(1, j, k) - D.ph2.ld(0, j, k)));
+      t = t - (div_msf(D.msftx(i, j), D.msfty(i, j))) * D.r.rdx * muf * (ul * (D.ph2.ld(1, j, k) - D.ph2.ld(0, j, k)));
     } else {
       const R ur = ub > R(0) ? ub : R(0);
-      t = t - (div_msf(D.msftx(i, j), D.msfty(i, j))) * R(D.rdx) * muf * (ur * (D.ph2.ld(i, j, k) - D.ph2.ld(i - 1, j, k)));
+      t = t - (div_msf(D.msftx(i, j), D.msfty(i, j))) * D.r.rdx * muf * (ur * (D.ph2.ld(i, j, k) - D.ph2.ld(i - 1, j, k)));
     }
   }
   if (use_tendf) t = t + div_msf(D.ph_tendf.ld(i, j, k), D.msfty(i, j));
@@ -1044,7 +1044,7 @@ struct XkField {
 template <class R, class XK>
 __device__ R hdiff_u(const Dom<R>& D, const V3<R>& f, const V3<R>& mut, XK X, int i, int j, int k) {
   const double *c1 = D.c1h, *c2 = D.c2h;
-  const R rdx = R(D.rdx), rdy = R(D.rdy);
+  const R rdx = D.r.rdx, rdy = D.r.rdy;
   const R mkrdxm = (div_msf(D.msftx(i - 1, j), D.msfty(i - 1, j))) * mk(c1, c2, mut, i - 1, j, k) * X(i - 1, j, k) * rdx;
   const R mkrdxp = (div_msf(D.msftx(i, j), D.msfty(i, j))) * mk(c1, c2, mut, i, j, k) * X(i, j, k) * rdx;
   const R mrdx = D.msfux(i, j) * D.msfuy(i, j) * rdx;
@@ -1061,7 +1061,7 @@ __device__ R hdiff_u(const Dom<R>& D, const V3<R>& f, const V3<R>& mut, XK X, in
 template <class R, class XK>
 __device__ R hdiff_v(const Dom<R>& D, const V3<R>& f, const V3<R>& mut, XK X, int i, int j, int k) {
   const double *c1 = D.c1h, *c2 = D.c2h;
-  const R rdx = R(D.rdx), rdy = R(D.rdy);
+  const R rdx = D.r.rdx, rdy = D.r.rdy;
   const R mkrdxm = ((D.msfvx(i, j) + D.msfvx(i - 1, j)) / (D.msfvy(i, j) + D.msfvy(i - 1, j))) * R(0.25) *
                    (mk(c1, c2, mut, i, j, k) + mk(c1, c2, mut, i, j - 1, k) + mk(c1, c2, mut, i - 1, j - 1, k) + mk(c1, c2, mut, i - 1, j, k)) *
                    R(0.25) * (X(i, j, k) + X(i, j - 1, k) + X(i - 1, j - 1, k) + X(i - 1, j, k)) * rdx;
@@ -1078,7 +1078,7 @@ __device__ R hdiff_v(const Dom<R>& D, const V3<R>& f, const V3<R>& mut, XK X, in
 template <class R, class XK>
 __device__ R hdiff_w(const Dom<R>& D, const V3<R>& f, const V3<R>& mut, XK X, int i, int j, int k) {
   const double *c1 = D.c1f, *c2 = D.c2f;
-  const R rdx = R(D.rdx), rdy = R(D.rdy);
+  const R rdx = D.r.rdx, rdy = D.r.rdy;
   const R mkrdxm = (div_msf(D.msfux(i, j), D.msfuy(i, j))) * R(0.25) *
                    (mk(c1, c2, mut, i, j, k) + mk(c1, c2, mut, i - 1, j, k) + mk(c1, c2, mut, i, j, k) + mk(c1, c2, mut, i - 1, j, k)) *
                    R(0.25) * (X(i, j, k) + X(i - 1, j, k) + X(i, j, k - 1) + X(i - 1, j, k - 1)) * rdx;
@@ -1100,7 +1100,7 @@ __device__ R hdiff_w(const Dom<R>& D, const V3<R>& f, const V3<R>& mut, XK X, in
 template <class R, class XK>
 __device__ R hdiff_m(const Dom<R>& D, const V3<R>& f, const VB<R>* base, const V3<R>& mut, XK X, int i, int j, int k) {
   const double *c1 = D.c1h, *c2 = D.c2h;
-  const R rdx = R(D.rdx), rdy = R(D.rdy);
+  const R rdx = D.r.rdx, rdy = D.r.rdy;
   const R mkrdxm = (div_msf(D.msfux(i, j), D.msfuy(i, j))) * R(0.5) * (X(i, j, k) + X(i - 1, j, k)) * R(0.5) * (mk(c1, c2, mut, i, j, k) + mk(c1, c2, mut, i - 1, j, k)) * rdx;
   const R mkrdxp = (div_msf(D.msfux(i + 1, j), D.msfuy(i + 1, j))) * R(0.5) * (X(i + 1, j, k) + X(i, j, k)) * R(0.5) * (mk(c1, c2, mut, i + 1, j, k) + mk(c1, c2, mut, i, j, k)) * rdx;
   const R mrdx = D.msftx(i, j) * D.msfty(i, j) * rdx;
@@ -1121,51 +1121,51 @@ __device__ R hdiff_m(const Dom<R>& D, const V3<R>& f, const VB<R>* base, const V
 template <class R>
 __device__ __forceinline__ R vflux_w(const Dom<R>& D, const V3<R>& f, R kv, int i, int j, int k) {
   if (k >= D.nz - 1) return 0;
-  return (kv / D.alt.ld(i, j, k)) * R(D.rdnw[k]) * (f.ld(i, j, k + 1) - f.ld(i, j, k));
+  return (kv / D.alt.ld(i, j, k)) * D.r.rdnw[k] * (f.ld(i, j, k + 1) - f.ld(i, j, k));
 }
 template <class R>
 __device__ __forceinline__ R vflux_m(const Dom<R>& D, const V3<R>& f, const VB<R>* base, R kv, int i, int j, int k) {
   if (k >= D.nz - 1) return 0;
   const R dpert = base ? f.ld(i, j, k + 1) - f.ld(i, j, k) - (*base)(i, j, k + 1) + (*base)(i, j, k) : f.ld(i, j, k + 1) - f.ld(i, j, k);
-  return kv * R(D.rdn[k + 1]) / (R(0.5) * (D.alt.ld(i, j, k) + D.alt.ld(i, j, k + 1))) * dpert;
+  return kv * D.r.rdn[k + 1] / (R(0.5) * (D.alt.ld(i, j, k) + D.alt.ld(i, j, k + 1))) * dpert;
 }
 template <class R, int DI, int DJ>
 __device__ __forceinline__ R vflux_uv(const Dom<R>& D, const V3<R>& f, const double* ub, R kv, int i, int j, int k) {
   if (k >= D.nz - 1) return 0;
   const R a = R(0.25) * (D.alt.ld(i, j, k) + D.alt.ld(i - DI, j - DJ, k) + D.alt.ld(i, j, k + 1) + D.alt.ld(i - DI, j - DJ, k + 1));
   const R dpert = f.ld(i, j, k + 1) - f.ld(i, j, k) - R(ub[k + 1]) + R(ub[k]);
-  return kv * R(D.rdn[k + 1]) / a * dpert;
+  return kv * D.r.rdn[k + 1] / a * dpert;
 }
 // vertical_diffusion 'w' (KVertDiffW1), 'm' / mp (KVertDiffM1 / MP1), u / v (KVertDiffU1 / V1): the
 // increment of level k
 template <class R>
 __device__ __forceinline__ R vdiff_w(const Dom<R>& D, const V3<R>& f, const V3<R>& mut, R kv, int i, int j, int k) {
   const R G = R(k::g);
-  const R mu = R(D.c1f[k]) * mut.ld(i, j, 0) + R(D.c2f[k]);
+  const R mu = D.r.c1f[k] * mut.ld(i, j, 0) + D.r.c2f[k];
   const R alt_avg = R(0.5) * (D.alt.ld(i, j, k) + D.alt.ld(i, j, k - 1));
-  return R(D.rdn[k]) * G * G / mu / alt_avg * (vflux_w(D, f, kv, i, j, k) - vflux_w(D, f, kv, i, j, k - 1));
+  return D.r.rdn[k] * G * G / mu / alt_avg * (vflux_w(D, f, kv, i, j, k) - vflux_w(D, f, kv, i, j, k - 1));
 }
 template <class R>
 __device__ __forceinline__ R vdiff_m(const Dom<R>& D, const V3<R>& f, const VB<R>* base, const V3<R>& mut, R kv, int i, int j, int k) {
   const R G = R(k::g);
   if (k == 0) {
     const R vf0 = vflux_m(D, f, base, kv, i, j, 0);
-    return G * G / (R(D.c1h[0]) * mut.ld(i, j, 0) + R(D.c2h[0])) / D.alt.ld(i, j, 0) * R(D.rdnw[0]) * (vf0 - vf0);
+    return G * G / (D.r.c1h[0] * mut.ld(i, j, 0) + D.r.c2h[0]) / D.alt.ld(i, j, 0) * D.r.rdnw[0] * (vf0 - vf0);
   }
-  const R mu = R(D.c1h[k]) * mut.ld(i, j, 0) + R(D.c2h[k]);
-  return G * G / mu / D.alt.ld(i, j, k) * R(D.rdnw[k]) * (vflux_m(D, f, base, kv, i, j, k) - vflux_m(D, f, base, kv, i, j, k - 1));
+  const R mu = D.r.c1h[k] * mut.ld(i, j, 0) + D.r.c2h[k];
+  return G * G / mu / D.alt.ld(i, j, k) * D.r.rdnw[k] * (vflux_m(D, f, base, kv, i, j, k) - vflux_m(D, f, base, kv, i, j, k - 1));
 }
 template <class R, int DI, int DJ>
 __device__ __forceinline__ R vdiff_uv(const Dom<R>& D, const V3<R>& f, const double* ub, const V3<R>& muf, R kv, int i, int j, int k) {
   const R G = R(k::g);
   if (k == 0) {
     const R vf0 = vflux_uv<R, DI, DJ>(D, f, ub, kv, i, j, 0);
-    return G * G * R(D.rdnw[0]) / (R(D.c1h[0]) * muf.ld(i, j, 0) + R(D.c2h[0])) /
+    return G * G * D.r.rdnw[0] / (D.r.c1h[0] * muf.ld(i, j, 0) + D.r.c2h[0]) /
            (R(0.5) * (D.alt.ld(i - DI, j - DJ, 0) + D.alt.ld(i, j, 0))) * (vf0 - vf0);
   }
-  const R mu = R(D.c1h[k]) * muf.ld(i, j, 0) + R(D.c2h[k]);
+  const R mu = D.r.c1h[k] * muf.ld(i, j, 0) + D.r.c2h[k];
   const R a = R(0.5) * (D.alt.ld(i - DI, j - DJ, k) + D.alt.ld(i, j, k));
-  return G * G * R(D.rdnw[k]) / mu / a * (vflux_uv<R, DI, DJ>(D, f, ub, kv, i, j, k) - vflux_uv<R, DI, DJ>(D, f, ub, kv, i, j, k - 1));
+  return G * G * D.r.rdnw[k] / mu / a * (vflux_uv<R, DI, DJ>(D, f, ub, kv, i, j, k) - vflux_uv<R, DI, DJ>(D, f, ub, kv, i, j, k - 1));
 }
 
 // rk 1: zero the held tendencies, add the constant-K diffusion; with lateral boundaries mu_tend = 0 and the
@@ -1296,7 +1296,7 @@ __device__ bool ray_u(const Dom<R>& D, int i, int j, int k, R& term) {
     return R(0.25) * (D.phb(a, j, kk) + D.phb(a, j, kk + 1) + D.phb(b, j, kk) + D.phb(b, j, kk + 1) + D.ph2.ld(a, j, kk) +
                       D.ph2.ld(a, j, kk + 1) + D.ph2.ld(b, j, kk) + D.ph2.ld(b, j, kk + 1)) / R(k::g);
   };
-  return ray_term(D, D.u_base, ztop, zlev, R(D.c1h[k]) * D.muu.ld(i, j, 0) + R(D.c2h[k]), D.u2.ld(i, j, k), k, term);
+  return ray_term(D, D.u_base, ztop, zlev, D.r.c1h[k] * D.muu.ld(i, j, 0) + D.r.c2h[k], D.u2.ld(i, j, k), k, term);
 }
 template <class R>
 __device__ bool ray_v(const Dom<R>& D, int i, int j, int k, R& term) {
@@ -1308,7 +1308,7 @@ __device__ bool ray_v(const Dom<R>& D, int i, int j, int k, R& term) {
     return R(0.25) * (D.phb(i, a, kk) + D.phb(i, a, kk + 1) + D.phb(i, b, kk) + D.phb(i, b, kk + 1) + D.ph2.ld(i, a, kk) +
                       D.ph2.ld(i, a, kk + 1) + D.ph2.ld(i, b, kk) + D.ph2.ld(i, b, kk + 1)) / R(k::g);
   };
-  return ray_term(D, D.v_base, ztop, zlev, R(D.c1h[k]) * D.muv.ld(i, j, 0) + R(D.c2h[k]), D.v2.ld(i, j, k), k, term);
+  return ray_term(D, D.v_base, ztop, zlev, D.r.c1h[k] * D.muv.ld(i, j, 0) + D.r.c2h[k], D.v2.ld(i, j, k), k, term);
 }
 template <class R>
 __device__ bool ray_t(const Dom<R>& D, int i, int j, int k, R& term) {
@@ -1316,14 +1316,14 @@ __device__ bool ray_t(const Dom<R>& D, int i, int j, int k, R& term) {
   auto zlev = [&](int kk) {
     return R(0.5) * (D.phb(i, j, kk) + D.phb(i, j, kk + 1) + D.ph2.ld(i, j, kk) + D.ph2.ld(i, j, kk + 1)) / R(k::g);
   };
-  return ray_term(D, D.t_base, ztop, zlev, R(D.c1h[k]) * D.mut.ld(i, j, 0) + R(D.c2h[k]), D.t2.ld(i, j, k), k, term);
+  return ray_term(D, D.t_base, ztop, zlev, D.r.c1h[k] * D.mut.ld(i, j, 0) + D.r.c2h[k], D.t2.ld(i, j, k), k, term);
 }
 // w: every level (0..nz) within zdamp of the top, toward w = 0
 template <class R>
 __device__ bool ray_w(const Dom<R>& D, int i, int j, int k, R& term) {
   const R ztop = phz(D, i, j, D.nz) / R(k::g), z = phz(D, i, j, k) / R(k::g);
   if (!(z >= ztop - R(D.zdamp))) return false;
-  term = (R(D.c1f[k]) * D.mut.ld(i, j, 0) + R(D.c2f[k])) * (ray_weight(D, ztop, z) * R(D.dampcoef)) * D.w2.ld(i, j, k);
+  term = (D.r.c1f[k] * D.mut.ld(i, j, 0) + D.r.c2f[k]) * (ray_weight(D, ztop, z) * R(D.dampcoef)) * D.w2.ld(i, j, k);
   return true;
 }
 
@@ -1356,8 +1356,8 @@ __device__ R dm_zx(const Dom<R>& D, int i, int j, int k) {
     if (i == nx) i0 = 0;
     if (i == 0) im1 = nx - 1;
   }
-  R v = R(D.rdx) * (D.phb(i0, j, k) - D.phb(im1, j, k)) / R(k::g);
-  v += R(D.rdx) * (D.ph2.ld(i0, j, k) - D.ph2.ld(im1, j, k)) / R(k::g);
+  R v = D.r.rdx * (D.phb(i0, j, k) - D.phb(im1, j, k)) / R(k::g);
+  v += D.r.rdx * (D.ph2.ld(i0, j, k) - D.ph2.ld(im1, j, k)) / R(k::g);
   return v;
 }
 // zy at V points j = 0..ny (KDiffMetricsZY)
@@ -1375,8 +1375,8 @@ __device__ R dm_zy(const Dom<R>& D, int i, int j, int k) {
     if (j == ny) j0 = 0;
     if (j == 0) jm1 = ny - 1;
   }
-  R v = R(D.rdy) * (D.phb(i, j0, k) - D.phb(i, jm1, k)) / R(k::g);
-  v += R(D.rdy) * (D.ph2.ld(i, j0, k) - D.ph2.ld(i, jm1, k)) / R(k::g);
+  R v = D.r.rdy * (D.phb(i, j0, k) - D.phb(i, jm1, k)) / R(k::g);
+  v += D.r.rdy * (D.ph2.ld(i, j0, k) - D.ph2.ld(i, jm1, k)) / R(k::g);
   return v;
 }
 // the average of two columns a(0, .), a(1, .) at w level k (the hatavg arrays of cal_deform_and_div)
@@ -1384,13 +1384,13 @@ template <class R, class A>
 __device__ __forceinline__ R dm_hatavg(const Dom<R>& D, const A& a, int k) {
   const int nz = D.nz;
   if (k == 0)
-    return R(0.5) * (R(D.cf1) * a(0, 0) + R(D.cf2) * a(0, 1) + R(D.cf3) * a(0, 2) + R(D.cf1) * a(1, 0) +
-                     R(D.cf2) * a(1, 1) + R(D.cf3) * a(1, 2));
+    return R(0.5) * (D.r.cf1 * a(0, 0) + D.r.cf2 * a(0, 1) + D.r.cf3 * a(0, 2) + D.r.cf1 * a(1, 0) +
+                     D.r.cf2 * a(1, 1) + D.r.cf3 * a(1, 2));
   if (k == nz) {
-    const R cft2 = -R(0.5) * R(D.dnw[nz - 1]) / R(D.dn[nz - 1]), cft1 = R(1.0) - cft2;
+    const R cft2 = -R(0.5) * D.r.dnw[nz - 1] / R(D.dn[nz - 1]), cft1 = R(1.0) - cft2;
     return R(0.5) * (cft1 * (a(0, nz - 1) + a(1, nz - 1)) + cft2 * (a(0, nz - 2) + a(1, nz - 2)));
   }
-  return R(0.5) * (R(D.fnm[k]) * (a(0, k) + a(1, k)) + R(D.fnp[k]) * (a(0, k - 1) + a(1, k - 1)));
+  return R(0.5) * (D.r.fnm[k] * (a(0, k) + a(1, k)) + D.r.fnp[k] * (a(0, k - 1) + a(1, k - 1)));
 }
 // defor12 at vorticity point (ci, cj), level k, after the edge copies: the point computed there
 template <class R>
@@ -1420,10 +1420,10 @@ __device__ R dm_defor12(const Dom<R>& D, int ci, int cj, int k) {
   const R r00 = dm_rdzw(D, i0, j0, k), r10 = dm_rdzw(D, im1, j0, k), r11 = dm_rdzw(D, im1, jm1, k),
           r01 = dm_rdzw(D, i0, jm1, k);
   const R tmp1_u = (dm_hatavg(D, hu, k + 1) - dm_hatavg(D, hu, k)) * R(0.25) * tmpzy * (r00 + r10 + r11 + r01);
-  const R term_u = mm * (R(D.rdy) * (hu(1, k) - hu(0, k)) - tmp1_u);
+  const R term_u = mm * (D.r.rdy * (hu(1, k) - hu(0, k)) - tmp1_u);
   const R tmpzx = R(0.25) * (dm_zx(D, i, jm1, k) + dm_zx(D, i, j0, k) + dm_zx(D, i, jm1, k + 1) + dm_zx(D, i, j0, k + 1));
   const R tmp1_v = (dm_hatavg(D, hv, k + 1) - dm_hatavg(D, hv, k)) * R(0.25) * tmpzx * (r00 + r01 + r11 + r10);
-  const R term_v = mm * (R(D.rdx) * (hv(1, k) - hv(0, k)) - tmp1_v);
+  const R term_v = mm * (D.r.rdx * (hv(1, k) - hv(0, k)) - tmp1_v);
   return term_u + term_v;
 }
 // calculate_km_kh with km_opt 4 (km_kh.hpp:585-625): KSmag2dKm one row inside open and specified sides, 0 elsewhere
@@ -1454,10 +1454,10 @@ __global__ void __launch_bounds__(PX) k_smag(const __grid_constant__ Pack<R, NM>
   const R rdzw = dm_rdzw(D, i, j, k);
   const R tmpzx = R(0.25) * (dm_zx(D, i, j, k) + dm_zx(D, i + 1, j, k) + dm_zx(D, i, j, k + 1) + dm_zx(D, i + 1, j, k + 1));
   const R tmp1_u = (dm_hatavg(D, au, k + 1) - dm_hatavg(D, au, k)) * tmpzx * rdzw;
-  const R d11 = R(2.0) * (mm * (R(D.rdx) * (au(1, k) - au(0, k)) - tmp1_u));
+  const R d11 = R(2.0) * (mm * (D.r.rdx * (au(1, k) - au(0, k)) - tmp1_u));
   const R tmpzy = R(0.25) * (dm_zy(D, i, j, k) + dm_zy(D, i, j + 1, k) + dm_zy(D, i, j, k + 1) + dm_zy(D, i, j + 1, k + 1));
   const R tmp1_v = (dm_hatavg(D, av, k + 1) - dm_hatavg(D, av, k)) * tmpzy * rdzw;
-  const R d22 = R(2.0) * (mm * (R(D.rdy) * (av(1, k) - av(0, k)) - tmp1_v));
+  const R d22 = R(2.0) * (mm * (D.r.rdy * (av(1, k) - av(0, k)) - tmp1_v));
   const R dd = d11 - d22;
   R def2 = R(0.25) * (dd * dd);
   const R d12 = R(0.25) * (dm_defor12(D, i, j, k) + dm_defor12(D, i, j + 1, k) + dm_defor12(D, i + 1, j, k) +
@@ -1637,24 +1637,24 @@ __global__ void __launch_bounds__(PX) k_ring(const __grid_constant__ Pack<R, NM>
       const R dtbc = R(*D.dtbc);
       if (k < nz && ring_for(nx, ny, 'u').map(pos, side, 0, i, j) && owns(D, i, j, 'u')) {
         const R bval = slab_val(D.lbc_var[0], sl, pos, k, 0, dtbc);
-        D.u2(i, j, k) = D.msfuy(i, j) * bval / (R(D.c1h[k]) * D.muus(i, j, 0) + R(D.c2h[k]));
+        D.u2(i, j, k) = D.msfuy(i, j) * bval / (D.r.c1h[k] * D.muus(i, j, 0) + D.r.c2h[k]);
       }
       if (k < nz && ring_for(nx, ny, 'v').map(pos, side, 0, i, j) && owns(D, i, j, 'v')) {
         const R bval = slab_val(D.lbc_var[1], sl, pos, k, 0, dtbc);
-        D.v2(i, j, k) = D.msfvx(i, j) * bval / (R(D.c1h[k]) * D.muvs(i, j, 0) + R(D.c2h[k]));
+        D.v2(i, j, k) = D.msfvx(i, j) * bval / (D.r.c1h[k] * D.muvs(i, j, 0) + D.r.c2h[k]);
       }
       if (k < nz && ring_for(nx, ny, 't').map(pos, side, 0, i, j) && owns(D, i, j, 't')) {
         const R bval = slab_val(D.lbc_var[2], sl, pos, k, 0, dtbc);
-        D.t2(i, j, k) = R(1) * bval / (R(D.c1h[k]) * D.muts(i, j, 0) + R(D.c2h[k]));
+        D.t2(i, j, k) = R(1) * bval / (D.r.c1h[k] * D.muts(i, j, 0) + D.r.c2h[k]);
         for (int n = 0; n < D.n_scalars; ++n)
           if (D.lbc_q[n].have) {
             const R qb = slab_val(D.lbc_q[n], sl, pos, k, 0, dtbc);
-            D.q2[n](i, j, k) = R(1) * qb / (R(D.c1h[k]) * D.muts(i, j, 0) + R(D.c2h[k]));
+            D.q2[n](i, j, k) = R(1) * qb / (D.r.c1h[k] * D.muts(i, j, 0) + D.r.c2h[k]);
           }
       }
       if (ring_for(nx, ny, 'h').map(pos, side, 0, i, j) && owns(D, i, j, 'h')) {
         const R bval = slab_val(D.lbc_var[3], sl, pos, k, 0, dtbc);
-        D.ph2(i, j, k) = R(1) * bval / (R(D.c1f[k]) * D.muts(i, j, 0) + R(D.c2f[k]));
+        D.ph2(i, j, k) = R(1) * bval / (D.r.c1f[k] * D.muts(i, j, 0) + D.r.c2f[k]);
       }
       if (k == 0 && ring_for(nx, ny, 'm').map(pos, side, 0, i, j) && owns(D, i, j, 'm')) {
         const R bval = slab_val(D.lbc_var[4], sl, pos, 0, 0, dtbc);
@@ -1699,9 +1699,9 @@ __global__ void __launch_bounds__(PX) k_cfl(const __grid_constant__ Pack<R, NM> 
   double vert = 0, horiz = 0;
   if (in && k >= 1) {
     const R dt = R(D.dt);
-    const R x = D.ww.ld(i, j, k) / (R(D.c1f[k]) * D.mut.ld(i, j, 0) + R(D.c2f[k])) * R(D.rdnw[k]) * dt;
+    const R x = D.ww.ld(i, j, k) / (D.r.c1f[k] * D.mut.ld(i, j, 0) + D.r.c2f[k]) * D.r.rdnw[k] * dt;
     vert = double(x < R(0) ? -x : x);
-    R a = D.u2.ld(i, j, k) * R(D.rdx) * D.msfux(i, j) * dt, b = D.v2.ld(i, j, k) * R(D.rdy) * D.msfvy(i, j) * dt;
+    R a = D.u2.ld(i, j, k) * D.r.rdx * D.msfux(i, j) * dt, b = D.v2.ld(i, j, k) * D.r.rdy * D.msfvy(i, j) * dt;
     a = a < R(0) ? -a : a;
     b = b < R(0) ? -b : b;
     horiz = double(b > a ? b : a);

@@ -22,9 +22,9 @@ __device__ __forceinline__ bool edge_vface(const Dom<R>& D, int i, int j) {
   return (D.sx && (i == 0 || i == D.nx - 1)) || (D.sy && (j <= 0 || j >= D.ny));
 }
 template <class R>
-__device__ __forceinline__ R mh_(const Dom<R>& D, int k, R m) { return R(D.c1h[k]) * m + R(D.c2h[k]); }
+__device__ __forceinline__ R mh_(const Dom<R>& D, int k, R m) { return D.r.c1h[k] * m + D.r.c2h[k]; }
 template <class R>
-__device__ __forceinline__ R mf_(const Dom<R>& D, int k, R m) { return R(D.c1f[k]) * m + R(D.c2f[k]); }
+__device__ __forceinline__ R mf_(const Dom<R>& D, int k, R m) { return D.r.c1f[k] * m + D.r.c2f[k]; }
 
 // p_rho_point (small_step.cpp:97-112): calc_p_rho, with smdiv divergence damping when damp.
 // The mixed form evaluates it in double (the hydrostatic p'' / al'' relation).
@@ -101,18 +101,18 @@ __device__ __forceinline__ R uv_dp(const Dom<R>& D, const UvPoint<R>& C, int om,
         (((C.ph1 - ph1) + (C.ph0 - ph0)) + alts * (C.p0 - p0) + (C.al + al) * dpb);
   R lo, hi;  // p'' at w levels k and k + 1
   if (k == 0) {
-    lo = R(0.5) * (R(D.cf1) * ps + R(D.cf2) * psp + R(D.cf3) * (__ldg(D.p.p + C.o + 2 * C.sk) + __ldg(q + 2 * C.sk)));
+    lo = R(0.5) * (D.r.cf1 * ps + D.r.cf2 * psp + D.r.cf3 * (__ldg(D.p.p + C.o + 2 * C.sk) + __ldg(q + 2 * C.sk)));
   } else {
-    lo = R(0.5) * (R(D.fnm[k]) * ps + R(D.fnp[k]) * psm);
+    lo = R(0.5) * (D.r.fnm[k] * ps + D.r.fnp[k] * psm);
   }
   if (k + 1 == nz) {
     hi = R(0);
     if (D.top_lid)
-      hi = R(0.5) * (R(D.cf1) * ps + R(D.cf2) * psm + R(D.cf3) * (__ldg(D.p.p + C.o - 2 * C.sk) + __ldg(q - 2 * C.sk)));
+      hi = R(0.5) * (D.r.cf1 * ps + D.r.cf2 * psm + D.r.cf3 * (__ldg(D.p.p + C.o - 2 * C.sk) + __ldg(q - 2 * C.sk)));
   } else {
-    hi = R(0.5) * (R(D.fnm[k + 1]) * psp + R(D.fnp[k + 1]) * ps);
+    hi = R(0.5) * (D.r.fnm[k + 1] * psp + D.r.fnp[k + 1] * ps);
   }
-  d += rm * rd * dphp * (R(D.rdnw[k]) * (hi - lo) - R(0.5) * (c1h * mu + c1h * C.mu));
+  d += rm * rd * dphp * (D.r.rdnw[k] * (hi - lo) - R(0.5) * (c1h * mu + c1h * C.mu));
   return d;
 }
 // over the staggered index range; with lateral boundaries the spec zone's faces take
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(PX, sizeof(R) == 8 ? 8 : 10) k_uv(const __grid
   const Dom<R>& D = *Dp;
   const int nx = D.nx, ny = D.ny;
   if (k >= D.nz) return;
-  const R dts = R(rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound);
+  const R dts = rk == 1 ? D.r.dt3 : D.r.dts;
   const int oU = i + j * D.u2.sj + k * D.u2.sk, oV = i + j * D.v2.sj + k * D.v2.sk;
   // the faces of the spec zone and of open sides; the faces that the pressure gradient moves
   bool hu = false, hv = false;
@@ -149,24 +149,24 @@ __global__ void __launch_bounds__(PX, sizeof(R) == 8 ? 8 : 10) k_uv(const __grid
   if (hv || gv) vn = D.v2.p[oV] + dts * __ldg(D.rv_tend.p + oV);
   if (gu || gv) {
     const int sj = D.t2.sj, o = i + j * sj + k * D.t2.sk, o2 = i + j * sj;
-    const R c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
+    const R c1h = D.r.c1h[k], c2h = D.r.c2h[k];
     const UvPoint<R> C(D, o, o2, k);
     const R alt = __ldg(D.alt.p + o), php = __ldg(D.php.p + o), pb = D.pb(i, j, k), mudf = __ldg(D.mudf.p + o2);
     if (gu) {
       const int m = edge_lo(i, nx, D.bc_x);
       const R msfuy = D.msfuy(i, j);
-      const R emdx = R(D.emdiv) * (R(1.) / R(D.rdx));
+      const R emdx = D.r.emdx;
       const R mudf_x = div_msf(-emdx * (mudf - __ldg(D.mudf.p + o2 + m)), msfuy);
       const R dp = uv_dp(D, C, o + m, o2 + m, alt + __ldg(D.alt.p + o - 1), pb - D.pb(i - 1, j, k),
-                         php - __ldg(D.php.p + o - 1), D.muu.ld(i, j, 0), R(D.rdx), div_msf(D.msfux(i, j), msfuy), c1h, c2h);
+                         php - __ldg(D.php.p + o - 1), D.muu.ld(i, j, 0), D.r.rdx, div_msf(D.msfux(i, j), msfuy), c1h, c2h);
       un = un - dts * (D.n_moist > 0 ? __ldg(D.cqu.p + oU) : R(1)) * dp + c1h * mudf_x;
     }
     if (gv) {
       const int m = edge_lo(j, ny, D.bc_y) * sj;
-      const R emdy = R(D.emdiv) * (R(1.) / R(D.rdy));
+      const R emdy = D.r.emdy;
       const R mudf_y = -emdy * (mudf - __ldg(D.mudf.p + o2 + m)) * D.msfvx_inv(i, j);
       const R dp = uv_dp(D, C, o + m, o2 + m, alt + __ldg(D.alt.p + o - sj), pb - D.pb(i, j - 1, k),
-                         php - __ldg(D.php.p + o - sj), D.muv.ld(i, j, 0), R(D.rdy), div_msf(D.msfvy(i, j), D.msfvx(i, j)), c1h, c2h);
+                         php - __ldg(D.php.p + o - sj), D.muv.ld(i, j, 0), D.r.rdy, div_msf(D.msfvy(i, j), D.msfvx(i, j)), c1h, c2h);
       vn = vn - dts * (D.n_moist > 0 ? __ldg(D.cqv.p + oV) : R(1)) * dp + c1h * mudf_y;
     }
   }
@@ -200,7 +200,7 @@ __device__ __forceinline__ void p_rho_phi_val(const Dom<R>& D, int i, int j, int
     a = R((double(ph_kp) - double(ph_k) + D.phb64(i, j, k + 1) - D.phb64(i, j, k)) / phm / hypso_log<R>(pfd / pfu) -
           D.alb64(i, j, k));
   } else {
-    a = R(-1) / (R(D.c1h[k]) * muts + R(D.c2h[k])) * (D.alb(i, j, k) * (R(D.c1h[k]) * mu) + R(D.rdnw[k]) * (ph_kp - ph_k));
+    a = R(-1) / (D.r.c1h[k] * muts + D.r.c2h[k]) * (D.alb(i, j, k) * (D.r.c1h[k] * mu) + D.r.rdnw[k] * (ph_kp - ph_k));
   }
   // the equation of state in double in both forms: p'' is a small difference of totals of ~1e5 Pa (in float the
   // rounding of the total's base, 6e-8, would be ~1e-4 of p'') -- for the FP64 form the same operations
@@ -244,7 +244,7 @@ __device__ __forceinline__ bool spec_cell(const Dom<R>& D, int i, int j) {
   return (D.sx && (i == 0 || i == D.nx - 1)) || (D.sy && (j == 0 || j == D.ny - 1));
 }
 template <class R>
-__device__ __forceinline__ R m_full(const Dom<R>& D, int k, R mub, R mu) { return R(D.c1h[k]) * (mub + mu) + R(D.c2h[k]); }
+__device__ __forceinline__ R m_full(const Dom<R>& D, int k, R mub, R mu) { return D.r.c1h[k] * (mub + mu) + D.r.c2h[k]; }
 
 // rk 1: q_tendf = 0 + constant-K diffusion (DiffusionDriver::scalar, diffusion_driver.cpp:293-322); for the
 // species with boundary data the relaxation of rows 1..3 (relax_scalars, lateral_bc.cpp:388-401) and the
@@ -295,13 +295,13 @@ __device__ R q_adv_h(const Dom<R>& D, const V3<R>& q, int i, int j, int k, R fx0
   const bool ocol = D.open_x && (i == 0 || i == D.nx - 1), orow = D.open_y && (j == 0 || j == D.ny - 1);
   if (ocol || orow) {  // open boundary (:129-134): y flux, x flux, open x, open y (field_old = the scalar), vertical
     r = R(0);
-    if (D.do_y && !orow) r = r - (D.msftx(i, j) * R(D.rdy)) * (fy1 - fy0);
-    if (!ocol) r = r - (D.msftx(i, j) * R(D.rdx)) * (fx1 - fx0);
+    if (D.do_y && !orow) r = r - (D.msftx(i, j) * D.r.rdy) * (fy1 - fy0);
+    if (!ocol) r = r - (D.msftx(i, j) * D.r.rdx) * (fx1 - fx0);
     if (ocol) r = r - open_scalar<R, 1>(D, q, q, D.ru_m, i, j, k);
     if (orow) r = r - open_scalar<R, 0>(D, q, q, D.rv_m, i, j, k);
   } else {
-    r = -(D.msftx(i, j) * R(D.rdx)) * (fx1 - fx0);
-    if (D.do_y) r -= (D.msftx(i, j) * R(D.rdy)) * (fy1 - fy0);
+    r = -(D.msftx(i, j) * D.r.rdx) * (fx1 - fx0);
+    if (D.do_y) r -= (D.msftx(i, j) * D.r.rdy) * (fy1 - fy0);
   }
   return r;
 }
@@ -309,7 +309,7 @@ template <class R>
 __device__ R q_adv(const Dom<R>& D, const V3<R>& q, int i, int j, int k, R fx0, R fx1, R fy0, R fy1) {
   if (spec_cell(D, i, j)) return 0;
   const R r = q_adv_h(D, q, i, j, k, fx0, fx1, fy0, fy1);
-  return r - R(D.rdnw[k]) * (sc_fz(D, q, D.ww_m, i, j, k + 1, false) - sc_fz(D, q, D.ww_m, i, j, k, false));
+  return r - D.r.rdnw[k] * (sc_fz(D, q, D.ww_m, i, j, k + 1, false) - sc_fz(D, q, D.ww_m, i, j, k, false));
 }
 // KUpdate (:145-156) for the non-PD species of this stage, every species of the point in one thread (the mass
 // fluxes, column masses and map factors loaded once for all of them); the horizontal face fluxes of the block's tile
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(PX, 12) k_q_update(const __grid_constant__ Pac
   const bool rx = j < r.j1 && j < ny, ry = i < r.i1 && i < nx;
   const bool fx0 = rx && i <= nx && i <= r.i1, fx1 = tx == SX - 1 && rx && i + 1 <= nx && i + 1 <= r.i1;
   const bool fy0 = D.do_y && ry && j <= ny && j <= r.j1, fy1 = D.do_y && ty == SY - 1 && ry && j + 1 <= ny && j + 1 <= r.j1;
-  const R dt_rk = R(rk == 1 ? D.dt / 3.0 : (rk == 2 ? 0.5 * D.dt : D.dt));
+  const R dt_rk = rk == 1 ? D.r.dt3 : (rk == 2 ? D.r.dt2 : D.r.dt);
   R mub = 0, mu1 = 0, mu2 = 0, msfty = 0;
   if (in) {
     mub = D.mub(i, j);
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(q_march_threads(SH), 1024 / q_march_threads(SH
   const int nx = D.nx, ny = D.ny;
   const bool lev = k < c1;  // this thread's point: its update
   const bool col = i < r.i1 && j < r.j1, in = col && lev;
-  const R dt_rk = R(rk == 1 ? D.dt / 3.0 : (rk == 2 ? 0.5 * D.dt : D.dt));
+  const R dt_rk = rk == 1 ? D.r.dt3 : (rk == 2 ? D.r.dt2 : D.r.dt);
   R mub = 0, mu1 = 0, mu2 = 0, msfty = 0;
   if (in) {
     mub = D.mub(i, j);
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(q_march_threads(SH), 1024 / q_march_threads(SH
       R a = 0;
       if (!spec_cell(D, i, j)) {
         const R h = q_adv_h(D, D.q2[n], i, j, k, sfx[tk][ty][tx], sfx[tk][ty][tx + 1], sfy[tk][ty][tx], sfy[tk][ty + 1][tx]);
-        a = h - R(D.rdnw[k]) * (sfz[tk + 1][ty][tx] - sfz[tk][ty][tx]);
+        a = h - D.r.rdnw[k] * (sfz[tk + 1][ty][tx] - sfz[tk][ty][tx]);
       }
       R tend = a * msfty;
       tend += D.qtf[n].ld(i, j, k);
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(PX) k_q_pre_pd(const __grid_constant__ Pack<R,
   int i, j, k;
   if (!thread_index<SH>(P, RG_MASS, Dp, i, j, k)) return;
   const Dom<R>& D = *Dp;
-  const R dt_rk = R(rk == 1 ? D.dt / 3.0 : (rk == 2 ? 0.5 * D.dt : D.dt));
+  const R dt_rk = rk == 1 ? D.r.dt3 : (rk == 2 ? D.r.dt2 : D.r.dt);
   const R m = m_full(D, k, D.mub(i, j), D.mu1(i, j, 0));
   const int n = blockIdx.y;  // the species
   if (n >= D.n_scalars) return;
@@ -511,10 +511,10 @@ __global__ void __launch_bounds__(PX) k_q_pre_pd(const __grid_constant__ Pack<R,
 }
 // advect_scalar_pd face fluxes: lo = first-order upwind (fxl/fyl/fzl :81-99), dh = high-order - lo
 template <class R>
-__device__ __forceinline__ R pd_mh(const Dom<R>& D, int i, int j, int k) { return R(D.c1h[k]) * D.muts(i, j, 0) + R(D.c2h[k]); }
+__device__ __forceinline__ R pd_mh(const Dom<R>& D, int i, int j, int k) { return D.r.c1h[k] * D.muts(i, j, 0) + D.r.c2h[k]; }
 template <class R>
 __device__ void pd_fx(const Dom<R>& D, const V3<R>& q, const V3<R>& qo, R dt, int i, int j, int k, R& dh, R& lo) {
-  const R dx = R(2) / (D.msfty(i, j) + D.msfty(i - 1, j)) / R(D.rdx), mu = R(0.5) * (pd_mh(D, i, j, k) + pd_mh(D, i - 1, j, k)),
+  const R dx = R(2) / (D.msfty(i, j) + D.msfty(i - 1, j)) / D.r.rdx, mu = R(0.5) * (pd_mh(D, i, j, k) + pd_mh(D, i - 1, j, k)),
           vel = D.ru_m(i, j, k);
   const R cr = (D.spec_x && i == 1) ? (vel / mu) * dt / dx : vel * dt / dx / mu;
   lo = mu * (dx / dt) * flux_upwind(qo(i - 1, j, k), qo(i, j, k), cr);
@@ -522,7 +522,7 @@ __device__ void pd_fx(const Dom<R>& D, const V3<R>& q, const V3<R>& qo, R dt, in
 }
 template <class R>
 __device__ void pd_fy(const Dom<R>& D, const V3<R>& q, const V3<R>& qo, R dt, int i, int j, int k, R& dh, R& lo) {
-  const R dy = R(2) / (D.msftx(i, j) + D.msftx(i, j - 1)) / R(D.rdy), mu = R(0.5) * (pd_mh(D, i, j, k) + pd_mh(D, i, j - 1, k)),
+  const R dy = R(2) / (D.msftx(i, j) + D.msftx(i, j - 1)) / D.r.rdy, mu = R(0.5) * (pd_mh(D, i, j, k) + pd_mh(D, i, j - 1, k)),
           vel = D.rv_m(i, j, k);
   const R cr = vel * dt / dy / mu;
   lo = mu * (dy / dt) * flux_upwind(qo(i, j - 1, k), qo(i, j, k), cr);
@@ -535,7 +535,7 @@ __device__ void pd_fz(const Dom<R>& D, const V3<R>& q, const V3<R>& qo, R dt, in
     dh = R(0) - R(0);
     return;
   }
-  const R dz = R(2) / (R(D.rdnw[k]) + R(D.rdnw[k - 1])), mu = pd_mh(D, i, j, k), vel = D.ww_m(i, j, k);
+  const R dz = R(2) / (D.r.rdnw[k] + D.r.rdnw[k - 1]), mu = pd_mh(D, i, j, k), vel = D.ww_m(i, j, k);
   const R cr = vel * dt / dz / mu;
   lo = mu * (dz / dt) * flux_upwind(qo(i, j, k - 1), qo(i, j, k), cr);
   dh = sc_fz(D, q, D.ww_m, i, j, k, true) - lo;
@@ -552,24 +552,24 @@ __global__ void __launch_bounds__(PX, 10) k_q_face_pd(const __grid_constant__ Pa
   if (!thread_index<SH>(P, RG_FACES, Dp, i, j, k)) return;
   const Dom<R>& D = *Dp;
   const int nx = D.nx, ny = D.ny, nz = D.nz;
-  const R dt = R(rk == 1 ? D.dt / 3.0 : (rk == 2 ? 0.5 * D.dt : D.dt));
+  const R dt = rk == 1 ? D.r.dt3 : (rk == 2 ? D.r.dt2 : D.r.dt);
   const bool fx = j < ny && k < nz, fy = D.do_y && i < nx && k < nz, fz = i < nx && j < ny;
   const bool zin = fz && k != 0 && k != nz;
   R crx = 0, facx = 0, cry = 0, facy = 0, crz = 0, facz = 0;
   if (fx) {
-    const R dx = R(2) / (D.msfty(i, j) + D.msfty(i - 1, j)) / R(D.rdx), mu = R(0.5) * (pd_mh(D, i, j, k) + pd_mh(D, i - 1, j, k)),
+    const R dx = R(2) / (D.msfty(i, j) + D.msfty(i - 1, j)) / D.r.rdx, mu = R(0.5) * (pd_mh(D, i, j, k) + pd_mh(D, i - 1, j, k)),
             vel = D.ru_m.ld(i, j, k);
     crx = (D.spec_x && i == 1) ? (vel / mu) * dt / dx : vel * dt / dx / mu;
     facx = mu * (dx / dt);
   }
   if (fy) {
-    const R dy = R(2) / (D.msftx(i, j) + D.msftx(i, j - 1)) / R(D.rdy), mu = R(0.5) * (pd_mh(D, i, j, k) + pd_mh(D, i, j - 1, k)),
+    const R dy = R(2) / (D.msftx(i, j) + D.msftx(i, j - 1)) / D.r.rdy, mu = R(0.5) * (pd_mh(D, i, j, k) + pd_mh(D, i, j - 1, k)),
             vel = D.rv_m.ld(i, j, k);
     cry = vel * dt / dy / mu;
     facy = mu * (dy / dt);
   }
   if (zin) {
-    const R dz = R(2) / (R(D.rdnw[k]) + R(D.rdnw[k - 1])), mu = pd_mh(D, i, j, k), vel = D.ww_m.ld(i, j, k);
+    const R dz = R(2) / (D.r.rdnw[k] + D.r.rdnw[k - 1]), mu = pd_mh(D, i, j, k), vel = D.ww_m.ld(i, j, k);
     crz = vel * dt / dz / mu;
     facz = mu * (dz / dt);
   }
@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(PX) k_q_scale_pd(const __grid_constant__ Pack<
   int i, j, k;
   if (!thread_index<SH>(P, RG_MASS, Dp, i, j, k)) return;
   const Dom<R>& D = *Dp;
-  const R dt = R(rk == 1 ? D.dt / 3.0 : (rk == 2 ? 0.5 * D.dt : D.dt));
+  const R dt = rk == 1 ? D.r.dt3 : (rk == 2 ? D.r.dt2 : D.r.dt);
   const bool edge = (D.spec_x && (i == 0 || i == D.nx - 1)) || (D.spec_y && (j == 0 || j == D.ny - 1));
   const int n = blockIdx.y;  // the species
   if (n >= D.n_scalars) return;
@@ -635,13 +635,13 @@ __global__ void __launch_bounds__(PX) k_q_scale_pd(const __grid_constant__ Pack<
   }
   const R dhz0 = f[4](i, j, k), loz0 = f[5](i, j, k), dhz1 = f[4](i, j, k + 1), loz1 = f[5](i, j, k + 1);
   const R mxy = D.msftx(i, j) * D.msfty(i, j);
-  R hlow = R(D.rdx) * (lox1 - lox0);
-  if (D.do_y) hlow += R(D.rdy) * (loy1 - loy0);
-  const R ph_low = ((R(D.c1h[k]) * D.mub(i, j) + R(D.c2h[k])) + R(D.c1h[k]) * D.mu1(i, j, 0)) * qo(i, j, k) -
-                   dt * (mxy * hlow + D.msfty(i, j) * R(D.rdnw[k]) * (loz1 - loz0));
-  R hout = R(D.rdx) * ((dhx1 > 0 ? dhx1 : R(0)) - (dhx0 < 0 ? dhx0 : R(0)));
-  if (D.do_y) hout += R(D.rdy) * ((dhy1 > 0 ? dhy1 : R(0)) - (dhy0 < 0 ? dhy0 : R(0)));
-  const R out = mxy * hout + D.msfty(i, j) * R(D.rdnw[k]) * ((dhz1 < 0 ? dhz1 : R(0)) - (dhz0 > 0 ? dhz0 : R(0)));
+  R hlow = D.r.rdx * (lox1 - lox0);
+  if (D.do_y) hlow += D.r.rdy * (loy1 - loy0);
+  const R ph_low = ((D.r.c1h[k] * D.mub(i, j) + D.r.c2h[k]) + D.r.c1h[k] * D.mu1(i, j, 0)) * qo(i, j, k) -
+                   dt * (mxy * hlow + D.msfty(i, j) * D.r.rdnw[k] * (loz1 - loz0));
+  R hout = D.r.rdx * ((dhx1 > 0 ? dhx1 : R(0)) - (dhx0 < 0 ? dhx0 : R(0)));
+  if (D.do_y) hout += D.r.rdy * ((dhy1 > 0 ? dhy1 : R(0)) - (dhy0 < 0 ? dhy0 : R(0)));
+  const R out = mxy * hout + D.msfty(i, j) * D.r.rdnw[k] * ((dhz1 < 0 ? dhz1 : R(0)) - (dhz0 > 0 ? dhz0 : R(0)));
   const R flux_out = dt * out;
   R sc = 1;
   if (flux_out > ph_low) {
@@ -669,16 +669,16 @@ __device__ __noinline__ void q_update_pd_open(const Dom<R>& D, int n, R dt, int 
   R tend = R(0);
   if (ocol) tend = tend - open_scalar<R, 1>(D, D.q2[n], qo, D.ru_m, i, j, k);
   if (orow) tend = tend - open_scalar<R, 0>(D, D.q2[n], qo, D.rv_m, i, j, k);
-  tend = tend - R(D.rdnw[k]) * (dz1 - dz0 + loz1 - loz0);
+  tend = tend - D.r.rdnw[k] * (dz1 - dz0 + loz1 - loz0);
   if (!ocol) {
     const R dhx0 = f[0](i, j, k), lox0 = f[1](i, j, k), dhx1 = f[0](i + 1, j, k), lox1 = f[1](i + 1, j, k);
     const R dx0 = lim(dhx0, sc(i - 1, j, k), s0), dx1 = lim(dhx1, s0, sc(i + 1, j, k));
-    tend -= D.msftx(i, j) * (R(D.rdx) * (dx1 - dx0 + lox1 - lox0));
+    tend -= D.msftx(i, j) * (D.r.rdx * (dx1 - dx0 + lox1 - lox0));
   }
   if (D.do_y && !orow) {
     const R dhy0 = f[2](i, j, k), loy0 = f[3](i, j, k), dhy1 = f[2](i, j + 1, k), loy1 = f[3](i, j + 1, k);
     const R dy0 = lim(dhy0, sc(i, j - 1, k), s0), dy1 = lim(dhy1, s0, sc(i, j + 1, k));
-    tend -= D.msftx(i, j) * (R(D.rdy) * (dy1 - dy0 + loy1 - loy0));
+    tend -= D.msftx(i, j) * (D.r.rdy * (dy1 - dy0 + loy1 - loy0));
   }
   D.qn[n](i, j, k) = (m_full(D, k, mub, mu1) * qo(i, j, k) + dt * (tend * D.msfty(i, j))) / m_full(D, k, mub, mu2);
 }
@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(PX, 12) k_q_update_pd(const __grid_constant__ 
   int i, j, k;
   if (!thread_index<SH>(P, RG_MASS, Dp, i, j, k)) return;
   const Dom<R>& D = *Dp;
-  const R dt = R(rk == 1 ? D.dt / 3.0 : (rk == 2 ? 0.5 * D.dt : D.dt));
+  const R dt = rk == 1 ? D.r.dt3 : (rk == 2 ? D.r.dt2 : D.r.dt);
   const R mub = D.mub(i, j), mu1 = D.mu1(i, j, 0), mu2 = D.mu2(i, j, 0);
   const int n = blockIdx.y;  // the species
   if (n >= D.n_scalars) return;
@@ -714,12 +714,12 @@ __global__ void __launch_bounds__(PX, 12) k_q_update_pd(const __grid_constant__ 
   const R dx0 = lim(dhx0, sxm, s0), dx1 = lim(dhx1, s0, sxp);
   const R dz0 = (k == 0) ? R(0) : lim(dhz0, s0, szm);
   const R dz1 = (k + 1 == D.nz) ? R(0) : lim(dhz1, szp, s0);
-  R tend = -R(D.rdnw[k]) * (dz1 - dz0 + loz1 - loz0);
-  tend -= D.msftx(i, j) * (R(D.rdx) * (dx1 - dx0 + lox1 - lox0));
+  R tend = -D.r.rdnw[k] * (dz1 - dz0 + loz1 - loz0);
+  tend -= D.msftx(i, j) * (D.r.rdx * (dx1 - dx0 + lox1 - lox0));
   if (D.do_y) {
     const R dhy0 = f[2](i, j, k), loy0 = f[3](i, j, k), dhy1 = f[2](i, j + 1, k), loy1 = f[3](i, j + 1, k);
     const R dy0 = lim(dhy0, sc(i, j - 1, k), s0), dy1 = lim(dhy1, s0, sc(i, j + 1, k));
-    tend -= D.msftx(i, j) * (R(D.rdy) * (dy1 - dy0 + loy1 - loy0));
+    tend -= D.msftx(i, j) * (D.r.rdy * (dy1 - dy0 + loy1 - loy0));
   }
   D.qn[n](i, j, k) = (m_full(D, k, mub, mu1) * qo(i, j, k) + dt * (tend * D.msfty(i, j))) / m_full(D, k, mub, mu2);
 }

@@ -85,9 +85,9 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_ls_prep(const __g
         ph0 = D.ph2.ld(i, j, k);
         ph1 = D.ph2.ld(i, j, k + 1);
       }
-      if (has_u) D.ru(i, j, k) = div_msf(u2 * (R(D.c1h[k]) * muu + R(D.c2h[k])), msfuy);
-      if (has_v) D.rv(i, j, k) = v2 * (R(D.c1h[k]) * muv + R(D.c2h[k])) * mvxi;
-      if (has_w) D.rw(i, j, k) = div_msf(w2 * (R(D.c1f[k]) * mut + R(D.c2f[k])), msfty);
+      if (has_u) D.ru(i, j, k) = div_msf(u2 * (D.r.c1h[k] * muu + D.r.c2h[k]), msfuy);
+      if (has_v) D.rv(i, j, k) = v2 * (D.r.c1h[k] * muv + D.r.c2h[k]) * mvxi;
+      if (has_w) D.rw(i, j, k) = div_msf(w2 * (D.r.c1f[k] * mut + D.r.c2f[k]), msfty);
       if (has_m) {
         D.alt(i, j, k) = al + alb;
         D.php(i, j, k) = R(0.5) * (phb0 + phb1 + ph0 + ph1);
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_ls_prep(const __g
     R w = 0;
 #pragma unroll 4
     for (int k = 1; k < nz; ++k) {  // ww of level k into the slot of the divergence it consumed
-      w = w - R(D.dnw[k - 1]) * R(D.c1h[k - 1]) * dmdt - R(s_div[(k - 1) * CX + lane]);
+      w = w - D.r.dnw[k - 1] * D.r.c1h[k - 1] * dmdt - R(s_div[(k - 1) * CX + lane]);
       s_div[(k - 1) * CX + lane] = double(w);
     }
   }
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_ss_prep(const __g
       if (i < nx && j < nyv) D.muvs(i, j, 0) = mus_v;
     }
     CB_LOOP_U2(k, nz + 1) {  // KPrep (every load of a level before its first store)
-      const R c1h = k < nz ? R(D.c1h[k]) : R(0), c2h = k < nz ? R(D.c2h[k]) : R(0);
+      const R c1h = k < nz ? D.r.c1h[k] : R(0), c2h = k < nz ? D.r.c2h[k] : R(0);
       const bool has_u = j < ny && k < nz, has_v = i < nx && j < nyv && k < nz;
       R ui = 0, u1 = 0, muu = 0, msfuy = 1, vi = 0, v1 = 0, muv = 0, mvxi = 0;
       if (has_u) {
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_ss_prep(const __g
           D.c2a(i, j, k) = R(k::cpovcv) * (pb + pp) / alt;
         }
         D.w_save(i, j, k) = wi;
-        D.w2(i, j, k) = div_msf(((R(D.c1f[k]) * mts + R(D.c2f[k])) * w1 - (R(D.c1f[k]) * mut + R(D.c2f[k])) * wi), msfty);
+        D.w2(i, j, k) = div_msf(((D.r.c1f[k] * mts + D.r.c2f[k]) * w1 - (D.r.c1f[k] * mut + D.r.c2f[k]) * wi), msfty);
         D.ph_save(i, j, k) = phi;
         D.ph2(i, j, k) = ph1 - phi;
         D.ww1(i, j, k) = ww;
@@ -220,8 +220,8 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_ss_prep(const __g
   double* s_a = cb_array(0, nz);
   double* s_b = cb_array(1, nz);
   double* s_c = cb_array(2, nz);
-  const A dts = rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound;
-  const A cof_h = 0.5 * A(R(dts)) * k::g * (1.0 + A(R(D.epssm)));
+  const A dts = rk == 1 ? D.dt3 : D.dtsn;
+  const A cof_h = 0.5 * A(R(dts)) * k::g * (1.0 + A(D.r.epssm));
   const A cof = A(R(cof_h * cof_h));
   const A m = A(mut);
   auto mh = [&](int kk, A mm) { return D.c1h[kk] * mm + D.c2h[kk]; };
@@ -275,14 +275,14 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __gr
   const int nx = D.nx, ny = D.ny, nz = D.nz, nyv = D.nyv;
   const bool col = i < ilim;  // a column of the member (its faces' range)
   const bool mass = col && i < nx && j < ny;
-  const R dts = R(rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound);
+  const R dts = rk == 1 ? D.r.dt3 : D.r.dts;
   const R hd_dt = (rk == 3 && D.n_moist > 0) ? dts * R(nsmall) : R(0);
   // mu_ts of the neighbour columns: past the domain's edge the column that a halo fill would copy
   auto mts_at = [&](int ii, int jj) { return D.muts.ld(edge_col(ii, nx, D.bc_x), edge_col(jj, ny, D.bc_y), 0); };
   if (col) {
     CB_LOOP(k, nz + 1) {  // every load of a level before its first store
       const bool has_u = j < ny && k < nz, has_v = i < nx && j < nyv && k < nz;
-      const R c1h = k < nz ? R(D.c1h[k]) : R(0), c2h = k < nz ? R(D.c2h[k]) : R(0);
+      const R c1h = k < nz ? D.r.c1h[k] : R(0), c2h = k < nz ? D.r.c2h[k] : R(0);
       R u2 = 0, usv = 0, msfuy = 0, muu = 0, mts_u0 = 0, mts_u1 = 0;
       if (has_u) {
         u2 = D.u2(i, j, k);
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __gr
         D.v2(i, j, k) = (msfvx * v2 + vsv * (c1h * muv + c2h)) / (c1h * mus_v + c2h);
       }
       if (mass) {
-        D.w2(i, j, k) = (msfty * w2 + wsv * (R(D.c1f[k]) * m + R(D.c2f[k]))) / (R(D.c1f[k]) * mts + R(D.c2f[k]));
+        D.w2(i, j, k) = (msfty * w2 + wsv * (D.r.c1f[k] * m + D.r.c2f[k])) / (D.r.c1f[k] * mts + D.r.c2f[k]);
         D.ph2(i, j, k) = ph2 + phsv;
         D.ww(i, j, k) = ww + ww1;
         if (k < nz)
@@ -464,7 +464,7 @@ __global__ void __maxnreg__(64) k_ls_prep_lc(const __grid_constant__ Pack<R, NM>
   }
   if (has_m) {
     s_div[x] = double(ww_divv(D, i, j, k, ww_mu_u(D, i + 1, j), ww_mu_u(D, i, j), ww_mu_v(D, i, j + 1), ww_mu_v(D, i, j)));
-    s_c[x] = double(R(D.dnw[k]) * R(D.c1h[k]));
+    s_c[x] = double(D.r.dnw[k] * D.r.c1h[k]);
   }
   lc_bar();
   // KPrep3 while the column warp integrates (every load of a point before its first store)
@@ -481,9 +481,9 @@ __global__ void __maxnreg__(64) k_ls_prep_lc(const __grid_constant__ Pack<R, NM>
       ph0 = __ldg(D.ph2.p + o);
       ph1 = __ldg(D.ph2.p + o + D.ph2.sk);
     }
-    if (has_u) D.ru.p[oU] = div_msf(u2 * (R(D.c1h[k]) * muu + R(D.c2h[k])), msfuy);
-    if (has_v) D.rv.p[oV] = v2 * (R(D.c1h[k]) * muv + R(D.c2h[k])) * mvxi;
-    if (has_w) D.rw.p[o] = div_msf(w2 * (R(D.c1f[k]) * mut + R(D.c2f[k])), msfty);
+    if (has_u) D.ru.p[oU] = div_msf(u2 * (D.r.c1h[k] * muu + D.r.c2h[k]), msfuy);
+    if (has_v) D.rv.p[oV] = v2 * (D.r.c1h[k] * muv + D.r.c2h[k]) * mvxi;
+    if (has_w) D.rw.p[o] = div_msf(w2 * (D.r.c1f[k] * mut + D.r.c2f[k]), msfty);
     if (has_m) {
       D.alt.p[o] = al + alb;
       D.php.p[o] = R(0.5) * (phb0 + phb1 + ph0 + ph1);
@@ -567,7 +567,7 @@ __global__ void __maxnreg__(64) k_ss_prep_lc(const __grid_constant__ Pack<R, NM>
       if (k == 0) D.mu_save.p[o2] = mu;
     }
     // KPrep (every load of a point before its first store)
-    const R c1h = lm ? R(D.c1h[k]) : R(0), c2h = lm ? R(D.c2h[k]) : R(0);
+    const R c1h = lm ? D.r.c1h[k] : R(0), c2h = lm ? D.r.c2h[k] : R(0);
     R ui = 0, u1 = 0, muu = 0, msfuy = 1, vi = 0, v1 = 0, muv = 0, mvxi = 0;
     if (has_u) {
       ui = D.u2.p[oU];
@@ -619,7 +619,7 @@ __global__ void __maxnreg__(64) k_ss_prep_lc(const __grid_constant__ Pack<R, NM>
       ph_new = A(pn);
       s_ph[x] = ph_new;
       D.w_save.p[o] = wi;
-      D.w2.p[o] = div_msf(((R(D.c1f[k]) * mts + R(D.c2f[k])) * w1 - (R(D.c1f[k]) * mut + R(D.c2f[k])) * wi), msfty);
+      D.w2.p[o] = div_msf(((D.r.c1f[k] * mts + D.r.c2f[k]) * w1 - (D.r.c1f[k] * mut + D.r.c2f[k]) * wi), msfty);
       D.ph_save.p[o] = phi;
       D.ph2.p[o] = pn;
       D.ww1.p[o] = ww;
@@ -635,8 +635,8 @@ __global__ void __maxnreg__(64) k_ss_prep_lc(const __grid_constant__ Pack<R, NM>
     if (i < nx && j < nyv) D.muvs(i, j, 0) = mus_v;
   }
   if (mass) {  // calc_coef_w: the coefficients a, b, c of the level
-    const A dts = rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound;
-    const A cof_h = 0.5 * A(R(dts)) * k::g * (1.0 + A(R(D.epssm)));
+    const A dts = rk == 1 ? D.dt3 : D.dtsn;
+    const A cof_h = 0.5 * A(R(dts)) * k::g * (1.0 + A(D.r.epssm));
     const A cof = A(R(cof_h * cof_h));
     const A m = A(mut);
     auto mh = [&](int kk) { return D.c1h[kk] * m + D.c2h[kk]; };
@@ -692,7 +692,7 @@ __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int 
   const Dom<R>& D = lc_member<SH>(P, i, j, ilim);
   const int c = threadIdx.x, k = threadIdx.y;
   const int nx = D.nx, ny = D.ny, nz = D.nz;
-  const A dtsA = rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound;
+  const A dtsA = rk == 1 ? D.dt3 : D.dtsn;
   const R dts = R(dtsA);
   const bool pcol = i < nx && i < ilim && j < ny;  // a column of mass points
   const bool espec = pcol && edge_mass(D, i, j);
@@ -752,7 +752,7 @@ __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int 
       const A mtend = A(mt);
       const A mu_new = A(mu_old) + A(dts) * (dmdt + mtend);
       const R muts = mut + R(mu_new);
-      const R mav = R(0.5) * ((R(1) + R(D.epssm)) * R(mu_new) + (R(1) - R(D.epssm)) * R(A(mu_old)));
+      const R mav = R(0.5) * ((R(1) + D.r.epssm) * R(mu_new) + (R(1) - D.r.epssm) * R(A(mu_old)));
       D.mu2.p[o2] = R(mu_new);
       D.mudf.p[o2] = R(dmdt + mtend);
       D.muts.p[o2] = muts;
@@ -817,12 +817,12 @@ __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int 
   // KSumEdge: the east face (specified or open x) and the north face (specified or open y)
   if (lm && i < ilim && D.spec_x && i == nx && j < ny) {
     const R su = (first ? R(0) : D.ru_m.p[oU]) + __ldg(D.u2.p + oU);
-    const R cpl = (R(D.c1h[k]) * __ldg(D.muu.p + oU2) + R(D.c2h[k])) * __ldg(D.u_save.p + oU);
+    const R cpl = (D.r.c1h[k] * __ldg(D.muu.p + oU2) + D.r.c2h[k]) * __ldg(D.u_save.p + oU);
     D.ru_m.p[oU] = last ? su / rn + div_msf(cpl, D.msfuy(i, j)) : su;
   }
   if (lm && i < ilim && D.spec_y && j == ny && i < nx) {
     const R su = (first ? R(0) : D.rv_m.p[oV]) + __ldg(D.v2.p + oV);
-    const R cpl = (R(D.c1h[k]) * __ldg(D.muv.p + oV2) + R(D.c2h[k])) * __ldg(D.v_save.p + oV);
+    const R cpl = (D.r.c1h[k] * __ldg(D.muv.p + oV2) + D.r.c2h[k]) * __ldg(D.v_save.p + oV);
     D.rv_m.p[oV] = last ? su / rn + cpl * D.msfvx_inv(i, j) : su;
   }
   if (mass) {
@@ -856,7 +856,7 @@ __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int 
       msftx = D.msftx(i, j);
     }
     if (lm) {
-      const R c1h = R(D.c1h[k]), c2h = R(D.c2h[k]);
+      const R c1h = D.r.c1h[k], c2h = D.r.c2h[k];
       const R u_k = __ldg(D.u2.p + oU), usv = __ldg(D.u_save.p + oU), muu = __ldg(D.muu.p + oU2), msfuy = D.msfuy(i, j);
       const R rum = first ? R(0) : D.ru_m.p[oU];
       R v_k = 0, vsv = 0, muv = 0, mvxi = 0, rvm = 0;
@@ -877,14 +877,14 @@ __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int 
         const R* const pts = D.t_save.p + o;
         const R ts = __ldg(pts), ts_ip = __ldg(pts + edge_hi(i, nx, D.bc_x)), ts_im = __ldg(pts + edge_lo(i, nx, D.bc_x));
         const R fx = (u_ip + div_msf((c1h * muu_ip + c2h) * usv_ip, msfuy_ip)) - (u_k + cu);
-        R d = R(D.rdx) * fx;
-        hflux = R(0.5) * R(D.rdx) * (u_ip * (ts_ip + ts) - u_k * (ts + ts_im));
+        R d = D.r.rdx * fx;
+        hflux = R(0.5) * D.r.rdx * (u_ip * (ts_ip + ts) - u_k * (ts + ts_im));
         if (D.do_y) {
           const R v_jp = __ldg(D.v2.p + oV + face_hi(j, ny, D.bc_y) * sjV), vsv_jp = __ldg(D.v_save.p + oV + sjV);
           const R muv_jp = __ldg(D.muv.p + oV2 + D.muv.sj), mvxi_jp = D.msfvx_inv(i, j + 1);
           const R ts_jp = __ldg(pts + edge_hi(j, ny, D.bc_y) * sjM), ts_jm = __ldg(pts + edge_lo(j, ny, D.bc_y) * sjM);
-          d += R(D.rdy) * ((v_jp + (c1h * muv_jp + c2h) * vsv_jp * mvxi_jp) - (v_k + cv));
-          hflux += R(0.5) * R(D.rdy) * (v_jp * (ts_jp + ts) - v_k * (ts + ts_jm));
+          d += D.r.rdy * ((v_jp + (c1h * muv_jp + c2h) * vsv_jp * mvxi_jp) - (v_k + cv));
+          hflux += R(0.5) * D.r.rdy * (v_jp * (ts_jp + ts) - v_k * (ts + ts_jm));
         }
         dv = A(msftx * msfty * d);
         s1[x] = D.dnw[k] * dv;  // the term of the column sum
@@ -918,9 +918,9 @@ __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int 
     D.ww_m.p[o] = last ? sw / rn + ww1k : sw;
     if (lm) {
       const R ts = s_ts[x];
-      const R wd_kp = (k + 1 == nz) ? R(0) : R(s2[x + CB]) * (R(D.fnm[k + 1]) * s_ts[x + CB] + R(D.fnp[k + 1]) * ts);
-      const R wd_k = (k == 0) ? R(0) : wpp * (R(D.fnm[k]) * ts + R(D.fnp[k]) * s_ts[x - CB]);
-      tnew = tn - dts * msfty * (msftx * hflux + R(D.rdnw[k]) * (wd_kp - wd_k));
+      const R wd_kp = (k + 1 == nz) ? R(0) : R(s2[x + CB]) * (D.r.fnm[k + 1] * s_ts[x + CB] + D.r.fnp[k + 1] * ts);
+      const R wd_k = (k == 0) ? R(0) : wpp * (D.r.fnm[k] * ts + D.r.fnp[k] * s_ts[x - CB]);
+      tnew = tn - dts * msfty * (msftx * hflux + D.r.rdnw[k] * (wd_kp - wd_k));
       D.t2.p[o] = tnew;
       // t_2ave and the buoyancy term (advance_w in double in both forms: the explicit phi'' and w'' right-hand sides are
       // differences of nearly equal terms; in the FP64 form every conversion is the identity)
@@ -940,7 +940,7 @@ __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int 
     }
     // phi'' (LateralBC::update_ph_w, KUpdatePh :374-386)
     const R mts = R(sc[3 * CB]), mold = mts - dts * R(sc[CB]);
-    const R m_old = R(D.c1f[k]) * mold + R(D.c2f[k]), m_new = R(D.c1f[k]) * mts + R(D.c2f[k]);
+    const R m_old = D.r.c1f[k] * mold + D.r.c2f[k], m_new = D.r.c1f[k] * mts + D.r.c2f[k];
     const R pn = s_ph[x] * m_old / m_new + dts * s_pht[x] / m_new + s_phs[x] * (m_old / m_new - R(1));
     D.ph2.p[o] = pn;
     phn = A(pn);
@@ -1031,7 +1031,7 @@ __global__ void __maxnreg__(64) k_finish_lc(const __grid_constant__ Pack<R, NM> 
   double* const s_ph = lc_smem();
   const bool col = i < ilim && k <= nz, lm = k < nz;  // a column of the member (its faces' range)
   const bool mass = col && i < nx && j < ny, has_u = col && j < ny && lm, has_v = col && i < nx && j < nyv && lm;
-  const R dts = R(rk == 1 ? D.dt / 3.0 : D.dt / D.n_sound);
+  const R dts = rk == 1 ? D.r.dt3 : D.r.dts;
   const R hd_dt = (rk == 3 && D.n_moist > 0) ? dts * R(nsmall) : R(0);
   const int o = i + j * D.t2.sj + k * D.t2.sk, oU = i + j * D.u2.sj + k * D.u2.sk, oV = i + j * D.v2.sj + k * D.v2.sk;
   const int o2 = i + j * D.mu2.sj;
@@ -1039,7 +1039,7 @@ __global__ void __maxnreg__(64) k_finish_lc(const __grid_constant__ Pack<R, NM> 
   auto mts_at = [&](int ii, int jj) { return D.muts.ld(edge_col(ii, nx, D.bc_x), edge_col(jj, ny, D.bc_y), 0); };
   R mts = 0, mu_new = 0, tnew = 0, pn = 0;
   if (col) {  // every load of a point before its first store
-    const R c1h = lm ? R(D.c1h[k]) : R(0), c2h = lm ? R(D.c2h[k]) : R(0);
+    const R c1h = lm ? D.r.c1h[k] : R(0), c2h = lm ? D.r.c2h[k] : R(0);
     mts = mts_at(i, j);
     R u2 = 0, usv = 0, msfuy = 0, muu = 0, mts_im = 0;
     if (has_u) {
@@ -1083,7 +1083,7 @@ __global__ void __maxnreg__(64) k_finish_lc(const __grid_constant__ Pack<R, NM> 
       D.v2.p[oV] = (msfvx * v2 + vsv * (c1h * muv + c2h)) / (c1h * mus_v + c2h);
     }
     if (mass) {
-      D.w2.p[o] = (msfty * w2 + wsv * (R(D.c1f[k]) * m + R(D.c2f[k]))) / (R(D.c1f[k]) * mts + R(D.c2f[k]));
+      D.w2.p[o] = (msfty * w2 + wsv * (D.r.c1f[k] * m + D.r.c2f[k])) / (D.r.c1f[k] * mts + D.r.c2f[k]);
       pn = ph2 + phsv;
       D.ph2.p[o] = pn;
       s_ph[x] = double(pn);
@@ -1173,11 +1173,11 @@ __global__ void __launch_bounds__(CX * NW) k_w_surface(const __grid_constant__ P
   int i, j, ilim;
   const Dom<R>& D = cb_member(P, RG_COLS_MASS, i, j, ilim);
   if (threadIdx.y != 0 || i >= ilim) return;
-  const R cf1 = R(D.cf1), cf2 = R(D.cf2), cf3 = R(D.cf3);
-  const R ws = D.msfty(i, j) * R(0.5) * R(D.rdy) *
+  const R cf1 = D.r.cf1, cf2 = D.r.cf2, cf3 = D.r.cf3;
+  const R ws = D.msfty(i, j) * R(0.5) * D.r.rdy *
                    ((D.ht(i, j + 1) - D.ht(i, j)) * (cf1 * D.v2(i, j + 1, 0) + cf2 * D.v2(i, j + 1, 1) + cf3 * D.v2(i, j + 1, 2)) +
                     (D.ht(i, j) - D.ht(i, j - 1)) * (cf1 * D.v2(i, j, 0) + cf2 * D.v2(i, j, 1) + cf3 * D.v2(i, j, 2))) +
-               D.msftx(i, j) * R(0.5) * R(D.rdx) *
+               D.msftx(i, j) * R(0.5) * D.r.rdx *
                    ((D.ht(i + 1, j) - D.ht(i, j)) * (cf1 * D.u2(i + 1, j, 0) + cf2 * D.u2(i + 1, j, 1) + cf3 * D.u2(i + 1, j, 2)) +
                     (D.ht(i, j) - D.ht(i - 1, j)) * (cf1 * D.u2(i, j, 0) + cf2 * D.u2(i, j, 1) + cf3 * D.u2(i, j, 2)));
   D.w2(i, j, 0) = ws;
