@@ -226,7 +226,7 @@ constexpr int kWideBlocks = 250, kWide16Blocks = 1000;
 // their shared memory: k_ac's level arrays of doubles and of the fields' type and its per-column scalars, the others'
 // level arrays of doubles
 constexpr int kAcArrays = 5, kAcFields = 13, kAcScalars = 8, kLsArrays = 2, kSsArrays = 5;
-constexpr int kCbArrays = 6;  // shared-memory level arrays of the acoustic column block: kCbArrays x (nz + 2) x CX doubles
+constexpr int kCbArrays = 6;  // shared-memory level arrays of the microphysics' column block: kCbArrays x (nz + 2) x CX doubles
 __host__ __device__ __forceinline__ int cdiv(int a, int b) { return (a + b - 1) / b; }
 
 // ---- WRF flux statement functions (src/dyn/kernels_common.hpp:11-105) ----

@@ -26,36 +26,21 @@ __device__ __forceinline__ R mh_(const Dom<R>& D, int k, R m) { return D.r.c1h[k
 template <class R>
 __device__ __forceinline__ R mf_(const Dom<R>& D, int k, R m) { return D.r.c1f[k] * m + D.r.c2f[k]; }
 
-// p_rho_point (small_step.cpp:97-112): calc_p_rho, with smdiv divergence damping when damp.
-// The mixed form evaluates it in double (the hydrostatic p'' / al'' relation).
-// RO: alt, t_save and c2a are read-only in the calling kernel (the read-only load path). ph_k, ph_kp: the
-// values of phi'' at levels k and k + 1.
-template <bool RO, class R>
-__device__ __forceinline__ void p_rho_point_ph(const Dom<R>& D, int i, int j, int k, bool damp, R ph_k_in, R ph_kp_in) {
+// p_rho_point (small_step.cpp:97-112): calc_p_rho of small_step_prep, without divergence damping (the substeps' damped
+// form is part of k_ac). The mixed form evaluates it in double (the hydrostatic p'' / al'' relation).
+template <class R>
+__device__ __forceinline__ void p_rho_point(const Dom<R>& D, int i, int j, int k) {
   using A = double;
   // every load before the first store
   const A c1h = D.c1h[k];
-  const A muts = A(D.muts(i, j, 0)), alt = A(RO ? D.alt.ld(i, j, k) : D.alt(i, j, k)), mu = A(D.mu2(i, j, 0));
-  const A ts = A(RO ? D.t_save.ld(i, j, k) : D.t_save(i, j, k));
-  const A ph_kp = A(ph_kp_in), ph_k = A(ph_k_in), t2 = A(D.t2(i, j, k));
-  const A c2a = A(RO ? D.c2a.ld(i, j, k) : D.c2a(i, j, k));
-  const A pm1 = damp ? A(D.pm1(i, j, k)) : A(0);
+  const A muts = A(D.muts(i, j, 0)), alt = A(D.alt(i, j, k)), mu = A(D.mu2(i, j, 0)), ts = A(D.t_save(i, j, k));
+  const A ph_kp = A(D.ph2(i, j, k + 1)), ph_k = A(D.ph2(i, j, k)), t2 = A(D.t2(i, j, k)), c2a = A(D.c2a(i, j, k));
   const A m = c1h * muts + A(D.c2h[k]);
   const A a = -((1. / m) * (alt * (c1h * mu) + A(D.rdnw[k]) * (ph_kp - ph_k)));
-  A pp = c2a * (alt * (t2 - c1h * mu * ts) / (m * (k::t0 + ts)) - a);
+  const A pp = c2a * (alt * (t2 - c1h * mu * ts) / (m * (k::t0 + ts)) - a);
   D.al(i, j, k) = R(a);
-  if (damp) {
-    const A ptmp = pp;
-    pp = pp + A(D.smdiv) * (pp - pm1);
-    D.pm1(i, j, k) = R(ptmp);
-  } else {
-    D.pm1(i, j, k) = R(pp);
-  }
+  D.pm1(i, j, k) = R(pp);
   D.p(i, j, k) = R(pp);
-}
-template <bool RO, class R>
-__device__ __forceinline__ void p_rho_point(const Dom<R>& D, int i, int j, int k, bool damp) {
-  p_rho_point_ph<RO>(D, i, j, k, damp, D.ph2(i, j, k), D.ph2(i, j, k + 1));
 }
 
 // The acoustic substeps read the fields that they advance at most one point away, so at the domain's edges they take the

@@ -1,9 +1,10 @@
 // SPDX-License-Identifier: GPL-3.0-or-later
-// Column-block kernels: a CTA holds CX neighbouring columns along i (the lanes, so every global access is
-// coalesced along i) and CNW warps. The pointwise work of the levels is split over the warps; the
-// vertical recurrences -- column sums, running integrals, the tridiagonal sweeps -- run on warp 0, one lane
-// per column, in the reference's order, on per-level terms staged in shared memory. Every value is the
-// same expression as the reference's column functor, so the results are bit-identical to it.
+// Column kernels. Two forms. A column block holds CX neighbouring columns along i (the lanes, so every global access is
+// coalesced along i) and CNW or 2 CNW warps that take its levels in turn; the vertical recurrences -- column sums, running
+// integrals, eliminations -- run on warp 0, one lane per column. A level-thread block holds fewer columns and a thread for
+// each of their levels, and runs the recurrences on a warp of its own. Both run them in the reference's order, on per-level
+// terms staged in shared memory; every value is the same expression as the reference's column functor, so the results are
+// bit-identical to it.
 #pragma once
 
 #include "kernels_ac.cuh"
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_ss_prep(const __g
   auto mf = [&](int kk, A mm) { return D.c1f[kk] * mm + D.c2f[kk]; };
   auto cq1 = [&](int kk) { return A(R(1) / (R(1) + cqw_(D, i, j, kk))); };
   if (mass) {
-    CB_LOOP(k, nz) p_rho_point<false>(D, i, j, k, false);
+    CB_LOOP(k, nz) p_rho_point(D, i, j, k);
     // calc_coef_w: the pointwise coefficients a, b, c of each level
     CB_LOOP(k, nz + 1) {
       A a = 0, b = 0, cc = 0;
