@@ -362,7 +362,7 @@ template <class R, int NM>
 void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
   const Member& M0 = h->m[0];
   bool lbc = false, terrain = false, scalars = false, any_pd = false, mp = false, open = false, dampkm = false,
-       smag = false, any_plain = false;
+       smag = false, any_plain = false, overlap = false;
   // The acoustic substeps take the points past a domain's edge from the domain itself (edge_lo, edge_hi, face_hi, edge_col),
   // so the fills before and between them (H_SS0, H_UV, H_AC) are left out and the fills after them (H_POST, H_FIN) refresh
   // those halos before anything reads them. A decomposed domain runs them: its patches read each other's points there.
@@ -378,6 +378,7 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
     open |= M.g.bc_x == CW_BC_OPEN || M.g.bc_y == CW_BC_OPEN;
     dampkm |= M.o.damp_opt == 1 && M.o.diff_opt == 1;
     smag |= M.o.km_opt == 4 && M.o.diff_opt == 1;
+    overlap |= M.o.lbc && relax_overlaps(M.g.nx, M.g.ny);
     mp |= M.o.mp_physics != 0;
     terrain |= !M.o.flat;
     scalars |= M.o.n_scalars > 0;
@@ -408,6 +409,7 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
       L.halo(cw_handle::H_XK);
     }
     if (rk == 1) L.run_t("k_tendf_rk1", RG_STAG, 1, KV(k_tendf_rk1), d);
+    if (rk == 1 && overlap) L.run("k_relax_rest", RG_STAG, k_relax_rest<R, NM>, d, 0);
     if constexpr (sizeof(R) == 8) {  // FP64: the tendencies in two launches (-1.4 % per step); mixed: one (faster)
       if (open) {
         L.run_t("k_tend", RG_STAG, 1, KV_OP2(k_tend, true, 3), d, rk);
@@ -439,6 +441,7 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
     L.halo(cw_handle::H_FIN);
     if (scalars) {
       if (rk == 1) L.run_t("k_q_tendf_rk1", RG_MASS, nq, KV(k_q_tendf_rk1), d);
+      if (rk == 1 && overlap) L.run("k_relax_rest", RG_STAG, k_relax_rest<R, NM>, d, 1);
       // at rk 3 the PD species take k_q_*_pd: the plain update runs only when some species is not PD
       if (rk != 3 || any_plain || !any_pd) {
         // the TMA-staged update where the tuner chose it; while tuning, the point kernel in the first round of

@@ -866,8 +866,8 @@ __device__ void relax_terms(const Dom<R>& D, const V3<R>& f, const double* c1, c
   fb = R(D.gcx[b]) * (fls1 + fls2 + fls3 + fls4 - R(4) * fls0);
 }
 
-// The ring point (side, row b, pos) of (i, j) when it lies in rows b_lo .. b_hi of the variable's ring;
-// then fa, fb of its relaxation term (relax_terms).
+// The ring point (side, row b, pos) of (i, j) when the row of its nearest side is one of rows 1 .. 3 of the variable's
+// ring; then fa, fb of its relaxation term (relax_terms).
 template <class R, bool Two>
 __device__ __forceinline__ bool relax_at(const Dom<R>& D, const V3<R>& f, const double* c1, const double* c2,
                                          const Slabs<R>& s, Ring r, int i, int j, int k, R& fa, R& fb) {
@@ -875,6 +875,27 @@ __device__ __forceinline__ bool relax_at(const Dom<R>& D, const V3<R>& f, const 
   if (!ring_locate(r.ibe, r.jbe, i, j, side, b, pos) || b < 1 || b > 3) return false;
   relax_terms<R, Two>(D, f, c1, c2, s, r, pos, side, b, k, i, j, fa, fb);
   return true;
+}
+// Rows 1 .. 3 of opposite sides overlap in some variable of an nx x ny domain (the mass points' ring has nx x ny points)
+__host__ __device__ __forceinline__ bool relax_overlaps(int nx, int ny) { return nx < 8 || ny < 8; }
+// The relaxation terms that relax_at leaves out: on a ring of fewer than 8 points along a direction the rows of opposite
+// sides overlap, and a point takes a term of every row 1 .. 3 that it lies in. add(fa, fb) for each of them but relax_at's
+// (the row of its nearest side, the first in the reference's order), in that order: the rows from the edge inwards, the
+// sides S, N, W, E of each.
+template <class R, bool Two, class Add>
+__device__ __forceinline__ void relax_rest(const Dom<R>& D, const V3<R>& f, const double* c1, const double* c2,
+                                           const Slabs<R>& s, Ring r, int i, int j, int k, Add add) {
+  int side0, b0, pos0;
+  if (!ring_locate(r.ibe, r.jbe, i, j, side0, b0, pos0)) b0 = -1;
+#pragma unroll 1
+  for (int n = 0; n < 12; ++n) {
+    const int side = n % 4, b = 1 + n / 4, pos = side <= 1 ? i : j;
+    int ri, rj;
+    if (!r.map(pos, side, b, ri, rj) || ri != i || rj != j || (side == side0 && b == b0)) continue;
+    R fa, fb;
+    relax_terms<R, Two>(D, f, c1, c2, s, r, pos, side, b, k, i, j, fa, fb);
+    add(fa, fb);
+  }
 }
 // (i, j) in the spec zone (row 0) of the ring: slab index sl and position pos of its boundary value
 __device__ __forceinline__ bool spec_at(Ring r, int i, int j, int& sl, int& pos) {
@@ -1592,6 +1613,59 @@ __global__ void __launch_bounds__(PX, 10) k_tendf_rk1(const __grid_constant__ Pa
       if (relax_at<R, true>(D, D.mu2, nullptr, nullptr, D.lbc_var[4], ring_for(nx, ny, 'm'), i, j, 0, fa, fb)) tm += fa - fb;
       D.mu_tend(i, j, 0) = tm;
     }
+  }
+}
+
+// The relaxation terms that k_tendf_rk1 (scalars = 0) and k_q_tendf_rk1 (scalars = 1) leave out, added to the held
+// tendencies after them: only members of fewer than 8 points along a direction have any (relax_rest), and only steps with
+// such a member launch it, so that the kernels that every step runs stay as small as one term needs (with the loop over
+// the sides in them: 188 instead of 68 bytes of spills in k_tendf_rk1, 72 instead of 48 registers in k_q_tendf_rk1).
+template <class R, int NM>
+__global__ void __launch_bounds__(PX) k_relax_rest(const __grid_constant__ Pack<R, NM> P, int scalars) {
+  const Dom<R>* Dp;
+  int i, j, k;
+  if (!thread_index<0>(P, RG_STAG, Dp, i, j, k)) return;
+  const Dom<R>& D = *Dp;
+  const int nx = D.nx, ny = D.ny, nz = D.nz;
+  if (!D.lbc || !relax_overlaps(nx, ny)) return;
+  const bool cell = i < nx && j < ny;
+  if (scalars) {
+    const Ring rq = ring_for(nx, ny, 'q');
+    int sl, pos;
+    if (!cell || k >= nz || spec_at(rq, i, j, sl, pos)) return;
+    for (int n = 0; n < D.n_scalars; ++n)
+      if (D.lbc_q[n].have) {
+        R t = D.qtf[n](i, j, k);
+        relax_rest<R, false>(D, D.q2[n], D.c1h, D.c2h, D.lbc_q[n], rq, i, j, k, [&](R fa, R fb) { t = t + fa - fb; });
+        D.qtf[n](i, j, k) = t;
+      }
+    return;
+  }
+  if (j < ny && k < nz) {
+    R t = D.ru_tendf(i, j, k);
+    relax_rest<R, false>(D, D.ru, nullptr, nullptr, D.lbc_var[0], ring_for(nx, ny, 'u'), i, j, k,
+                         [&](R fa, R fb) { t += (fa - fb) * D.msfuy(i, j); });
+    D.ru_tendf(i, j, k) = t;
+  }
+  if (i < nx && j < D.nyv && k < nz) {
+    R t = D.rv_tendf(i, j, k);
+    relax_rest<R, false>(D, D.rv, nullptr, nullptr, D.lbc_var[1], ring_for(nx, ny, 'v'), i, j, k,
+                         [&](R fa, R fb) { t += (fa - fb) * D.msfvx(i, j); });
+    D.rv_tendf(i, j, k) = t;
+  }
+  if (!cell) return;
+  R t = D.ph_tendf(i, j, k);
+  relax_rest<R, false>(D, D.ph2, D.c1f, D.c2f, D.lbc_var[3], ring_for(nx, ny, 'h'), i, j, k, [&](R fa, R fb) { t += fa - fb; });
+  D.ph_tendf(i, j, k) = t;
+  if (k < nz) {
+    t = D.t_tendf(i, j, k);
+    relax_rest<R, false>(D, D.t2, D.c1h, D.c2h, D.lbc_var[2], ring_for(nx, ny, 't'), i, j, k, [&](R fa, R fb) { t += fa - fb; });
+    D.t_tendf(i, j, k) = t;
+  }
+  if (k == 0) {
+    t = D.mu_tend(i, j, 0);
+    relax_rest<R, true>(D, D.mu2, nullptr, nullptr, D.lbc_var[4], ring_for(nx, ny, 'm'), i, j, 0, [&](R fa, R fb) { t += fa - fb; });
+    D.mu_tend(i, j, 0) = t;
   }
 }
 

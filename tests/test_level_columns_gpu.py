@@ -13,8 +13,9 @@ from test_parity_gpu import compare_all, run_pair
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny,nz", [(9, 10, 3), (10, 9, 7), (15, 9, 30), (16, 9, 31), (17, 9, 32), (9, 9, 63),
-                                      (23, 9, 64), (12, 9, 123), (11, 9, 126)])
+@pytest.mark.parametrize("nx,ny,nz", [(7, 8, 3), (8, 7, 7), (9, 10, 3), (10, 9, 7), (15, 9, 30), (16, 8, 31), (16, 9, 31),
+                                      (17, 8, 32), (17, 9, 32), (9, 8, 63), (9, 9, 63), (23, 7, 64), (23, 9, 64), (12, 8, 123),
+                                      (12, 9, 123), (11, 9, 126)])
 def test_lam_levels_and_widths(nx, ny, nz):
     case = lam_case(nx=nx, ny=ny, nz=nz, n_moist=2, n_scalars=2, seed=nx + nz)
     dom, orc = run_pair(case, 2)
