@@ -217,7 +217,13 @@ struct cw_handle {
   bool autotune = false, tuned = false;  // (kTuneRounds steps per shape)
   int tuning_shape = -1, tune_steps_done = 0;
   std::vector<std::pair<std::string, int>> shape_choice;
-  std::vector<std::pair<std::string, std::array<double, kNumShapes>>> tune_ms;
+  struct ShapeTimes {  // a kernel's times in each shape that it ran in, summed over n steps
+    std::string name;
+    std::array<double, kNumShapes> ms{};
+    std::array<int, kNumShapes> n{};
+    double mean(int sh) const { return ms[size_t(sh)] / n[size_t(sh)]; }
+  };
+  std::vector<ShapeTimes> tune_ms;
   bool profiling = false;
   std::vector<std::pair<const char*, std::pair<cudaEvent_t, cudaEvent_t>>> prof_ev;
   std::vector<std::string> prof_names;

@@ -720,7 +720,14 @@ void invalidate_graph(cw_handle* h) {
   h->graph_ok = false;
 }
 
-// one eager step with every tunable point kernel in block shape `shape`, each launch timed by events
+// the shape that kernel `name` runs in when shape sh is asked for
+int effective_shape(const cw_handle* h, const std::string& name, int sh) {
+  if (name == "k_ac") return ac_shape(sh, h->nzmax);
+  if (name == "k_ls_prep" || name == "k_ss_prep" || name == "k_finish") return col_shape(sh, h->nzmax);
+  return sh;
+}
+
+// one eager step with every tunable kernel in block shape `shape`, each launch timed by events
 void tune_step(cw_handle* h, int shape) {
   auto saved = std::move(h->prof_ev);
   h->prof_ev.clear();
@@ -738,17 +745,23 @@ void tune_step(cw_handle* h, int shape) {
   h->profiling = was;
   h->tuning_shape = -1;
   CW_CUDA(cudaStreamSynchronize(h->stream));
+  std::vector<std::string> seen;  // the kernels of this step
   for (auto& [name, ev] : h->prof_ev) {
     float ms = 0;
     CW_CUDA(cudaEventElapsedTime(&ms, ev.first, ev.second));
     cudaEventDestroy(ev.first);
     cudaEventDestroy(ev.second);
-    auto it = std::find_if(h->tune_ms.begin(), h->tune_ms.end(), [&](const auto& e) { return e.first == name; });
+    auto it = std::find_if(h->tune_ms.begin(), h->tune_ms.end(), [&](const auto& e) { return e.name == name; });
     if (it == h->tune_ms.end()) {
-      h->tune_ms.push_back({name, {}});
+      h->tune_ms.push_back({name});
       it = h->tune_ms.end() - 1;
     }
-    it->second[size_t(shape)] += ms;
+    const size_t sh = size_t(effective_shape(h, name, shape));
+    it->ms[sh] += ms;
+    if (std::find(seen.begin(), seen.end(), it->name) == seen.end()) {
+      seen.push_back(it->name);
+      ++it->n[sh];
+    }
   }
   h->prof_ev = std::move(saved);
   h->launches_last += L.count;
@@ -759,14 +772,14 @@ void tune_step(cw_handle* h, int shape) {
 // one round of steps, in every shape)
 void finish_tuning(cw_handle* h) {
   h->shape_choice.clear();
-  float best_update = -1, best_march = -1;
-  for (const auto& [name, ms] : h->tune_ms) {
-    int best = 0;
-    for (int sh = 1; sh < kNumShapes; ++sh)
-      if (ms[size_t(sh)] < ms[size_t(best)]) best = sh;
-    h->shape_choice.push_back({name, best});
-    if (name == "k_q_update") best_update = ms[size_t(best)];
-    if (name == "k_q_march") best_march = ms[size_t(best)];
+  double best_update = -1, best_march = -1;
+  for (const auto& t : h->tune_ms) {
+    int best = -1;
+    for (int sh = 0; sh < kNumShapes; ++sh)
+      if (t.n[size_t(sh)] > 0 && (best < 0 || t.mean(sh) < t.mean(best))) best = sh;
+    h->shape_choice.push_back({t.name, best});
+    if (t.name == "k_q_update") best_update = t.mean(best);
+    if (t.name == "k_q_march") best_march = t.mean(best);
   }
   h->q_march = best_march >= 0 && best_update >= 0 && best_march < best_update;
   h->tuned = true;
@@ -2054,7 +2067,7 @@ int cw_autotune_choice(cw_handle* h, const char* kernel, int* shape) {
   *shape = -1;
   if (!h->tuned) return 0;
   for (const auto& [n, sh] : h->shape_choice)
-    if (n == kernel) *shape = sh;
+    if (n == kernel) *shape = effective_shape(h, n, sh);
   return 0;
 }
 int cw_use_device(int device) {

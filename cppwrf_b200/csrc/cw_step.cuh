@@ -304,9 +304,7 @@ struct Launcher {
               const Packs<R, NM>& ps, Args... args) {
     flush();
     if (plan) return;
-    int sh = std::max(0, shape_for(name));
-    if (lc_threads(sh, h->nzmax) > kLcMaxThreads) sh = 0;
-    if (lc_threads(sh, h->nzmax) > kLcMaxThreads) sh = 2;
+    const int sh = ac_shape(std::max(0, shape_for(name)), h->nzmax);
     launch_lc(name, sh, arrays, fields, scalars, kerns[size_t(sh)], ps, args...);
   }
   template <class R, int NM, class K, class... Args>
@@ -336,7 +334,7 @@ struct Launcher {
       for (const auto& b : ps.blocks) nb += b[size_t(RG_COLS_STAG)][0];
       sh = nb < kWideBlocks ? 2 : (recurrence && nb >= kWide16Blocks ? 1 : 0);
     }
-    if (sh == 2 && lc_threads(0, h->nzmax) > kLcMaxThreads) sh = 1;
+    sh = col_shape(sh, h->nzmax);
     if (sh == 2) launch_lc(name, 0, lc_arrays, 0, 8, lc, ps, args...);
     else launch_cb(name, RG_COLS_STAG, arrays, wide[size_t(sh)], cb_warps(sh), ps, args...);
   }

@@ -216,6 +216,14 @@ __host__ __device__ constexpr int cb_minblocks(int nw) { return nw == CNW ? 3 : 
 __host__ __device__ constexpr int lc_cols(int s) { return s == 0 ? 8 : (s == 1 ? 16 : 4); }
 __host__ __device__ constexpr int lc_threads(int s, int nz) { return (lc_cols(s) * (nz + 1) + 31) / 32 * 32 + 32; }
 constexpr int kLcMaxThreads = 1024;
+// the shape that a column kernel runs in when sh is asked for: the shapes whose blocks would have more than kLcMaxThreads
+// threads at nz levels are replaced, k_ac's by narrower ones (16 columns above 61 levels by 8, 8 above 123 by 4), the
+// level-thread form of the preparation and finish kernels above 123 levels by rows of 32 columns x 16 warps
+__host__ __device__ constexpr int ac_shape(int sh, int nz) {
+  if (lc_threads(sh, nz) > kLcMaxThreads) sh = 0;
+  return lc_threads(sh, nz) > kLcMaxThreads ? 2 : sh;
+}
+__host__ __device__ constexpr int col_shape(int sh, int nz) { return sh == 2 && lc_threads(0, nz) > kLcMaxThreads ? 1 : sh; }
 // Where the preparation and finish kernels change form, in blocks of 32 columns over the launch's rows. Below kWideBlocks
 // (under two such blocks per SM) the latency of a column's levels in turn is what they take, and a thread per level is
 // faster: k_ls_prep, k_ss_prep, k_finish 33 / 49 / 57 -> 11 / 19 / 15 us at 200 x 100 (7 blocks), 17 / 27 / 30 -> 15 / 23

@@ -218,8 +218,10 @@ int cw_check_div_const(unsigned long long n, unsigned long long seed, unsigned l
  * in one of its shapes -- a point kernel's block of 0: 128 x 1, 1: 64 x 2, 2: 32 x 4 points along i x j, a column
  * kernel's 0: 32 columns x 8 warps, 1: 32 x 16, 2: 8 columns with a thread per level (the acoustic kernel's, a thread per
  * level always: 8, 16 or 4 columns) -- two steps per shape (orders 0 1 2, then 2 1 0), timed per launch; afterwards each
- * kernel keeps its fastest shape and the step is captured again. The tuning steps are ordinary steps: every shape computes
- * the same values. Calling it again re-tunes. cw_autotune_choice gives a kernel's chosen shape (-1 before the tuning has finished). */
+ * kernel keeps its fastest shape and the step is captured again. A shape whose blocks would be too large at the handle's
+ * largest nz (16 columns above 61 levels, 8 with a thread per level above 123) runs as another one and counts as that
+ * one. The tuning steps are ordinary steps: every shape computes the same values. Calling it again re-tunes.
+ * cw_autotune_choice gives a kernel's chosen shape (-1 before the tuning has finished). */
 int cw_set_autotune(cw_handle* h, int on);
 /* LargeStep::cfl_max (src/dyn/large_step.cpp:865-877), the maxima behind RK3::on_cfl (rk3.hpp) that the reference's
  * adaptive time step (src/cases/adapt_timestep.cpp) and w_damp read: with on = 1 every step records, after each RK

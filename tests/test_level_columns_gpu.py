@@ -48,3 +48,17 @@ def test_every_tuned_shape_gives_the_same_bits(nz, precision):
     b = Domain(case.g, case.o).upload_case(case).step(6)
     for name in capi.STATE_FIELDS:
         assert np.array_equal(a.field(name).view(np.uint64), b.field(name).view(np.uint64)), name
+
+
+@pytest.mark.parametrize("nz", [61, 70, 124, 126])
+def test_reported_shape_is_the_one_that_ran(nz):
+    """Where a shape's block does not fit, the kernel runs (and the tuner reports) another one: k_ac's 16 columns above 61
+    levels and its 8 above 123, the level-thread form of the other column kernels above 123. The tuner measures no shape
+    that did not run, however often it is asked."""
+    case = lam_case(nx=12, ny=9, nz=nz, n_moist=1, n_scalars=1, seed=4)
+    d = Domain(case.g, case.o).upload_case(case)
+    for _ in range(4):
+        d.set_autotune(True).step(6)
+        assert d.autotune_choice("k_ac") in ((0, 1, 2) if nz <= 61 else (0, 2) if nz <= 123 else (2,))
+        for k in ("k_ls_prep", "k_ss_prep", "k_finish"):
+            assert d.autotune_choice(k) in ((0, 1, 2) if nz <= 123 else (0, 1)), k
