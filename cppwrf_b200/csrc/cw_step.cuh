@@ -332,7 +332,7 @@ struct Launcher {
     if (sh < 0) {
       int nb = 0;
       for (const auto& b : ps.blocks) nb += b[size_t(RG_COLS_STAG)][0];
-      sh = nb < kWideBlocks ? 2 : (recurrence && nb >= kWide16Blocks ? 1 : 0);
+      sh = nb < kWideBlocks ? 2 : (recurrence && prep_wide16(nb, h->nzmax, arrays) ? 1 : 0);
     }
     sh = col_shape(sh, h->nzmax);
     if (sh == 2) launch_lc(name, 0, lc_arrays, 0, 8, lc, ps, args...);

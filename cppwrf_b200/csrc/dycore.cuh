@@ -229,13 +229,28 @@ __host__ __device__ constexpr int col_shape(int sh, int nz) { return sh == 2 && 
 // faster: k_ls_prep, k_ss_prep, k_finish 33 / 49 / 57 -> 11 / 19 / 15 us at 200 x 100 (7 blocks), 17 / 27 / 30 -> 15 / 23
 // / 19 us at 65 x 63 x 40 (192). Above it, their loads and stores are what they take, and rows of 32 columns are: 35 / 41
 // / 47 against 43 / 58 / 43 us at 119 x 89 x 44 (360 blocks), 129 / 185 / 190 against 172 / 248 / 188 at 200 x 200 x 60.
-// From kWide16Blocks on, 16 warps a block instead of 8: 129 against 153 and 185 against 203 us at 200 x 200 x 60.
-constexpr int kWideBlocks = 250, kWide16Blocks = 1000;
+constexpr int kWideBlocks = 250;
 // their shared memory: k_ac's level arrays of doubles and of the fields' type and its per-column scalars, the others'
 // level arrays of doubles
 constexpr int kAcArrays = 5, kAcFields = 13, kAcScalars = 8, kLsArrays = 2, kSsArrays = 5;
 constexpr int kCbArrays = 6;  // shared-memory level arrays of the microphysics' column block: kCbArrays x (nz + 2) x CX doubles
-__host__ __device__ __forceinline__ int cdiv(int a, int b) { return (a + b - 1) / b; }
+__host__ __device__ __forceinline__ constexpr int cdiv(int a, int b) { return (a + b - 1) / b; }
+// Whether k_ls_prep and k_ss_prep run their nb blocks of 32 columns (at least kWideBlocks) with 16 warps instead of 8; `arrays`:
+// the shared level arrays of the kernel. An SM holds three blocks of 8 warps or two of 16 (cb_minblocks), which advance the
+// levels equally fast together, so what decides is how full the last wave of blocks is: 16 warps where two blocks times
+// their waves are fewer. us per launch, k_ls_prep and k_ss_prep, 8 / 16 warps: 200 x 200 x 48 (1407 blocks) 106 / 95 and 162 /
+// 150, 250 x 250 x 60 (2008) 170 / 162 and 290 / 279; the other way 100 x 320 x 60 (1284) 98 / 105 and 159 / 171, 300 x 300 x 60
+// mixed (3010) 184 / 187 and 296 / 305. Below 28 levels 16 warps have too few each (400 x 400 x 8: 89 / 117 and 117 / 142,
+// x 20: 167 / 193 and 234 / 270). Where shared memory leaves two blocks of either form (k_ss_prep from 98 levels on) the
+// one with more warps: 100 x 320 x 100 349 / 286, 119 x 89 x 100 139 / 113.
+constexpr int kSMs = 148, kWide16Blocks = 1000, kWide16Levels = 28, kSmemPerSM = 228 * 1024;
+__host__ __device__ constexpr bool prep_wide16(int nb, int nz, int arrays) {
+  if (3 * (arrays * (nz + 2) * CX * int(sizeof(double)) + 1024) > kSmemPerSM) return true;
+  return nb >= kWide16Blocks && nz >= kWide16Levels && 2 * cdiv(nb, 2 * kSMs) < 3 * cdiv(nb, 3 * kSMs);
+}
+static_assert(prep_wide16(1407, 48, 1) && prep_wide16(2008, 60, 3) && prep_wide16(1284, 100, 3) && prep_wide16(360, 100, 3));
+static_assert(!prep_wide16(5213, 8, 1) && !prep_wide16(5213, 20, 3) && !prep_wide16(1284, 60, 3) && !prep_wide16(3010, 60, 1) &&
+              !prep_wide16(1284, 100, 1) && !prep_wide16(360, 60, 3));
 
 // ---- WRF flux statement functions (src/dyn/kernels_common.hpp:11-105) ----
 template <class R>
