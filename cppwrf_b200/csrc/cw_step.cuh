@@ -322,17 +322,22 @@ struct Launcher {
     }
   }
   // A column kernel in its two forms: column blocks of 32 columns x 8 or 16 warps (shapes 0, 1; `arrays` shared level
-  // arrays of doubles) and level-thread columns of 8 (shape 2; `lc_arrays`).
+  // arrays of doubles) and level-thread columns of 8 (shape 2; `lc_arrays`), by default in at most max_waves waves.
   template <class R, int NM, class K, class K2, class... Args>
-  void run_col(const char* name, bool recurrence, int arrays, const std::array<K, 2>& wide, int lc_arrays, K2 lc,
+  void run_col(const char* name, int max_waves, bool recurrence, int arrays, const std::array<K, 2>& wide, int lc_arrays, K2 lc,
                const Packs<R, NM>& ps, Args... args) {
     flush();
     if (plan) return;
     int sh = shape_for(name);
     if (sh < 0) {
-      int nb = 0;
-      for (const auto& b : ps.blocks) nb += b[size_t(RG_COLS_STAG)][0];
-      sh = nb < kWideBlocks ? 2 : (recurrence && prep_wide16(nb, h->nzmax, arrays) ? 1 : 0);
+      int nb = 0, nlc = 0;
+      for (const auto& b : ps.blocks) {
+        nb += b[size_t(RG_COLS_STAG)][0];
+        nlc += b[size_t(RG_LCOLS_STAG)][0];
+      }
+      const bool fits = col_shape(2, h->nzmax) == 2;
+      if (nb < kWideBlocks) sh = fits && lc_waves(nlc, h->nzmax) > max_waves ? 0 : 2;
+      else sh = recurrence && prep_wide16(nb, h->nzmax, arrays) ? 1 : 0;
     }
     sh = col_shape(sh, h->nzmax);
     if (sh == 2) launch_lc(name, 0, lc_arrays, 0, 8, lc, ps, args...);
@@ -399,7 +404,7 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
     // fill would make them (only the scalars change in between), so only the first stage runs it (the fill merges
     // with the scalars' H_Q2 into one launch: fewer cells, not fewer launches)
     if (rk == 1) L.halo(cw_handle::H_PREP0);
-    L.run_col("k_ls_prep", true, 1, std::array{k_ls_prep<R, NM, cb_warps(0)>, k_ls_prep<R, NM, cb_warps(1)>}, kLsArrays, k_ls_prep_lc<R, NM, 0>, d);
+    L.run_col("k_ls_prep", kLsWaves, true, 1, std::array{k_ls_prep<R, NM, cb_warps(0)>, k_ls_prep<R, NM, cb_warps(1)>}, kLsArrays, k_ls_prep_lc<R, NM, 0>, d);
     L.halo(cw_handle::H_PREP1);
     if (rk == 1 && (dampkm || smag)) {  // DiffusionDriver::prepare: km_opt 4's and damp_opt 1's eddy viscosities
       if (smag) L.run_t("k_smag", RG_MASS, 1, KV(k_smag), d);
@@ -422,7 +427,7 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
     }
     if (h->cfl_on) L.run_t("k_cfl", RG_MASS, 1, KV(k_cfl), d, rk);
     if (rk == 1) L.copy_list(h->zeros_d, h->zeros_start_d, h->zeros.size(), h->zeros_total);
-    L.run_col("k_ss_prep", true, 3, std::array{k_ss_prep<R, NM, cb_warps(0)>, k_ss_prep<R, NM, cb_warps(1)>}, kSsArrays, k_ss_prep_lc<R, NM, 0>, d, rk);
+    L.run_col("k_ss_prep", ss_waves(sizeof(R)), true, 3, std::array{k_ss_prep<R, NM, cb_warps(0)>, k_ss_prep<R, NM, cb_warps(1)>}, kSsArrays, k_ss_prep_lc<R, NM, 0>, d, rk);
     if (dec) L.halo(cw_handle::H_SS0);
     for (int it = 1; it <= ns; ++it) {
       L.run_t("k_uv", RG_STAG, 1, KV(k_uv), d, rk);
@@ -434,7 +439,7 @@ void enqueue_step(cw_handle* h, Launcher& L, const Packs<R, NM>& d) {
     // (k_finish reads mu_ts past the edge as the substeps do: elsewhere than on specified domains its fill waits for the
     // one after it, in one launch)
     if (dec || spec_all) L.halo(cw_handle::H_POST);
-    L.run_col("k_finish", false, 0, std::array{k_finish<R, NM, cb_warps(0)>, k_finish<R, NM, cb_warps(1)>}, 1, k_finish_lc<R, NM, 0>, d, rk, ns);
+    L.run_col("k_finish", kFinishWaves, false, 0, std::array{k_finish<R, NM, cb_warps(0)>, k_finish<R, NM, cb_warps(1)>}, 1, k_finish_lc<R, NM, 0>, d, rk, ns);
     if (!dec && !spec_all) L.halo(cw_handle::H_POST);
     L.halo(cw_handle::H_FIN);
     if (scalars) {

@@ -224,17 +224,28 @@ __host__ __device__ constexpr int ac_shape(int sh, int nz) {
   return lc_threads(sh, nz) > kLcMaxThreads ? 2 : sh;
 }
 __host__ __device__ constexpr int col_shape(int sh, int nz) { return sh == 2 && lc_threads(0, nz) > kLcMaxThreads ? 1 : sh; }
-// Where the preparation and finish kernels change form, in blocks of 32 columns over the launch's rows. Below kWideBlocks
-// (under two such blocks per SM) the latency of a column's levels in turn is what they take, and a thread per level is
-// faster: k_ls_prep, k_ss_prep, k_finish 33 / 49 / 57 -> 11 / 19 / 15 us at 200 x 100 (7 blocks), 17 / 27 / 30 -> 15 / 23
-// / 19 us at 65 x 63 x 40 (192). Above it, their loads and stores are what they take, and rows of 32 columns are: 35 / 41
-// / 47 against 43 / 58 / 43 us at 119 x 89 x 44 (360 blocks), 129 / 185 / 190 against 172 / 248 / 188 at 200 x 200 x 60.
-constexpr int kWideBlocks = 250;
+// Where the preparation and finish kernels change form, in blocks of 32 columns over the launch's rows. From kWideBlocks on
+// (two such blocks per SM are nearly there) rows of 32 columns: at 119 x 89 x 44 (360 blocks) k_ls_prep and k_ss_prep take 35 and
+// 41 us against 43 and 58 of the level-thread form, at 200 x 200 x 60 129 and 185 against 172 and 248. k_finish is even there (47
+// against 43 and 190 against 188) and slower on the larger and taller ones (400 x 400 x 40 424 against 501, mixed 282 against
+// 310). Below kWideBlocks the latency of a column's levels in turn is what the rows take, and a thread per level is faster
+// while its blocks are few waves: an SM holds 1024 of its threads (64 registers), so a block of 8 columns x 61 levels is
+// alone there, and the rows, one wave at any nz, win again. us per launch, rows / level-thread, FP64 | mixed: k_ls_prep
+// 40 x 40 x 35 (1 wave) 19 / 11 | 19 / 11, 62 x 90 x 44 (3) 25 / 21 | 23 / 21, 119 x 60 x 44 (4) 25 / 25 | 22 / 23, 119 x 60 x 60 (7) 32 / 43
+// | 28 / 38; k_ss_prep 40 x 40 x 100 (2) 58 / 33 | 48 / 37, 62 x 90 x 44 (3) 37 / 35 | 31 / 35, 100 x 30 x 100 (3) 63 / 49 | 54 / 55, 119 x 60
+// x 44 (4) 37 / 44 | 30 / 43, 119 x 60 x 60 (7) 47 / 75 | 39 / 83; k_finish, without recurrences, 100 x 30 x 60 (3) 39 / 25 | 25 / 15,
+// 119 x 60 x 60 (7) 50 / 53 | 36 / 27.
+constexpr int kWideBlocks = 250, kLsWaves = 4, kFinishWaves = 7;
+constexpr int ss_waves(size_t real) { return real == 8 ? 3 : 2; }
 // their shared memory: k_ac's level arrays of doubles and of the fields' type and its per-column scalars, the others'
 // level arrays of doubles
 constexpr int kAcArrays = 5, kAcFields = 13, kAcScalars = 8, kLsArrays = 2, kSsArrays = 5;
 constexpr int kCbArrays = 6;  // shared-memory level arrays of the microphysics' column block: kCbArrays x (nz + 2) x CX doubles
 __host__ __device__ __forceinline__ constexpr int cdiv(int a, int b) { return (a + b - 1) / b; }
+constexpr int kSMs = 148;
+// the waves of nb level-thread blocks of 8 columns and 64 registers a thread at nz levels (nz <= 123)
+__host__ __device__ constexpr int lc_waves(int nb, int nz) { return cdiv(nb, kSMs * (1024 / lc_threads(0, nz))); }
+static_assert(lc_waves(246, 35) == 1 && lc_waves(246, 100) == 2 && lc_waves(728, 44) == 3 && lc_waves(915, 60) == 7);
 // Whether k_ls_prep and k_ss_prep run their nb blocks of 32 columns (at least kWideBlocks) with 16 warps instead of 8; `arrays`:
 // the shared level arrays of the kernel. An SM holds three blocks of 8 warps or two of 16 (cb_minblocks), which advance the
 // levels equally fast together, so what decides is how full the last wave of blocks is: 16 warps where two blocks times
@@ -243,7 +254,7 @@ __host__ __device__ __forceinline__ constexpr int cdiv(int a, int b) { return (a
 // mixed (3010) 184 / 187 and 296 / 305. Below 28 levels 16 warps have too few each (400 x 400 x 8: 89 / 117 and 117 / 142,
 // x 20: 167 / 193 and 234 / 270). Where shared memory leaves two blocks of either form (k_ss_prep from 98 levels on) the
 // one with more warps: 100 x 320 x 100 349 / 286, 119 x 89 x 100 139 / 113.
-constexpr int kSMs = 148, kWide16Blocks = 1000, kWide16Levels = 28, kSmemPerSM = 228 * 1024;
+constexpr int kWide16Blocks = 1000, kWide16Levels = 28, kSmemPerSM = 228 * 1024;
 __host__ __device__ constexpr bool prep_wide16(int nb, int nz, int arrays) {
   if (3 * (arrays * (nz + 2) * CX * int(sizeof(double)) + 1024) > kSmemPerSM) return true;
   return nb >= kWide16Blocks && nz >= kWide16Levels && 2 * cdiv(nb, 2 * kSMs) < 3 * cdiv(nb, 3 * kSMs);

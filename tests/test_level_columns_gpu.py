@@ -40,6 +40,16 @@ def test_both_sides_of_the_whole_row_blocks(ny):
     assert not bad, "\n".join(bad)
 
 
+@pytest.mark.parametrize("ny", [108, 115, 150])
+def test_around_the_waves_of_the_level_thread_form(ny):
+    """At 61 w levels an SM holds one level-thread block: 4 (ny + 1) blocks are 3, 4 and 5 waves, where k_ss_prep, then
+    k_ls_prep too, run in rows."""
+    case = lam_case(nx=30, ny=ny, nz=60, n_moist=1, n_scalars=1, seed=6)
+    dom, orc = run_pair(case, 1)
+    bad = compare_all(dom, orc, case, names=capi.STATE_FIELDS)
+    assert not bad, "\n".join(bad)
+
+
 @pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED], ids=["fp64", "mixed"])
 @pytest.mark.parametrize("nz", [20, 70, 126])
 def test_every_tuned_shape_gives_the_same_bits(nz, precision):
