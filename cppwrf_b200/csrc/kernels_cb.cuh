@@ -278,29 +278,26 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __gr
   const bool mass = col && i < nx && j < ny;
   const R dts = rk == 1 ? D.r.dt3 : D.r.dts;
   const R hd_dt = (rk == 3 && D.n_moist > 0) ? dts * R(nsmall) : R(0);
-  // mu_ts of the neighbour columns: past the domain's edge the column that a halo fill would copy
+  // mu_ts of the column and its neighbours: past the domain's edge the column that a halo fill would copy
   auto mts_at = [&](int ii, int jj) { return D.muts.ld(edge_col(ii, nx, D.bc_x), edge_col(jj, ny, D.bc_y), 0); };
   if (col) {
+    const R mts_ij = mts_at(i, j), mts_im = mts_at(i - 1, j), mts_jm = mts_at(i, j - 1);
     CB_LOOP(k, nz + 1) {  // every load of a level before its first store
       const bool has_u = j < ny && k < nz, has_v = i < nx && j < nyv && k < nz;
       const R c1h = k < nz ? D.r.c1h[k] : R(0), c2h = k < nz ? D.r.c2h[k] : R(0);
-      R u2 = 0, usv = 0, msfuy = 0, muu = 0, mts_u0 = 0, mts_u1 = 0;
+      R u2 = 0, usv = 0, msfuy = 0, muu = 0;
       if (has_u) {
         u2 = D.u2(i, j, k);
         usv = D.u_save.ld(i, j, k);
         msfuy = D.msfuy(i, j);
         muu = D.muu.ld(i, j, 0);
-        mts_u0 = mts_at(i, j);
-        mts_u1 = mts_at(i - 1, j);
       }
-      R v2 = 0, vsv = 0, msfvx = 0, muv = 0, mts_v0 = 0, mts_v1 = 0;
+      R v2 = 0, vsv = 0, msfvx = 0, muv = 0;
       if (has_v) {
         v2 = D.v2(i, j, k);
         vsv = D.v_save.ld(i, j, k);
         msfvx = D.msfvx(i, j);
         muv = D.muv.ld(i, j, 0);
-        mts_v0 = mts_at(i, j);
-        mts_v1 = mts_at(i, j - 1);
       }
       R m = 0, mts = 0, w2 = 0, wsv = 0, msfty = 0, ph2 = 0, phsv = 0, ww = 0, ww1 = 0, t2 = 0, tsv = 0, hd = 0;
       if (mass) {
@@ -319,14 +316,8 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __gr
           if (hd_dt != R(0)) hd = D.hd.ld(i, j, k);
         }
       }
-      if (has_u) {
-        const R mus_u = R(0.5) * (mts_u0 + mts_u1);
-        D.u2(i, j, k) = (msfuy * u2 + usv * (c1h * muu + c2h)) / (c1h * mus_u + c2h);
-      }
-      if (has_v) {
-        const R mus_v = R(0.5) * (mts_v0 + mts_v1);
-        D.v2(i, j, k) = (msfvx * v2 + vsv * (c1h * muv + c2h)) / (c1h * mus_v + c2h);
-      }
+      if (has_u) D.u2(i, j, k) = (msfuy * u2 + usv * (c1h * muu + c2h)) / (c1h * (R(0.5) * (mts_ij + mts_im)) + c2h);
+      if (has_v) D.v2(i, j, k) = (msfvx * v2 + vsv * (c1h * muv + c2h)) / (c1h * (R(0.5) * (mts_ij + mts_jm)) + c2h);
       if (mass) {
         D.w2(i, j, k) = (msfty * w2 + wsv * (D.r.c1f[k] * m + D.r.c2f[k])) / (D.r.c1f[k] * mts + D.r.c2f[k]);
         D.ph2(i, j, k) = ph2 + phsv;
@@ -337,8 +328,8 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __gr
     }
     if (threadIdx.y == 0) {
       if (mass) D.mu2(i, j, 0) = D.mu2(i, j, 0) + D.mu_save(i, j, 0);
-      if (j < ny) D.muus(i, j, 0) = R(0.5) * (mts_at(i, j) + mts_at(i - 1, j));
-      if (i < nx && j < nyv) D.muvs(i, j, 0) = R(0.5) * (mts_at(i, j) + mts_at(i, j - 1));
+      if (j < ny) D.muus(i, j, 0) = R(0.5) * (mts_ij + mts_im);
+      if (i < nx && j < nyv) D.muvs(i, j, 0) = R(0.5) * (mts_ij + mts_jm);
     }
   }
   __syncthreads();
