@@ -361,7 +361,7 @@ def run_ensemble(args, torch, capi, Domain, Batch, rank=0, world=1):
             b.upload_case(k, c)
         lib.cw_set_stream(b.h, C.c_void_p(stream.cuda_stream))
         if not args.no_autotune:
-            b.set_autotune(True)  # the warm-up steps pick the batch's block shapes and warps per column block
+            b.set_autotune(True)  # the warm-up steps pick the batch's block shapes
         b.step(args.warmup)
         if world > 1:
             torch.distributed.barrier()

@@ -297,7 +297,7 @@ struct Launcher {
     }
   }
   // a level-thread column kernel: shared level arrays of doubles (`arrays`) and of the fields' type (`fields`), and
-  // `scalars` per-column doubles; the shape is the columns per block (lc_cols), narrower where they would be too many
+  // `scalars` doubles per column (k_ac's per-column scalars, the others' read-ahead); the shape is the columns per block (lc_cols), narrower where they would be too many
   // threads
   template <class R, int NM, class K, class... Args>
   void run_lc(const char* name, int arrays, int fields, int scalars, const std::array<K, kNumShapes>& kerns,
@@ -340,7 +340,7 @@ struct Launcher {
       else sh = recurrence && prep_wide16(nb, h->nzmax, arrays) ? 1 : 0;
     }
     sh = col_shape(sh, h->nzmax);
-    if (sh == 2) launch_lc(name, 0, lc_arrays, 0, 8, lc, ps, args...);
+    if (sh == 2) launch_lc(name, 0, lc_arrays, 0, kLcPad, lc, ps, args...);
     else launch_cb(name, RG_COLS_STAG, arrays, wide[size_t(sh)], cb_warps(sh), ps, args...);
   }
   // one block per member

@@ -240,6 +240,10 @@ constexpr int ss_waves(size_t real) { return real == 8 ? 3 : 2; }
 // their shared memory: k_ac's level arrays of doubles and of the fields' type and its per-column scalars, the others'
 // level arrays of doubles
 constexpr int kAcArrays = 5, kAcFields = 13, kAcScalars = 8, kLsArrays = 2, kSsArrays = 5;
+// lc_serial reads up to kLcAhead levels past the last one that it steps through. Level arrays hold nz + 1 levels, so where
+// a recurrence reads the block's last array (k_ls_prep's, over levels 0 .. nz - 2) the read-ahead ends kLcPad levels after it;
+// elsewhere another array of at least four levels follows (going down: comes before).
+constexpr int kLcAhead = 4, kLcPad = kLcAhead - 2;
 constexpr int kCbArrays = 6;  // shared-memory level arrays of the microphysics' column block: kCbArrays x (nz + 2) x CX doubles
 __host__ __device__ __forceinline__ constexpr int cdiv(int a, int b) { return (a + b - 1) / b; }
 constexpr int kSMs = 148;

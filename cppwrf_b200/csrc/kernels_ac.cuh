@@ -22,8 +22,6 @@ __device__ __forceinline__ bool edge_vface(const Dom<R>& D, int i, int j) {
   return (D.sx && (i == 0 || i == D.nx - 1)) || (D.sy && (j <= 0 || j >= D.ny));
 }
 template <class R>
-__device__ __forceinline__ R mh_(const Dom<R>& D, int k, R m) { return D.r.c1h[k] * m + D.r.c2h[k]; }
-template <class R>
 __device__ __forceinline__ R mf_(const Dom<R>& D, int k, R m) { return D.r.c1f[k] * m + D.r.c2f[k]; }
 
 // p_rho_point (small_step.cpp:97-112): calc_p_rho of small_step_prep, without divergence damping (the substeps' damped
@@ -103,9 +101,10 @@ __device__ __forceinline__ R uv_dp(const Dom<R>& D, const UvPoint<R>& C, int om,
 // over the staggered index range; with lateral boundaries the spec zone's faces take
 // u += dts ru_tend (LateralBC::update_uv, lateral_bc.cpp:353-361) instead, and so do the faces of open boundaries
 // (no pressure gradient or divergence damping on them, :175-184). Bound by the latency of its loads: every value that the
-// two faces share is loaded once, from one offset per storage class. Registers: 64 in double (at 48 it spills: 36.7
-// against 31.9 us at 119 x 89 x 44, where the form that indexed each field for itself took 31.3), 48 in float (22.3 us; 26.0
-// before; 300 x 300 x 60: 221 -> 175 us).
+// two faces share is loaded once, from one offset per storage class. Registers: 64 in double, 48 in float. In double it
+// spills 24 bytes a thread (a batch's instance 100), at 48 registers far more: 36.7 against 31.9 us at 119 x 89 x 44. The form
+// that indexed each field for itself took 31.3 us there; the constants in the fields' type took this one to 29.8. In
+// float 26.0 -> 22.3 us, 300 x 300 x 60 221 -> 175 us.
 template <class R, int NM, int SH>
 __global__ void __launch_bounds__(PX, sizeof(R) == 8 ? 8 : 10) k_uv(const __grid_constant__ Pack<R, NM> P, int rk) {
   const Dom<R>* Dp;

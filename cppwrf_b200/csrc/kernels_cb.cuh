@@ -356,9 +356,8 @@ __device__ __forceinline__ const Dom<R>& lc_member(const Pack<R, NM>& P, int& i,
 // arrays' first one and v[a] the element of array a (S = CB upwards, -CB downwards). The values of the next kLcAhead levels
 // are read while the present ones are stepped through, ahead of the stores that the steps make (the compiler may not move
 // a load across those): the chain is then its arithmetic, and not a shared-memory load a level as well. The last
-// read-ahead runs up to 2 kLcAhead - 1 levels past the arrays' last element: the callers' arrays have others of the
-// block's shared memory there.
-constexpr int kLcAhead = 4;
+// read-ahead runs up to kLcAhead levels past element n - 1 (n = 4 m + r ends at element 4 m + 3): the callers' arrays have
+// others of the block's shared memory there, or kLcPad levels.
 template <int S, class F, class... T>
 __device__ __forceinline__ void lc_serial(int n, F step, const T*... a) {
   constexpr int NA = sizeof...(T);
@@ -672,10 +671,13 @@ __global__ void __maxnreg__(64) k_ss_prep_lc(const __grid_constant__ Pack<R, NM>
 // own launch.
 // What bounds it: a block's latency (the loads, ten barriers, the column warp's chains of about 60 cycles a level), so
 // what counts is how many points an SM holds: 48 registers keep two blocks of 8 columns resident up to nz = 79 (64
-// registers: one block from nz = 60 on, 414 us instead of 268 at 200 x 200 x 60). 8 columns are the narrowest segment
-// that serves double precision (4: 76 against 59 us at 119 x 89 x 44). One warp per level row of 32 columns and 8 or 16
-// levels in turn, the form this replaced, took (us per launch, now in parentheses): 64 x 32 30 (12.8), 200 x 100 83 (19),
-// 119 x 89 x 44 90 (59), mixed 67 (46), 200 x 200 x 60 308 (268), mixed 300 x 300 x 60 737 (516).
+// registers: one block from nz = 60 on, 414 us instead of 268 at 200 x 200 x 60), though in double they spill 64 bytes a
+// thread (a batch's instance 140; in float 0 and 56). 8 columns are the narrowest segment that serves double precision
+// (4: 76 against 59 us at 119 x 89 x 44). One warp per level row of 32 columns and 8 or 16 levels in turn, the form this
+// replaced, took (us per launch, the faster of 8 and 16; now in parentheses): 64 x 32 30 (12.8), 200 x 100 83 (19), 119 x 89
+// x 44 90 (59), mixed 67 (46), 200 x 200 x 60 308 (268), mixed 300 x 300 x 60 737 (516). One block of 8 columns is resident from
+// 80 levels on and blocks have 4 columns from 124 on, and they are still the faster: 200 x 200 x 100 764 (567), 119 x 89 x 100
+// 254 (162), 119 x 89 x 124 312 (205); 8 warps 200 x 200 x 80 887 (495), 100 x 100 x 126 484 (196), 119 x 89 x 124 mixed 419 (183).
 template <class R, int NM, int SH>
 __global__ void __maxnreg__(48) k_ac(const __grid_constant__ Pack<R, NM> P, int rk, int it, int nsteps) {
   using A = double;

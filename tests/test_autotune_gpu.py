@@ -1,7 +1,9 @@
 # SPDX-License-Identifier: GPL-3.0-or-later
 """Block-shape autotuning: the tuning steps are ordinary steps and every shape computes the same values, so an
 autotuned run is bit-identical to a run with the default shapes; afterwards each tunable kernel has a choice. A
-column kernel's shape is its warps per column block (8, 16 or 4): only the parallel loops over levels change."""
+column kernel's shapes are different kernels -- rows of 32 columns with 8 or 16 warps and a thread per column and level
+(k_ac: the latter with 8, 16 or 4 columns) -- whose arithmetic is written twice: that they give the same bits is what
+these tests and test_level_columns_gpu.py check."""
 import numpy as np
 import pytest
 
@@ -11,8 +13,7 @@ from cases import lam_case
 pytestmark = pytest.mark.gpu
 
 TUNABLE = ["k_tend", "k_tendf_rk1", "k_uv", "k_q_march", "k_q_face_pd", "k_q_scale_pd", "k_q_update_pd",
-           "k_ls_prep", "k_ss_prep", "k_ac", "k_finish"]  # k_q_march: levels per block; the last four: warps per
-#                                                             column block
+           "k_ls_prep", "k_ss_prep", "k_ac", "k_finish"]
 
 
 @pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED], ids=["fp64", "mixed"])

@@ -6,7 +6,7 @@ in blocks of whole rows. The FP64 form equals the oracle bit for bit; every auto
 import numpy as np
 import pytest
 
-from cppwrf_b200 import Domain, capi
+from cppwrf_b200 import Batch, Domain, capi
 from cases import golden_config, ideal_case, lam_case
 from test_parity_gpu import compare_all, run_pair
 
@@ -56,8 +56,27 @@ def test_every_tuned_shape_gives_the_same_bits(nz, precision):
     case = lam_case(nx=21, ny=11, nz=nz, n_moist=1, n_scalars=1, seed=nz, precision=precision)
     a = Domain(case.g, case.o).upload_case(case).set_autotune(True).step(6)
     b = Domain(case.g, case.o).upload_case(case).step(6)
-    for name in capi.STATE_FIELDS:
+    for name in capi.STATE_FIELDS + ["Q_2"]:
         assert np.array_equal(a.field(name).view(np.uint64), b.field(name).view(np.uint64)), name
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED], ids=["fp64", "mixed"])
+def test_every_tuned_shape_gives_the_same_bits_in_a_batch(precision):
+    """Members of uneven level counts in blocks sized for the tallest one; the batch untuned, tuned, and its members alone."""
+    cases = [lam_case(nx=nx, ny=9, nz=nz, n_moist=2, n_scalars=2, seed=nz, precision=precision)
+             for nx, nz in ((21, 12), (14, 70), (33, 31))]
+    a, b = (Batch([c.g for c in cases], [c.o for c in cases]) for _ in range(2))
+    for m, c in enumerate(cases):
+        a.upload_case(m, c)
+        b.upload_case(m, c)
+    a.set_autotune(True).step(6)
+    b.step(6)
+    for m, c in enumerate(cases):
+        d = Domain(c.g, c.o).upload_case(c).step(6)
+        for name in capi.STATE_FIELDS + ["Q_2"]:
+            x = d.field(name).view(np.uint64)
+            assert np.array_equal(a.field(m, name).view(np.uint64), x), (m, name)
+            assert np.array_equal(b.field(m, name).view(np.uint64), x), (m, name)
 
 
 @pytest.mark.parametrize("nz", [61, 70, 124, 126])
