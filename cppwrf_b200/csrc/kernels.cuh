@@ -837,7 +837,7 @@ __device__ __forceinline__ bool ring_locate(int ibe, int jbe, int i, int j, int&
 // KRelax (lateral_bc.cpp:79-118) at ring point (pos, side, b) level k of one variable: returns
 // fa = fcx * fls0 and fb = gcx * (fls1 + fls2 + fls3 + fls4 - 4 fls0); the relaxation term is fa - fb.
 template <class R, bool Two>
-__device__ void relax_terms(const Dom<R>& D, const V3<R>& f, const double* c1, const double* c2, const Slabs<R>& s,
+__device__ __forceinline__ void relax_terms(const Dom<R>& D, const V3<R>& f, const double* c1, const double* c2, const Slabs<R>& s,
                             Ring r, int pos, int side, int b, int k, int i, int j, R& fa, R& fb) {
   const int sl = slab_of_side(side);
   const R dtbc = R(*D.dtbc);
