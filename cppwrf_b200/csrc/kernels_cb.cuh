@@ -279,6 +279,7 @@ __global__ void __launch_bounds__(CX * NW, cb_minblocks(NW)) k_finish(const __gr
   const R dts = rk == 1 ? D.r.dt3 : D.r.dts;
   const R hd_dt = (rk == 3 && D.n_moist > 0) ? dts * R(nsmall) : R(0);
   // mu_ts of the column and its neighbours: past the domain's edge the column that a halo fill would copy
+  // (looked up once: in the level loop it cost 2 to 4 %, 468 -> 458 us at 400 x 400 x 44 FP64)
   auto mts_at = [&](int ii, int jj) { return D.muts.ld(edge_col(ii, nx, D.bc_x), edge_col(jj, ny, D.bc_y), 0); };
   if (col) {
     const R mts_ij = mts_at(i, j), mts_im = mts_at(i - 1, j), mts_jm = mts_at(i, j - 1);

@@ -33,3 +33,13 @@ def test_small_members_of_a_batch():
         orc.step(2)
         for name in capi.STATE_FIELDS:
             assert np.array_equal(b.field(m, name).view(np.uint64), orc.array(name).view(np.uint64)), (m, name)
+
+
+@pytest.mark.parametrize("nx,ny,px,py", [(14, 6, 2, 1), (7, 13, 1, 2)])
+def test_small_side_of_a_decomposed_domain(nx, ny, px, py):
+    from test_decomp_gpu import compare, run_both
+
+    case = lam_case(nx=nx, ny=ny, nz=8, n_moist=2, n_scalars=2, seed=nx)
+    dec, dom = run_both(case, px, py, 2)
+    bad = compare(dec, dom, case)
+    assert not bad, "\n".join(bad)
